@@ -33,68 +33,203 @@ struct EllLev {
   const float* __restrict__ Kf;     // 3*NN FP32 coefficient cf*Ie*ped/len (mixed-precision path)
   const float* __restrict__ hinvf;  // NN
   const float* __restrict__ diagf;  // NN
+  const float* __restrict__ oaf;    // 4*NN FP32 overlap areas
+  const int* __restrict__ bt;       // stencils of the border nodes, [18][10 * border_nodes(n)] (k_ell_border)
+  double cf;                        // theta1 theta2 dt^2
+  unsigned long long mg1, mg0;      // ceil(2^40 / (n + 1)), ceil(2^40 / n): divisions of thread indices
 };
 
 __device__ __forceinline__ double interp(double a, double b) { return 0.5 * (a + b); }
 
+// (d, i, j) of index t over the [0, m)^2 nodes of the ten lozenges, m = n + 1 or
+// n.  t / m = (t ceil(2^40 / m)) >> 40 exactly while t m < 2^40, which holds for
+// every level the context accepts (6 NN < 2^31); the two integer divisions it
+// replaces cost more than the stencil's own arithmetic.
 __device__ __forceinline__ void decode(const EllLev& L, int t, int& d, int& i, int& j, int m) {
-  d = t / (m * m);
-  int r = t - d * m * m;
-  j = r / m;
-  i = r - j * m;
+  const unsigned long long mg = m == L.n ? L.mg0 : L.mg1;
+  const int row = (int)(((unsigned long long)t * mg) >> 40);
+  d = (int)(((unsigned long long)row * mg) >> 40);
+  j = row - d * m;
+  i = t - row * m;
 }
 
-__device__ __forceinline__ int64_t nidx(const EllLev& L, int d, int i, int j) {
-  return ((int64_t)d * L.P + (j + 2)) * L.P + (i + 2);
+// Slots inside one level fit an int (6 NN < 2^31).
+__device__ __forceinline__ int nidx(const EllLev& L, int d, int i, int j) {
+  return (d * L.P + (j + 2)) * L.P + (i + 2);
 }
 
-// Flux of the edge slot through its remap (step1 itype 2, src/ops.f90:202-216):
+// Nodes whose whole stencil (radius 1) lies on owned nodes of the lozenge: every
+// remap there is the identity, so the operator reads its neighbours directly.  The
+// other nodes of [0, n]^2 (rows and columns 0, n-1, n) have their remapped stencil
+// in a table: through the remap each value hangs on two loads of codes, and the
+// FP32 sweep of a J8 level took 17 us, five times its bytes' time from L2.
+__device__ __forceinline__ bool ell_inner(const EllLev& L, int i, int j) {
+  return i >= 1 && j >= 1 && i <= L.n - 2 && j <= L.n - 2;
+}
+__host__ __device__ inline int border_nodes(int n) { return 3 * (n + 1) + 3 * (n - 2); }
+__device__ __forceinline__ int border_index(int n, int d, int i, int j) {
+  const int m = n + 1;
+  int b;
+  if (j == 0) b = i;
+  else if (j == n - 1) b = m + i;
+  else if (j == n) b = 2 * m + i;
+  else b = 3 * m + 3 * (j - 1) + (i == 0 ? 0 : i == n - 1 ? 1 : 2);
+  return d * border_nodes(n) + b;
+}
+
+// Flux of one edge (step1 itype 2, src/ops.f90:202-216):
 // interp(csq0, csq1) * (q1/phi1 - q0/phi0) / len * pedlen with phi = 1.
-__device__ __forceinline__ double ell_flux(const EllLev& L, const double* __restrict__ q, int64_t slot) {
-  const int code = L.esrc[slot];
-  const int64_t src = code >> 1;
-  const int e = (int)(src / L.NN);
-  const int64_t node = src - (int64_t)e * L.NN;
-  const double q0 = q[L.nsrc[node]];
-  double f;
-  if (e == RT) {
-    const double q1 = q[L.nsrc[node + 1]];
-    f = L.Ie[src] * (q1 / 1.0 - q0 / 1.0) / L.len[src] * L.ped[src];
-  } else if (e == DG) {
-    const double q2 = q[L.nsrc[node + L.P + 1]];
-    f = L.Ie[src] * (q0 / 1.0 - q2 / 1.0) / L.len[src] * L.ped[src];
-  } else {
-    const double q3 = q[L.nsrc[node + L.P]];
-    f = L.Ie[src] * (q3 / 1.0 - q0 / 1.0) / L.len[src] * L.ped[src];
+__device__ __forceinline__ double ell_edge(const EllLev& L, int slot, double dq) {
+  return L.Ie[slot] * dq / L.len[slot] * L.ped[slot];
+}
+__device__ __forceinline__ float ell_edge(const EllLev& L, int slot, float dq) { return L.Kf[slot] * dq; }
+
+// The six edges of a node in the order its divergence takes them (RT, RT of W, DG
+// of SW, DG, UP, UP of S): edge slot, and the nodes the flux takes its difference
+// from (q[b] - q[a]); a negated ghost edge has a and b exchanged, which negates
+// its flux exactly.
+__global__ void k_ell_border(int n, int P, int NN, const int* __restrict__ nsrc, const int* __restrict__ esrc,
+                             int* __restrict__ bt) {
+  const int m = n + 1, t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 10 * m * m) return;
+  const int d = t / (m * m), r = t - d * m * m, j = r / m, i = r - j * m;
+  if (i >= 1 && j >= 1 && i <= n - 2 && j <= n - 2) return;
+  const int id = (d * P + j + 2) * P + i + 2, nb = 10 * border_nodes(n), x = border_index(n, d, i, j);
+  const int at[6] = {RT * NN + id, RT * NN + id - 1, DG * NN + id - P - 1, DG * NN + id, UP * NN + id, UP * NN + id - P};
+  for (int e = 0; e < 6; ++e) {
+    const int code = esrc[at[e]], src = code >> 1, k = src / NN, node = src - k * NN;
+    const int q0 = nsrc[node], q1 = nsrc[node + (k == RT ? 1 : k == DG ? P + 1 : P)];
+    int a = k == DG ? q1 : q0, b = k == DG ? q0 : q1;
+    if (code & 1) {
+      const int x_ = a;
+      a = b;
+      b = x_;
+    }
+    bt[(3 * e) * nb + x] = src;
+    bt[(3 * e + 1) * nb + x] = a;
+    bt[(3 * e + 2) * nb + x] = b;
   }
-  return (code & 1) ? -f : f;
+}
+
+__device__ __forceinline__ double ell_hinv(const EllLev& L, int id, double) { return L.hinv[id]; }
+__device__ __forceinline__ float ell_hinv(const EllLev& L, int id, float) { return L.hinvf[id]; }
+__device__ __forceinline__ double ell_diag(const EllLev& L, int id, double) { return L.diag[id]; }
+__device__ __forceinline__ float ell_diag(const EllLev& L, int id, float) { return L.diagf[id]; }
+__device__ __forceinline__ double ell_scale(const EllLev& L, double div) { return L.cf * div; }
+__device__ __forceinline__ float ell_scale(const EllLev&, float div) { return div; }  // cf is in Kf
+
+// The node's six differences and edge slots, val(x) the value at node x, qc its own.
+template <class T, class Val>
+__device__ __forceinline__ void ell_stencil(const EllLev& L, Val val, int id, int d, int i, int j, bool inner, T qc,
+                                            T (&dq)[6], int (&slot)[6]) {
+  const int NN = (int)L.NN, P = L.P;
+  if (inner) {
+    const T qE = val(id + 1), qW = val(id - 1), qN = val(id + P), qS = val(id - P), qNE = val(id + P + 1),
+            qSW = val(id - P - 1);
+    dq[0] = qE - qc;
+    dq[1] = qc - qW;
+    dq[2] = qSW - qc;
+    dq[3] = qc - qNE;
+    dq[4] = qN - qc;
+    dq[5] = qc - qS;
+    slot[0] = RT * NN + id;
+    slot[1] = RT * NN + id - 1;
+    slot[2] = DG * NN + id - P - 1;
+    slot[3] = DG * NN + id;
+    slot[4] = UP * NN + id;
+    slot[5] = UP * NN + id - P;
+  } else {
+    const int nb = 10 * border_nodes(L.n), x = border_index(L.n, d, i, j);
+    int a[6], b[6];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      slot[e] = L.bt[(3 * e) * nb + x];
+      a[e] = L.bt[(3 * e + 1) * nb + x];
+      b[e] = L.bt[(3 * e + 2) * nb + x];
+    }
+    T va[6], vb[6];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      va[e] = val(a[e]);
+      vb[e] = val(b[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 6; ++e) dq[e] = vb[e] - va[e];
+  }
+}
+
+// elliptic_lo (src/barotropic_2d.f90:187-250) at node (d, i, j) = id, qc its own
+// value.  FP64 takes the reference's operand order; FP32 the coefficients K = cf
+// interp(csq) pedlen / len.
+template <class T, class Val>
+__device__ __forceinline__ T ell_lo(const EllLev& L, Val val, int id, int d, int i, int j, bool inner, T qc) {
+  T dq[6];
+  int slot[6];
+  ell_stencil(L, val, id, d, i, j, inner, qc, dq, slot);
+  T f[6];
+#pragma unroll
+  for (int e = 0; e < 6; ++e) f[e] = ell_edge(L, slot[e], dq[e]);
+  const T div = (f[0] - f[1] + f[2] - f[3] + f[4] - f[5]) * ell_hinv(L, id, qc);
+  return ell_scale(L, div) - qc;
 }
 
 enum { OP_APPLY = 0, OP_JACOBI = 1, OP_RESID = 2 };
 
-// elliptic_lo (src/barotropic_2d.f90:187-250) on [0, n]^2 of one level, fused
-// with its consumer: OP_APPLY out = L(q); OP_RESID out = f - L(q) (cal_res,
-// src/lin_solve.f90:574); OP_JACOBI out = q + w (f - L(q)) / diag (cal_jacobi,
-// src/lin_solve.f90:343).  Ghosts that are copies of another node are not
-// computed (every read of them goes to their source).
-template <int OP>
-__global__ void k_ell_op(EllLev L, double cf, const double* __restrict__ q, const double* __restrict__ f,
-                         double* __restrict__ out, double w) {
+// elliptic_lo on [0, n]^2 of one level, fused with its consumer: OP_APPLY out =
+// L(q); OP_RESID out = f - L(q) (cal_res, src/lin_solve.f90:574); OP_JACOBI out
+// = q + w (f - L(q)) / diag (cal_jacobi, src/lin_solve.f90:343).  Ghosts that
+// are copies of another node are not computed (every read of them goes to
+// their source).  acc (OP_JACOBI): add the result there in FP64.
+template <int OP, class T>
+__global__ void __launch_bounds__(256, 4) k_ell_op(EllLev L, const T* __restrict__ q, const T* __restrict__ f,
+                                                T* __restrict__ out, T w, double* __restrict__ acc) {
   const int m = L.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 10 * m * m) return;
   int d, i, j;
   decode(L, t, d, i, j, m);
-  const int64_t id = nidx(L, d, i, j);
-  if (L.nsrc[id] != id) return;
-  const int64_t NN = L.NN, P = L.P;
-  const double div = (ell_flux(L, q, RT * NN + id) - ell_flux(L, q, RT * NN + id - 1) + ell_flux(L, q, DG * NN + id - P - 1) -
-                      ell_flux(L, q, DG * NN + id) + ell_flux(L, q, UP * NN + id) - ell_flux(L, q, UP * NN + id - P)) *
-                     L.hinv[id];
-  const double lq = cf * div - q[id];
+  const int id = nidx(L, d, i, j);
+  const bool inner = ell_inner(L, i, j);
+  if (!inner && L.nsrc[id] != id) return;
+  const T qc = q[id];
+  const T fc = OP == OP_APPLY ? T(0) : f[id];
+  const T lq = ell_lo(L, [&](int x) { return q[x]; }, id, d, i, j, inner, qc);
   if (OP == OP_APPLY) out[id] = lq;
-  if (OP == OP_RESID) out[id] = f[id] - lq;
-  if (OP == OP_JACOBI) out[id] = q[id] + w * (f[id] - lq) / L.diag[id];
+  if (OP == OP_RESID) out[id] = fc - lq;
+  if (OP == OP_JACOBI) {
+    const T v = qc + w * (fc - lq) / ell_diag(L, id, qc);
+    out[id] = v;
+    if (acc) acc[id] = acc[id] + (double)v;
+  }
+}
+
+// The first two Jacobi sweeps (w = 1) from a zero guess in one pass: the first
+// leaves c1 = f / diag, which every thread forms at its stencil's nodes, so c1
+// is neither written nor read.  One sweep (two = 0) writes c1 itself.  Saves the
+// zeroing, one launch and one pass over the level per V-cycle and level.
+template <class T>
+__device__ __forceinline__ T ell_first(const EllLev& L, const T* __restrict__ f, int id) {
+  const T z = T(0);
+  return z + T(1) * (f[id] - z) / ell_diag(L, id, z);
+}
+template <class T>
+__global__ void __launch_bounds__(256, 4) k_ell_first2(EllLev L, const T* __restrict__ f, T* __restrict__ out, int two) {
+  const int m = L.n + 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 10 * m * m) return;
+  int d, i, j;
+  decode(L, t, d, i, j, m);
+  const int id = nidx(L, d, i, j);
+  const bool inner = ell_inner(L, i, j);
+  if (!inner && L.nsrc[id] != id) return;
+  const T qc = ell_first(L, f, id);
+  if (!two) {
+    out[id] = qc;
+    return;
+  }
+  const T fc = f[id];
+  const T lq = ell_lo(L, [&](int x) { return ell_first(L, f, x); }, id, d, i, j, inner, qc);
+  out[id] = qc + T(1) * (fc - lq) / ell_diag(L, id, qc);
 }
 
 // cal_lc (src/lin_solve.f90:529): s = a1 s1 + a2 s2 on [0, n]^2.  The
@@ -108,7 +243,7 @@ __global__ void k_ell_lc(EllLev L, double* __restrict__ s, double a1, const doub
   if (t >= 10 * m * m) return;
   int d, i, j;
   decode(L, t, d, i, j, m);
-  const int64_t id = nidx(L, d, i, j);
+  const int id = nidx(L, d, i, j);
   if (L.nsrc[id] != id) return;
   const double c1 = ap1 ? *ap1 : a1;
   const double c2 = ap2 ? sgn2 * *ap2 : a2;
@@ -117,181 +252,568 @@ __global__ void k_ell_lc(EllLev L, double* __restrict__ s, double a1, const doub
 
 // Weighted sums of l2 / dp (src/lin_solve.f90:433-502): every (i, j) in
 // [0, n]^2 of every lozenge, counted once per DOMAIN_LEVEL sub-domain whose
-// (0,1) range contains it.  Block partial sums; k_final_sum adds them in a
-// fixed order.
-template <int BS>
-__global__ void k_ell_dot(EllLev L, const double* __restrict__ a, const double* __restrict__ b,
-                          double* __restrict__ partial) {
-  __shared__ double sh[BS / 32];
+// (0,1) range contains it.  256 consecutive nodes give one partial (a fixed
+// shuffle order); the partials are added in a fixed order by 256 threads, so a
+// sum has the same bits whichever kernel forms it.
+__device__ __forceinline__ double ell_weigh(const EllLev& L, int i, int j, double x) {
+  const int wi = (i > 0 && i < L.n && i % L.nd == 0) ? 2 : 1;
+  const int wj = (j > 0 && j < L.n && j % L.nd == 0) ? 2 : 1;
+  double v = x;
+  if (wi * wj >= 2) v = v + x;
+  if (wi * wj == 4) v = v + x + x;
+  return v;
+}
+// Sum over a group of 256 threads (8 warps, `sh` its 8 doubles, bar their
+// barrier); the value is thread 0's.
+template <class Bar>
+__device__ __forceinline__ double ell_sum256(double v, double* sh, int tid, Bar bar) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((tid & 31) == 0) sh[tid >> 5] = v;
+  bar();
+  if (tid < 32) {
+    v = tid < 8 ? sh[tid] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+
+// mode 0: sum; 1: sqrt(sum); 2: sqrt(sum) / *den (res_err).
+__device__ __forceinline__ double ell_finish(double v, int mode, const double* den) {
+  if (mode == 1) v = sqrt(v);
+  if (mode == 2) v = sqrt(v) / *den;
+  return v;
+}
+
+// The partial of this block into partial[]; the last block of the grid to
+// arrive (ticket, which it resets) adds them all and writes *out.  One launch a
+// reduction instead of two; blocks of 256 threads.
+__device__ __forceinline__ void ell_reduce(double v, double* partial, unsigned* ticket, double* out, int mode,
+                                           const double* den) {
+  __shared__ double sh[8];
+  __shared__ bool last;
+  auto bar = [] { __syncthreads(); };
+  const int tid = threadIdx.x;
+  v = ell_sum256(v, sh, tid, bar);
+  if (tid == 0) {
+    partial[blockIdx.x] = v;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0;
+  for (int k = tid; k < (int)gridDim.x; k += 256) a += __ldcg(partial + k);
+  a = ell_sum256(a, sh, tid, bar);
+  if (tid == 0) {
+    *out = ell_finish(a, mode, den);
+    *ticket = 0;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_ell_dot(EllLev L, const double* __restrict__ a, const double* __restrict__ b,
+                                                 double* partial, unsigned* ticket, double* out, int mode,
+                                                 const double* den) {
   const int m = L.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0.0;
   if (t < 10 * m * m) {
     int d, i, j;
     decode(L, t, d, i, j, m);
-    const int64_t id = nidx(L, d, i, j);
-    const int64_t s = L.nsrc[id];
-    const double x = a[s] * b[s];
-    const int wi = (i > 0 && i < L.n && i % L.nd == 0) ? 2 : 1;
-    const int wj = (j > 0 && j < L.n && j % L.nd == 0) ? 2 : 1;
-    v = x;
-    if (wi * wj >= 2) v = v + x;
-    if (wi * wj == 4) v = v + x + x;
+    const int s = L.nsrc[nidx(L, d, i, j)];
+    v = ell_weigh(L, i, j, a[s] * b[s]);
   }
+  ell_reduce(v, partial, ticket, out, mode, den);
+}
+
+// r = f - L(u), its weighted norm into *out (mode, den) and, where given, r
+// itself in FP64 (r64) and FP32 (r32); with next, also the Jacobi sweep next =
+// u + w r / diag.  A copy of another node takes the residual of its source, as
+// the sum over stored values would.  One stencil pass instead of residual, dot
+// and conversion passes.
+__global__ void __launch_bounds__(256, 4) k_ell_resid_norm(EllLev L, const double* __restrict__ u,
+                                                        const double* __restrict__ f, double* __restrict__ r64,
+                                                        float* __restrict__ r32, double* __restrict__ next, double w,
+                                                        double* partial, unsigned* ticket, double* out, int mode,
+                                                        const double* den) {
+  const int m = L.n + 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  double v = 0.0;
+  if (t < 10 * m * m) {
+    int d, i, j;
+    decode(L, t, d, i, j, m);
+    const int id = nidx(L, d, i, j);
+    const bool inner = ell_inner(L, i, j);
+    int s = id, sd = d, si = i, sj = j;
+    if (!inner) {
+      s = L.nsrc[id];
+      const int row = s / L.P;
+      si = s - row * L.P - 2;
+      sd = row / L.P;
+      sj = row - sd * L.P - 2;
+    }
+    const double uc = u[s], fs = f[s];
+    const double r = fs - ell_lo(L, [&](int x) { return u[x]; }, s, sd, si, sj, inner || ell_inner(L, si, sj), uc);
+    if (s == id) {
+      if (r64) r64[id] = r;
+      if (r32) r32[id] = (float)r;
+      if (next) next[id] = uc + w * r / L.diag[id];
+    }
+    v = ell_weigh(L, i, j, r * r);
+  }
+  ell_reduce(v, partial, ticket, out, mode, den);
+}
+
+// ---------------------------------------------------------- cluster kernels ----
+// Small coarsest levels (up to CL_NODES nodes [0, n]^2) run inside one
+// thread-block cluster: the nodes' vectors live in registers, stencil operands
+// go through L2 (st / ld.cg) and barrier.cluster replaces kernel boundaries and
+// host round trips.
+constexpr int CL_THREADS = 512, CL_PER = 3, CL_MAX = 8;
+constexpr int CL_NODES = CL_THREADS * CL_PER * CL_MAX;
+
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The reduction of ell_reduce for nodes spread PER a thread: 256-node chunk c
+// holds nodes 256 c .. 256 c + 255, chunk 2 (rank + ctas p) + half for the half
+// of a block's threads and its p-th node.  Every block forms every sum.
+// Two sets of partials alternate: a block that is still adding one set's is passed by no
+// block that would write that set again, since the other set's barrier lies between.
+struct ClDot {
+  double* partial;  // [2][2][CL_NODES / 256]
+  int nchunk;
+  int phase;
+};
+constexpr int CL_PARTIALS = 4 * (CL_NODES / 256);
+template <int N, int PER>
+__device__ __forceinline__ void cl_dots(const double (*v)[PER], ClDot& E, int rank, int ctas, double* sh,
+                                        double* res) {
+  const int tid = threadIdx.x, half = tid >> 8, ht = tid & 255;
+  const ClDot D{E.partial + E.phase * 2 * (CL_NODES / 256), E.nchunk, 0};
+  E.phase ^= 1;
+  const int np = (D.nchunk + 2 * ctas - 1) / (2 * ctas);
+  for (int q = 0; q < N; ++q)
+    for (int p = 0; p < np; ++p) {
+      double x = v[q][0];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    v = threadIdx.x < BS / 32 ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) partial[blockIdx.x] = v;
+      for (int r = 1; r < PER; ++r)
+        if (p == r) x = v[q][r];
+      const double s = ell_sum256(x, sh + 8 * half, ht, [] { __syncthreads(); });
+      const int c = 2 * (rank + ctas * p) + half;
+      if (ht == 0 && c < D.nchunk) __stcg(D.partial + q * (CL_NODES / 256) + c, s);
+      __syncthreads();
+    }
+  cl_sync();
+  for (int q = 0; q < N; ++q) {
+    double a = 0.0;
+    for (int k = ht; k < D.nchunk; k += 256) a += __ldcg(D.partial + q * (CL_NODES / 256) + k);
+    a = ell_sum256(a, sh + 8 * half, ht, [] { __syncthreads(); });
+    if (tid == 0) sh[16] = a;
+    __syncthreads();
+    res[q] = sh[16];
+    __syncthreads();
   }
 }
 
-// Sum of nb partials by one block in a fixed order; optional sqrt and scaling.
-// mode 0: out = sum; 1: out = sqrt(sum); 2: out = sqrt(sum) / *den (res_err).
-__global__ void k_final_sum(const double* __restrict__ partial, int nb, double* __restrict__ out, int mode,
-                            const double* __restrict__ den) {
-  __shared__ double sh[32];
-  double v = 0.0;
-  for (int k = threadIdx.x; k < nb; k += blockDim.x) v += partial[k];
+// A thread's nodes on the level: their stencils' nodes in registers, the edges'
+// coefficients in shared memory (a cluster barrier's acquire empties L1, so they
+// would come from L2 again after each), `own` where the node is no copy.
+template <class T, int PER>
+struct ClNodes {
+  int id[PER], wi[PER], wj[PER], ia[PER][6], ib[PER][6];
+  bool on[PER], own[PER];
+  T h[PER];
+  T* co;  // FP32: K [6][PER * CL_THREADS]; FP64: Ie, len, ped, six each
+  static constexpr int NC = sizeof(T) == 8 ? 18 : 6;
+  static constexpr int SMEM = NC * PER * CL_THREADS * (int)sizeof(T);
+
+  __device__ __forceinline__ void init(const EllLev& L, int rank, int ctas, T* smem) {
+    co = smem;
+    const int m = L.n + 1, N = 10 * m * m, tid = threadIdx.x, NN = (int)L.NN, P = L.P;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    v = threadIdx.x < (int)(blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
+    for (int p = 0; p < PER; ++p) {
+      const int t = CL_THREADS * (rank + ctas * p) + tid;
+      on[p] = t < N;
+      int d = 0, i = 0, j = 0;
+      if (on[p]) decode(L, t, d, i, j, m);
+      wi[p] = i;
+      wj[p] = j;
+      const int k = nidx(L, d, i, j);
+      id[p] = L.nsrc[k];
+      own[p] = on[p] && id[p] == k;
+      if (id[p] != k) {  // a copy stands for its source
+        const int row = id[p] / P;
+        i = id[p] - row * P - 2;
+        d = row / P;
+        j = row - d * P - 2;
+      }
+      const int x = id[p];
+      int slot[6];
+      if (ell_inner(L, i, j)) {
+        const int nbr[6] = {x + 1, x - 1, x - P - 1, x + P + 1, x + P, x - P};
+        const int sl[6] = {RT * NN + x, RT * NN + x - 1, DG * NN + x - P - 1, DG * NN + x, UP * NN + x, UP * NN + x - P};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) {
-      if (mode == 1) v = sqrt(v);
-      if (mode == 2) v = sqrt(v) / *den;
-      *out = v;
+        for (int e = 0; e < 6; ++e) {  // q[b] - q[a]: the node itself (-1) is b of the odd edges, a of the even ones
+          ia[p][e] = (e & 1) ? nbr[e] : -1;
+          ib[p][e] = (e & 1) ? -1 : nbr[e];
+          slot[e] = sl[e];
+        }
+      } else {
+        const int nb = 10 * border_nodes(L.n), b = border_index(L.n, d, i, j);
+#pragma unroll
+        for (int e = 0; e < 6; ++e) {
+          slot[e] = L.bt[(3 * e) * nb + b];
+          const int a_ = L.bt[(3 * e + 1) * nb + b], b_ = L.bt[(3 * e + 2) * nb + b];
+          ia[p][e] = a_ == x ? -1 : a_;
+          ib[p][e] = b_ == x ? -1 : b_;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 6; ++e) coef(L, p, e, slot[e], T(0));
+      h[p] = ell_hinv(L, x, T(0));
     }
+  }
+  __device__ __forceinline__ T& c(int k, int p) { return co[(k * PER + p) * CL_THREADS + threadIdx.x]; }
+  __device__ __forceinline__ void coef(const EllLev& L, int p, int e, int slot, double) {
+    c(e, p) = L.Ie[slot];
+    c(6 + e, p) = L.len[slot];
+    c(12 + e, p) = L.ped[slot];
+  }
+  __device__ __forceinline__ void coef(const EllLev& L, int p, int e, int slot, float) { c(e, p) = L.Kf[slot]; }
+  __device__ __forceinline__ double flux(int p, int e, double dq) { return c(e, p) * dq / c(6 + e, p) * c(12 + e, p); }
+  __device__ __forceinline__ float flux(int p, int e, float dq) { return c(e, p) * dq; }
+  // L(q) at node p, q in memory written by the cluster, x the node's own value
+  __device__ __forceinline__ T lo(const EllLev& L, const T* q, int p, T x) {
+    T va[6], vb[6], f[6];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      va[e] = ia[p][e] < 0 ? x : __ldcg(q + ia[p][e]);
+      vb[e] = ib[p][e] < 0 ? x : __ldcg(q + ib[p][e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 6; ++e) f[e] = flux(p, e, vb[e] - va[e]);
+    const T div = (f[0] - f[1] + f[2] - f[3] + f[4] - f[5]) * h[p];
+    return ell_scale(L, div) - x;
+  }
+  __device__ __forceinline__ double weigh(const EllLev& L, int p, double v) const {
+    return on[p] ? ell_weigh(L, wi[p], wj[p], v) : 0.0;
+  }
+};
+
+// bicgstab (src/lin_solve.f90:361-431) on one level in one launch: the
+// recurrences, the operator and the sums have the operand order of the
+// kernel-by-kernel form, without its six host round trips an iteration.  u:
+// solution in place.  S, Pd: exchange buffers of the level.  nrm > 0 is the
+// right-hand side's norm; else the kernel forms it (1 when 0).  out[0] = error,
+// out[1] = iterations.
+template <int PER>
+__global__ void __launch_bounds__(CL_THREADS, 1)
+    k_ell_bicgstab(EllLev L, double* u, const double* __restrict__ f, double* S, double* Pd, double* partial,
+                   double nrm, double tol, int iter_max, double* out) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  __shared__ double sh[17];
+  unsigned rank, ctas;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+  const int m = L.n + 1, N = 10 * m * m, tid = threadIdx.x;
+  ClDot D{partial, (N + 255) / 256, 0};
+  ClNodes<double, PER> X;
+  X.init(L, rank, ctas, reinterpret_cast<double*>(cl_smem));
+  double U[PER], R[PER], R0[PER], P[PER], AP[PER], s[PER], AS[PER];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) U[p] = R[p] = R0[p] = P[p] = AP[p] = s[p] = AS[p] = 0.0;
+  double v[2][PER], res[2];
+  if (!(nrm > 0.0)) {
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const double x = X.on[p] ? f[X.id[p]] : 0.0;
+      v[0][p] = X.weigh(L, p, x * x);
+    }
+    cl_dots<1, PER>(v, D, rank, ctas, sh, res);
+    nrm = sqrt(res[0]);
+    if (nrm == 0.0) nrm = 1.0;
+  }
+#pragma unroll
+  for (int p = 0; p < PER; ++p)
+    if (X.on[p]) {
+      U[p] = u[X.id[p]];
+      R[p] = f[X.id[p]] - X.lo(L, u, p, U[p]);
+      R0[p] = P[p] = R[p];
+      if (X.own[p]) __stcg(Pd + X.id[p], P[p]);
+    }
+  cl_sync();
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    if (X.on[p]) AP[p] = X.lo(L, Pd, p, P[p]);
+    v[0][p] = X.weigh(L, p, R0[p] * R[p]);
+    v[1][p] = X.weigh(L, p, AP[p] * R0[p]);
+  }
+  cl_dots<2, PER>(v, D, rank, ctas, sh, res);
+  double rho = res[0], apr = res[1], err = 0.0;
+  int iter;
+  for (iter = 1; iter <= iter_max; ++iter) {
+    const double alph = rho / apr;
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      s[p] = 1.0 * R[p] + -alph * AP[p];
+      if (X.own[p]) __stcg(S + X.id[p], s[p]);
+    }
+    cl_sync();
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      if (X.on[p]) AS[p] = X.lo(L, S, p, s[p]);
+      v[0][p] = X.weigh(L, p, AS[p] * s[p]);
+      v[1][p] = X.weigh(L, p, AS[p] * AS[p]);
+    }
+    cl_dots<2, PER>(v, D, rank, ctas, sh, res);
+    const double omga = res[0] / res[1];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const double cc = alph * P[p] + omga * s[p];
+      U[p] = 1.0 * U[p] + 1.0 * cc;
+      R[p] = 1.0 * s[p] + -omga * AS[p];
+      v[0][p] = X.weigh(L, p, R[p] * R[p]);
+      v[1][p] = X.weigh(L, p, R0[p] * R[p]);
+    }
+    cl_dots<2, PER>(v, D, rank, ctas, sh, res);
+    err = sqrt(res[0]) / nrm;
+    if (err <= tol) break;
+    const double rho_old = rho;
+    rho = res[1];
+    const double b = (alph / omga) * (rho / rho_old);
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const double cc = 1.0 * P[p] + -omga * AP[p];
+      P[p] = 1.0 * R[p] + b * cc;
+      if (X.own[p]) __stcg(Pd + X.id[p], P[p]);
+    }
+    cl_sync();
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      if (X.on[p]) AP[p] = X.lo(L, Pd, p, P[p]);
+      v[0][p] = X.weigh(L, p, AP[p] * R0[p]);
+    }
+    cl_dots<1, PER>(v, D, rank, ctas, sh, res);
+    apr = res[0];
+  }
+#pragma unroll
+  for (int p = 0; p < PER; ++p)
+    if (X.own[p]) u[X.id[p]] = U[p];
+  if (rank == 0 && tid == 0 && out) {
+    out[0] = err;
+    out[1] = (double)iter;
+  }
+  cl_sync();
+}
+
+// `sweeps` Jacobi sweeps (w = 1) from a zero guess on one level in one launch;
+// a, b: ping-pong exchange buffers, the result ends in a.
+template <class T, int PER>
+__global__ void __launch_bounds__(CL_THREADS, 1)
+    k_ell_coarse_jacobi(EllLev L, const T* __restrict__ f, T* a, T* b, int sweeps) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  unsigned rank, ctas;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+  ClNodes<T, PER> X;
+  X.init(L, rank, ctas, reinterpret_cast<T*>(cl_smem));
+  T x[PER], rhs[PER], dg[PER];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    x[p] = T(0);
+    rhs[p] = X.own[p] ? f[X.id[p]] : T(0);
+    dg[p] = X.own[p] ? ell_diag(L, X.id[p], T(0)) : T(1);
+  }
+  for (int k = 0; k < sweeps; ++k) {
+    T* to = ((sweeps - 1 - k) & 1) ? b : a;
+    const T* from = ((sweeps - 1 - k) & 1) ? a : b;
+#pragma unroll
+    for (int p = 0; p < PER; ++p)
+      if (X.own[p]) {
+        const T lq = k ? X.lo(L, from, p, x[p]) : T(0);
+        x[p] = x[p] + T(1) * (rhs[p] - lq) / dg[p];
+        __stcg(to + X.id[p], x[p]);
+      }
+    cl_sync();
   }
 }
 
 // ------------------------------------------------------------- wavelets ----
-__device__ __forceinline__ double rdw(const EllLev& L, const double* __restrict__ f, int d, int i, int j) {
-  if (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1) return 0.0;
+// Reads of a level field and of its overlap areas at (i, j); DIR: the slot is an
+// owned node, read directly, else through the remap (0 outside the array).
+template <bool DIR, class T>
+__device__ __forceinline__ T rdw(const EllLev& L, const T* f, int d, int i, int j) {
+  if (DIR) return f[nidx(L, d, i, j)];
+  if (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1) return T(0);
   return f[L.nsrc[nidx(L, d, i, j)]];
 }
-__device__ __forceinline__ double oaw(const EllLev& L, int d, int i, int j, int k) {
-  if (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1) return 0.0;
-  return L.oa[(int64_t)(k - 1) * L.NN + nidx(L, d, i, j)];
+__device__ __forceinline__ double ell_oa(const EllLev& L, int slot, double) { return L.oa[slot]; }
+__device__ __forceinline__ float ell_oa(const EllLev& L, int slot, float) { return L.oaf[slot]; }
+template <bool DIR, class T>
+__device__ __forceinline__ T oaw(const EllLev& L, int d, int i, int j, int k) {
+  if (!DIR && (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1)) return T(0);
+  return ell_oa(L, (k - 1) * (int)L.NN + nidx(L, d, i, j), T(0));
+}
+// Parents whose interscale stencils (children 2 i - 2 .. 2 i + 2) read owned
+// child nodes only.
+__device__ __forceinline__ bool par_inner(const EllLev& C, int ip, int jp) {
+  return ip >= 1 && jp >= 1 && ip <= C.n - 2 && jp <= C.n - 2;
 }
 // Interp_node (src/wavelet.f90:1487)
-__device__ __forceinline__ double interp_node(const EllLev& F, const double* s, int d, int i, int j, int i1, int j1, int i2,
-                                              int j2, int i3, int j3, int i4, int j4) {
-  return (oaw(F, d, i, j, 1) * rdw(F, s, d, i1, j1) + oaw(F, d, i, j, 2) * rdw(F, s, d, i2, j2) +
-          oaw(F, d, i, j, 3) * rdw(F, s, d, i3, j3) + oaw(F, d, i, j, 4) * rdw(F, s, d, i4, j4)) *
-         F.hinv[nidx(F, d, i, j)];
+template <bool DIR, class T>
+__device__ __forceinline__ T interp_node(const EllLev& F, const T* s, int d, int i, int j, int i1, int j1, int i2, int j2,
+                                         int i3, int j3, int i4, int j4) {
+  return (oaw<DIR, T>(F, d, i, j, 1) * rdw<DIR>(F, s, d, i1, j1) + oaw<DIR, T>(F, d, i, j, 2) * rdw<DIR>(F, s, d, i2, j2) +
+          oaw<DIR, T>(F, d, i, j, 3) * rdw<DIR>(F, s, d, i3, j3) + oaw<DIR, T>(F, d, i, j, 4) * rdw<DIR>(F, s, d, i4, j4)) *
+         ell_hinv(F, nidx(F, d, i, j), T(0));
 }
 
 // Compute_scalar_wavelets (src/wavelet.f90:642) for parents [0, n_c)^2.
-__global__ void k_wc_compute(EllLev C, EllLev F, const double* __restrict__ s, double* __restrict__ wc) {
+template <bool DIR, class T>
+__device__ __forceinline__ void wc_parent(const EllLev& F, const T* __restrict__ s, T* __restrict__ wc, int d, int ip,
+                                          int jp) {
+  const int i = 2 * ip, j = 2 * jp;
+  wc[nidx(F, d, i + 1, j)] =
+      rdw<DIR>(F, s, d, i + 1, j) - interp_node<DIR>(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2);
+  wc[nidx(F, d, i + 1, j + 1)] = rdw<DIR>(F, s, d, i + 1, j + 1) -
+                                 interp_node<DIR>(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2);
+  wc[nidx(F, d, i, j + 1)] =
+      rdw<DIR>(F, s, d, i, j + 1) - interp_node<DIR>(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2);
+}
+template <class T>
+__global__ void __launch_bounds__(256) k_wc_compute(EllLev C, EllLev F, const T* __restrict__ s, T* __restrict__ wc) {
   const int m = C.n;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 10 * m * m) return;
   int d, ip, jp;
   decode(C, t, d, ip, jp, m);
-  const int i = 2 * ip, j = 2 * jp;
-  wc[nidx(F, d, i + 1, j)] = rdw(F, s, d, i + 1, j) - interp_node(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2);
-  wc[nidx(F, d, i + 1, j + 1)] =
-      rdw(F, s, d, i + 1, j + 1) - interp_node(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2);
-  wc[nidx(F, d, i, j + 1)] = rdw(F, s, d, i, j + 1) - interp_node(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2);
+  if (par_inner(C, ip, jp)) wc_parent<true>(F, s, wc, d, ip, jp);
+  else wc_parent<false>(F, s, wc, d, ip, jp);
 }
+
+#define W(a, b, k) (rdw<DIR>(F, wc, d, i + (a), j + (b)) * oaw<DIR, T>(F, d, i + (a), j + (b), k))
+template <bool DIR, class T>
+__device__ __forceinline__ T restrict_sum(const EllLev& F, const T* __restrict__ wc, int d, int i, int j) {
+  return W(1, 0, 1) + W(1, 1, 2) + W(2, 1, 3) + W(1, 2, 4) + W(0, 1, 1) + W(-1, 0, 2) + W(-1, 1, 3) +
+         W(-2, -1, 4) + W(-1, -1, 1) + W(0, -1, 2) + W(-1, -2, 3) + W(1, -1, 4);
+}
+template <bool DIR, class T>
+__device__ __forceinline__ T prolong_sum(const EllLev& F, const T* __restrict__ wc, int d, int i, int j) {
+  return W(1, 0, 1) + W(1, 1, 2) + W(2, 1, 3) + W(0, 1, 1) + W(-1, 0, 2) + W(-1, 1, 3) + W(-2, -1, 4) +
+         W(-1, -1, 1) + W(0, -1, 2) + W(-1, -2, 3) + W(1, -1, 4);
+}
+#undef W
 
 // Restrict_scalar (src/wavelet.f90:520) for parents [0, n_c]^2 (the +1 row
 // includes the pole copies); ghost parents that are copies are skipped.
-__global__ void k_restrict(EllLev C, EllLev F, const double* __restrict__ sf, const double* __restrict__ wc,
-                           double* __restrict__ sc) {
+template <class T>
+__global__ void __launch_bounds__(256) k_restrict(EllLev C, EllLev F, const T* __restrict__ sf,
+                                                  const T* __restrict__ wc, T* __restrict__ sc) {
   const int m = C.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 10 * m * m) return;
   int d, ip, jp;
   decode(C, t, d, ip, jp, m);
-  const int64_t kp = nidx(C, d, ip, jp);
-  if (C.nsrc[kp] != kp) return;
+  const int kp = nidx(C, d, ip, jp);
+  const bool in = par_inner(C, ip, jp);
+  if (!in && C.nsrc[kp] != kp) return;
   const int i = 2 * ip, j = 2 * jp;
-#define W(a, b, k) (rdw(F, wc, d, i + (a), j + (b)) * oaw(F, d, i + (a), j + (b), k))
-  const double sum = W(1, 0, 1) + W(1, 1, 2) + W(2, 1, 3) + W(1, 2, 4) + W(0, 1, 1) + W(-1, 0, 2) + W(-1, 1, 3) +
-                     W(-2, -1, 4) + W(-1, -1, 1) + W(0, -1, 2) + W(-1, -2, 3) + W(1, -1, 4);
-  sc[kp] = sf[nidx(F, d, i, j)] + sum * C.hinv[kp];
+  const T sum = in ? restrict_sum<true>(F, wc, d, i, j) : restrict_sum<false>(F, wc, d, i, j);
+  sc[kp] = sf[nidx(F, d, i, j)] + sum * ell_hinv(C, kp, T(0));
 }
 
 // Prolong_scalar (src/wavelet.f90:571; eleven terms, as in the reference) for
 // the children (2i, 2j) of parents [0, n_c]^2 that are not copies.
-__global__ void k_prolong_even(EllLev C, EllLev F, const double* __restrict__ sc, const double* __restrict__ wc,
-                               double* __restrict__ sf) {
+__global__ void __launch_bounds__(256) k_prolong_even(EllLev C, EllLev F, const double* __restrict__ sc,
+                                                      const double* __restrict__ wc, double* __restrict__ sf) {
   const int m = C.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 10 * m * m) return;
   int d, ip, jp;
   decode(C, t, d, ip, jp, m);
   const int i = 2 * ip, j = 2 * jp;
-  const int64_t kc = nidx(F, d, i, j);
-  if (F.nsrc[kc] != kc) return;
-  const int64_t kp = nidx(C, d, ip, jp);
-  const double sum = W(1, 0, 1) + W(1, 1, 2) + W(2, 1, 3) + W(0, 1, 1) + W(-1, 0, 2) + W(-1, 1, 3) + W(-2, -1, 4) +
-                     W(-1, -1, 1) + W(0, -1, 2) + W(-1, -2, 3) + W(1, -1, 4);
-#undef W
-  sf[kc] = sc[C.nsrc[kp]] - sum * C.hinv[kp];
+  const int kc = nidx(F, d, i, j), kp = nidx(C, d, ip, jp);
+  const bool in = par_inner(C, ip, jp);
+  if (!in && F.nsrc[kc] != kc) return;
+  const double sum = in ? prolong_sum<true>(F, wc, d, i, j) : prolong_sum<false>(F, wc, d, i, j);
+  sf[kc] = sc[in ? kp : C.nsrc[kp]] - sum * C.hinv[kp];
 }
 
 // Reconstruct_scalar (src/wavelet.f90:614) for parents [0, n_c)^2.
-__global__ void k_prolong_odd(EllLev C, EllLev F, double* __restrict__ s, const double* __restrict__ wc) {
-  const int m = C.n;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 10 * m * m) return;
-  int d, ip, jp;
-  decode(C, t, d, ip, jp, m);
+template <bool DIR>
+__device__ __forceinline__ void odd_parent(const EllLev& F, double* __restrict__ s, const double* __restrict__ wc, int d,
+                                           int ip, int jp) {
   const int i = 2 * ip, j = 2 * jp;
-  double a = interp_node(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2) + rdw(F, wc, d, i + 1, j);
-  double b = interp_node(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2) + rdw(F, wc, d, i + 1, j + 1);
-  double c = interp_node(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2) + rdw(F, wc, d, i, j + 1);
+  const double a = interp_node<DIR>(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2) +
+                   rdw<DIR>(F, wc, d, i + 1, j);
+  const double b = interp_node<DIR>(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2) +
+                   rdw<DIR>(F, wc, d, i + 1, j + 1);
+  const double c = interp_node<DIR>(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2) +
+                   rdw<DIR>(F, wc, d, i, j + 1);
   s[nidx(F, d, i + 1, j)] = a;
   s[nidx(F, d, i + 1, j + 1)] = b;
   s[nidx(F, d, i, j + 1)] = c;
 }
-
-// ------------------------------------------------ FP32 (mixed precision) ----
-// Same operator with per-edge coefficients K = cf*interp(csq)*pedlen/len in
-// FP32: L(q) = hinv * sum(+-K (q_b - q_a)) - q.  Used only inside the FP32
-// V-cycles of the mixed-precision solver; the outer residual stays FP64.
-__device__ __forceinline__ float flux32(const EllLev& L, const float* __restrict__ q, int64_t slot) {
-  const int code = L.esrc[slot];
-  const int64_t src = code >> 1;
-  const int e = (int)(src / L.NN);
-  const int64_t node = src - (int64_t)e * L.NN;
-  const float q0 = q[L.nsrc[node]];
-  float f;
-  if (e == RT) f = L.Kf[src] * (q[L.nsrc[node + 1]] - q0);
-  else if (e == DG) f = L.Kf[src] * (q0 - q[L.nsrc[node + L.P + 1]]);
-  else f = L.Kf[src] * (q[L.nsrc[node + L.P]] - q0);
-  return (code & 1) ? -f : f;
+__global__ void __launch_bounds__(256) k_prolong_odd(EllLev C, EllLev F, double* __restrict__ s,
+                                                     const double* __restrict__ wc) {
+  const int m = C.n;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 10 * m * m) return;
+  int d, ip, jp;
+  decode(C, t, d, ip, jp, m);
+  if (par_inner(C, ip, jp)) odd_parent<true>(F, s, wc, d, ip, jp);
+  else odd_parent<false>(F, s, wc, d, ip, jp);
 }
 
-template <int OP>
-__global__ void k_ell_op32(EllLev L, const float* __restrict__ q, const float* __restrict__ f, float* __restrict__ out,
-                           float w) {
-  const int m = L.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+// Inverse transform with zero wavelets (Prolong_scalar and Reconstruct_scalar of
+// a correction) from sc into level F, in one pass over the fine nodes: even
+// children take their parent's value, odd ones interpolate the even values,
+// which are read from their parents.  add: dst += the interpolation, else dst =
+// it.  The even, odd and add passes it replaces wrote and read the interpolated
+// level twice.
+template <bool DIR, class T>
+__device__ __forceinline__ T even_value(const EllLev& C, const EllLev& F, const T* __restrict__ sc, int d, int i, int j) {
+  if (DIR) return sc[nidx(C, d, i >> 1, j >> 1)];
+  if (i < -2 || j < -2 || i > F.n + 1 || j > F.n + 1) return T(0);
+  const int k = F.nsrc[nidx(F, d, i, j)];  // the even node's owner and its parent
+  const int row = k / F.P, fi = k - row * F.P - 2, fd = row / F.P, fj = row - fd * F.P - 2;
+  return sc[C.nsrc[nidx(C, fd, fi >> 1, fj >> 1)]];
+}
+template <bool DIR, class T>
+__device__ __forceinline__ T fine_value(const EllLev& C, const EllLev& F, const T* __restrict__ sc, int d, int i, int j,
+                                        int id) {
+  const int pi = i & 1, pj = j & 1;
+  if (!pi && !pj) return even_value<DIR>(C, F, sc, d, i, j);
+  const int i0 = i - pi, j0 = j - pj;  // the parent's child
+  auto E = [&](int a, int b) { return even_value<DIR>(C, F, sc, d, a, b); };
+  T v1, v2, v3, v4;
+  if (pi && !pj) {
+    v1 = E(i0, j0); v2 = E(i0 + 2, j0); v3 = E(i0 + 2, j0 + 2); v4 = E(i0, j0 - 2);
+  } else if (pi) {
+    v1 = E(i0 + 2, j0 + 2); v2 = E(i0, j0); v3 = E(i0 + 2, j0); v4 = E(i0, j0 + 2);
+  } else {
+    v1 = E(i0, j0); v2 = E(i0, j0 + 2); v3 = E(i0 - 2, j0); v4 = E(i0 + 2, j0 + 2);
+  }
+  return (oaw<DIR, T>(F, d, i, j, 1) * v1 + oaw<DIR, T>(F, d, i, j, 2) * v2 + oaw<DIR, T>(F, d, i, j, 3) * v3 +
+          oaw<DIR, T>(F, d, i, j, 4) * v4) * ell_hinv(F, id, T(0));
+}
+template <class T>
+__global__ void __launch_bounds__(256) k_interp(EllLev C, EllLev F, const T* __restrict__ sc, T* __restrict__ dst,
+                                                int add) {
+  const int m = F.n + 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 10 * m * m) return;
   int d, i, j;
-  decode(L, t, d, i, j, m);
-  const int64_t id = nidx(L, d, i, j);
-  if (L.nsrc[id] != id) return;
-  const int64_t NN = L.NN, P = L.P;
-  const float div = (flux32(L, q, RT * NN + id) - flux32(L, q, RT * NN + id - 1) + flux32(L, q, DG * NN + id - P - 1) -
-                     flux32(L, q, DG * NN + id) + flux32(L, q, UP * NN + id) - flux32(L, q, UP * NN + id - P)) *
-                    L.hinvf[id];
-  const float lq = div - q[id];
-  if (OP == OP_APPLY) out[id] = lq;
-  if (OP == OP_RESID) out[id] = f[id] - lq;
-  if (OP == OP_JACOBI) out[id] = q[id] + w * (f[id] - lq) / L.diagf[id];
+  decode(F, t, d, i, j, m);
+  const int id = nidx(F, d, i, j);
+  const bool in = par_inner(C, i >> 1, j >> 1);
+  if (!in && F.nsrc[id] != id) return;
+  const T v = in ? fine_value<true>(C, F, sc, d, i, j, id) : fine_value<false>(C, F, sc, d, i, j, id);
+  dst[id] = add ? T(1) * dst[id] + T(1) * v : v;
 }
 
 // Operator coefficients of elliptic_lo and elliptic_lo_diag from the old free

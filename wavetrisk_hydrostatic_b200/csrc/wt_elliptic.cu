@@ -37,8 +37,8 @@ struct ELevelDev {
   int level = 0, n = 0, P = 0, nd = 1;
   int64_t NN = 0;
   double *Ie = nullptr, *diag = nullptr;
-  int *nsrc = nullptr, *esrc = nullptr;
-  float *Kf = nullptr, *hinvf = nullptr, *diagf = nullptr;
+  int *nsrc = nullptr, *esrc = nullptr, *bt = nullptr;
+  float *Kf = nullptr, *hinvf = nullptr, *diagf = nullptr, *oaf = nullptr;
 };
 
 struct Ell {
@@ -47,12 +47,14 @@ struct Ell {
   double dt = 0, th1 = 1, th2 = 1, cf = 0;
   int domain_level = 2;
   std::vector<ELevelDev> L;
-  MField u, f, res, corr, pf, wc_mass, wc_temp, tmp, au, rr, r0, pp, ss, ap, as_, cc, rr2;
+  MField u, f, res, corr, wc_temp, tmp, au, rr, r0, pp, ss, ap, as_, cc;
   MField eta_wc;                   // the free surface's wavelets of its last WT_after_step
   bool eta_wc_valid = false;
   MField u32, f32, r32, c32, t32;  // FP32 V-cycle work
   double* partial = nullptr;
-  double* scal = nullptr;  // device scalars
+  unsigned* ticket = nullptr;  // arrivals of a reduction's blocks (0 between launches)
+  double* clpart = nullptr;    // partial sums of the cluster kernels
+  double* scal = nullptr;      // device scalars
   cudaGraphExec_t cycle_exec[2] = {nullptr, nullptr};  // captured correction cycles (FP32, FP64)
   int cycle_key[2] = {-1, -1};
   std::vector<const void*> cycle_ptrs[2];  // rotating() at each cycle graph's capture
@@ -63,8 +65,9 @@ struct Ell {
   EllLev view(int l) const {
     const DevLevel& D = const_cast<wt_handle*>(h)->at(l);
     const ELevelDev& E = L[l - ls];
+    const auto magic = [](int m) { return ((1ull << 40) + m - 1) / m; };
     return EllLev{D.n, D.P, E.nd, D.NN, D.len, D.pedlen, D.hex_inv, D.overl_a, E.Ie, E.diag, E.nsrc, E.esrc,
-                  E.Kf, E.hinvf, E.diagf};
+                  E.Kf, E.hinvf, E.diagf, E.oaf, E.bt, cf, magic(D.n + 1), magic(D.n)};
   }
   int m(int l) const { return L[l - ls].n + 1; }
   cudaStream_t s() const { return h->stream; }
@@ -149,6 +152,13 @@ int alloc_field(Ell& E, MField& F, bool fp32 = false) {
 // ---------------------------------------------------------------- setup ----
 void lp_release(void* p);
 
+namespace {
+__global__ void k_d2f(int64_t n, const double* __restrict__ a, float* __restrict__ b) {
+  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) b[t] = (float)a[t];
+}
+}  // namespace
+
 static void ell_free(Ell* E) {
   if (!E) return;
   lp_release(E->lp);
@@ -231,18 +241,26 @@ extern "C" int wt_elliptic_setup(wt_handle* h, double dt, double theta1, double 
     cudaMemcpy(X.Kf, Kf.data(), 4 * 3 * NN, cudaMemcpyHostToDevice);
     cudaMemcpy(X.hinvf, hinvf.data(), 4 * NN, cudaMemcpyHostToDevice);
     cudaMemcpy(X.diagf, diagf.data(), 4 * NN, cudaMemcpyHostToDevice);
+    if ((rc = dalloc(*E, &X.oaf, 4 * NN))) break;
+    k_d2f<<<nb(4 * NN), TPB>>>(4 * NN, D.overl_a, X.oaf);
+    if ((rc = dalloc(*E, &X.bt, 18 * 10 * (int64_t)border_nodes(D.n)))) break;
+    k_ell_border<<<nb(10 * (int64_t)(D.n + 1) * (D.n + 1)), TPB>>>(D.n, D.P, (int)NN, D.nsrc, D.esrc, X.bt);
     E->L.push_back(X);
     E->nbmax = std::max<int>(E->nbmax, (int)nb(10 * (int64_t)(D.n + 1) * (D.n + 1)));
   }
-  MField* fields[] = {&E->u, &E->f, &E->res, &E->corr, &E->pf, &E->wc_mass, &E->wc_temp, &E->tmp, &E->au,
-                      &E->rr, &E->r0, &E->pp, &E->ss, &E->ap, &E->as_, &E->cc, &E->rr2, &E->eta_wc};
+  MField* fields[] = {&E->u, &E->f, &E->res, &E->corr, &E->wc_temp, &E->tmp, &E->au,
+                      &E->rr, &E->r0, &E->pp, &E->ss, &E->ap, &E->as_, &E->cc, &E->eta_wc};
   for (MField* F : fields)
     if (rc == WT_OK) rc = alloc_field(*E, *F);
   MField* f32[] = {&E->u32, &E->f32, &E->r32, &E->c32, &E->t32};
   for (MField* F : f32)
     if (rc == WT_OK) rc = alloc_field(*E, *F, true);
   if (rc == WT_OK) rc = dalloc(*E, &E->partial, E->nbmax);
+  if (rc == WT_OK) rc = dalloc(*E, &E->ticket, 1);
+  if (rc == WT_OK) rc = dalloc(*E, &E->clpart, CL_PARTIALS);
   if (rc == WT_OK) rc = dalloc(*E, &E->scal, 64);
+  // the set-up ran on the default stream, which the handle's stream does not wait for
+  if (rc == WT_OK && cudaDeviceSynchronize() != cudaSuccess) rc = wt_handle_fail("elliptic setup", cudaGetLastError());
   if (rc != WT_OK) {
     ell_free(E);
     return rc;
@@ -257,17 +275,17 @@ namespace {
 void op(Ell& E, int OPK, int l, const double* q, const double* f, double* out, double w = 1.0) {
   EllLev V = E.view(l);
   unsigned g = nb(10 * E.m(l) * E.m(l));
-  if (OPK == OP_APPLY) k_ell_op<OP_APPLY><<<g, TPB, 0, E.s()>>>(V, E.cf, q, f, out, w);
-  if (OPK == OP_RESID) k_ell_op<OP_RESID><<<g, TPB, 0, E.s()>>>(V, E.cf, q, f, out, w);
-  if (OPK == OP_JACOBI) k_ell_op<OP_JACOBI><<<g, TPB, 0, E.s()>>>(V, E.cf, q, f, out, w);
+  if (OPK == OP_APPLY) k_ell_op<OP_APPLY, double><<<g, TPB, 0, E.s()>>>(V, q, f, out, w, nullptr);
+  if (OPK == OP_RESID) k_ell_op<OP_RESID, double><<<g, TPB, 0, E.s()>>>(V, q, f, out, w, nullptr);
+  if (OPK == OP_JACOBI) k_ell_op<OP_JACOBI, double><<<g, TPB, 0, E.s()>>>(V, q, f, out, w, nullptr);
 }
 
-// weighted dot / l2 into device scalar slot; returns nothing (async)
+// weighted dot / l2 into a device scalar; returns nothing (async)
+void dot_to(Ell& E, int l, const double* a, const double* b, double* out, int mode, const double* den = nullptr) {
+  k_ell_dot<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), a, b, E.partial, E.ticket, out, mode, den);
+}
 void dot_dev(Ell& E, int l, const double* a, const double* b, int slot, int mode, const double* den = nullptr) {
-  EllLev V = E.view(l);
-  unsigned g = nb(10 * E.m(l) * E.m(l));
-  k_ell_dot<TPB><<<g, TPB, 0, E.s()>>>(V, a, b, E.partial);
-  k_final_sum<<<1, 256, 0, E.s()>>>(E.partial, (int)g, E.scal + slot, mode, den);
+  dot_to(E, l, a, b, E.scal + slot, mode, den);
 }
 
 double fetch(Ell& E, int slot) {
@@ -304,35 +322,84 @@ void jacobi(Ell& E, MField& u, MField& f, int l, int iters, double w = 1.0) {
   }
 }
 
+// `iters` sweeps (w = 1) from a zero guess: u need not hold anything.
+void jacobi_zero(Ell& E, MField& u, MField& f, int l, int iters) {
+  const int q = l - E.ls;
+  if (iters < 1) {
+    zero_level(E, l, u.lv[q]);
+    return;
+  }
+  k_ell_first2<double><<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), f.lv[q], u.lv[q], iters > 1);
+  jacobi(E, u, f, l, iters - 2);
+}
+
 void residual(Ell& E, MField& f, MField& u, int l, MField& r) {
   op(E, OP_RESID, l, u.lv[l - E.ls], f.lv[l - E.ls], r.lv[l - E.ls]);
 }
 
-// forward_scalar_transform(s, wc, c, c+1): wavelets at c+1, lifted restriction to c
+// forward_scalar_transform(s, wc, c, c+1): wavelets at c+1, lifted restriction to
+// c.  Every child slot the restriction reads is an odd node of [0, n)^2, which
+// the wavelet pass writes; the rest of wc stays as it is.
 void restrict_level(Ell& E, MField& s, MField& wc, int c) {
-  for (int l = E.ls; l <= E.le; ++l) zero_level(E, l, wc.lv[l - E.ls]);   // zero_float(wavelet)
   EllLev C = E.view(c), F = E.view(c + 1);
   int n = E.L[c - E.ls].n;
-  k_wc_compute<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, s.lv[c + 1 - E.ls], wc.lv[c + 1 - E.ls]);
-  k_restrict<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, s.lv[c + 1 - E.ls], wc.lv[c + 1 - E.ls],
-                                                              s.lv[c - E.ls]);
+  k_wc_compute<double><<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, s.lv[c + 1 - E.ls], wc.lv[c + 1 - E.ls]);
+  k_restrict<double><<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, s.lv[c + 1 - E.ls], wc.lv[c + 1 - E.ls],
+                                                                     s.lv[c - E.ls]);
 }
 
-// inverse_scalar_transform(wc, s, f-1, f)
-void prolong_level(Ell& E, MField& wc, MField& s, int fl) {
-  int c = fl - 1;
-  EllLev C = E.view(c), F = E.view(fl);
-  int n = E.L[c - E.ls].n;
-  k_prolong_even<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, s.lv[c - E.ls], wc.lv[fl - E.ls], s.lv[fl - E.ls]);
-  k_prolong_odd<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, s.lv[fl - E.ls], wc.lv[fl - E.ls]);
+// inverse_scalar_transform(zero wavelets, s, fl-1, fl): src of level fl-1 into
+// dst of level fl, added to it or in its place
+void interp_level(Ell& E, int fl, const double* src, double* dst, bool add) {
+  k_interp<double><<<nb(10 * E.m(fl) * E.m(fl)), TPB, 0, E.s()>>>(E.view(fl - 1), E.view(fl), src, dst, add ? 1 : 0);
 }
 
+// |f - L u| / nrm on the device (residual and norm in one pass), to the host
 double res_err(Ell& E, MField& f, MField& u, double nrm_f, int l) {
-  residual(E, f, u, l, E.rr2);
-  return l2(E, l, E.rr2.lv[l - E.ls]) / nrm_f;
+  const int q = l - E.ls;
+  k_ell_resid_norm<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), u.lv[q], f.lv[q], nullptr, nullptr, nullptr,
+                                                                0.0, E.partial, E.ticket, E.scal, 1, nullptr);
+  return fetch(E, 0) / nrm_f;
 }
 
-// bicgstab (src/lin_solve.f90:361-431) at level l
+// Launch of a cluster kernel over one level: CTAs for its nodes [0, n]^2, per a
+// thread, all in one cluster.
+template <class... P, class... A>
+cudaError_t cluster_launch(Ell& E, int l, int per, int smem, void (*k)(P...), A... a) {
+  const int N = 10 * E.m(l) * E.m(l);
+  const unsigned ctas = nb(N, CL_THREADS * per);
+  if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(CL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = E.s();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+}
+// Levels small enough for one cluster's registers (up to J5: 10890 nodes); one
+// node a thread up to J4 (2890), so that each phase is one round of loads.
+bool cluster_level(const Ell& E, int l) { return 10 * E.m(l) * E.m(l) <= CL_NODES; }
+bool cluster_one(const Ell& E, int l) { return 10 * E.m(l) * E.m(l) <= CL_THREADS * CL_MAX; }
+
+// The coarsest level's Jacobi sweeps from a zero guess (cluster levels).
+template <class T>
+void coarse_jacobi(Ell& E, const T* f, T* a, T* b, int sweeps) {
+  if (cluster_one(E, E.ls))
+    cluster_launch(E, E.ls, 1, ClNodes<T, 1>::SMEM, k_ell_coarse_jacobi<T, 1>, E.view(E.ls), f, a, b, sweeps);
+  else
+    cluster_launch(E, E.ls, CL_PER, ClNodes<T, CL_PER>::SMEM, k_ell_coarse_jacobi<T, CL_PER>, E.view(E.ls), f, a, b,
+                   sweeps);
+}
+
+// bicgstab (src/lin_solve.f90:361-431) at level l.  nrm_f 0: the norm of f.
+// Small levels run in one cluster launch; J4, 40 iterations: ~100 us an iteration
+// of launches and host round trips became one launch.
 void bicgstab(Ell& E, MField& u, MField& f, double nrm_f, int l, double tol, int iter_max, double* err_out,
               int* iter_out) {
   const int q = l - E.ls;
@@ -340,6 +407,24 @@ void bicgstab(Ell& E, MField& u, MField& f, double nrm_f, int l, double tol, int
   double* F = f.lv[q];
   double *R = E.rr.lv[q], *R0 = E.r0.lv[q], *Pp = E.pp.lv[q], *S = E.ss.lv[q], *AP = E.ap.lv[q], *AS = E.as_.lv[q],
          *CC = E.cc.lv[q];
+  if (cluster_level(E, l)) {
+    if (cluster_one(E, l))
+      cluster_launch(E, l, 1, ClNodes<double, 1>::SMEM, k_ell_bicgstab<1>, E.view(l), U, F, S, Pp, E.clpart, nrm_f, tol,
+                     iter_max, E.scal + 4);
+    else
+      cluster_launch(E, l, CL_PER, ClNodes<double, CL_PER>::SMEM, k_ell_bicgstab<CL_PER>, E.view(l), U, F, S, Pp,
+                     E.clpart, nrm_f, tol, iter_max, E.scal + 4);
+    if (err_out || iter_out) {
+      double two[2];
+      cudaMemcpyAsync(two, E.scal + 4, 16, cudaMemcpyDeviceToHost, E.s());
+      cudaStreamSynchronize(E.s());
+      if (err_out) *err_out = two[0];
+      if (iter_out) *iter_out = (int)two[1];
+    }
+    return;
+  }
+  if (!(nrm_f > 0.0)) nrm_f = l2(E, l, F);
+  if (nrm_f == 0.0) nrm_f = 1.0;
   zero_level(E, l, CC);
   op(E, OP_RESID, l, U, F, R);
   copy_level(E, l, R0, R);
@@ -375,23 +460,18 @@ void bicgstab(Ell& E, MField& u, MField& f, double nrm_f, int l, double tol, int
 }
 
 void v_cycle(Ell& E, const wt_solver_opts& o, MField& u, MField& f, int l, double nrmf, wt_solver_report& rep) {
-  for (int j = E.ls; j <= l; ++j) zero_level(E, j, E.corr.lv[j - E.ls]);
   residual(E, f, u, l, E.res);
   for (int j = l; j >= E.ls + 1; --j) {
-    jacobi(E, E.corr, E.res, j, o.down_iter);
+    jacobi_zero(E, E.corr, E.res, j, o.down_iter);
     op(E, OP_RESID, j, E.corr.lv[j - E.ls], E.res.lv[j - E.ls], E.au.lv[j - E.ls]);
     std::swap(E.res.lv[j - E.ls], E.au.lv[j - E.ls]);
     restrict_level(E, E.res, E.wc_temp, j - 1);
   }
   int j = E.ls;
-  double nrm_rhs = l2(E, j, E.res.lv[0]);
-  if (nrm_rhs == 0.0) nrm_rhs = 1.0;
-  bicgstab(E, E.corr, E.res, nrm_rhs, j, o.coarse_tol, o.coarse_iter, nullptr, nullptr);
+  zero_level(E, j, E.corr.lv[0]);
+  bicgstab(E, E.corr, E.res, 0.0, j, o.coarse_tol, o.coarse_iter, nullptr, nullptr);
   for (j = E.ls + 1; j <= l; ++j) {
-    zero_level(E, j, E.wc_temp.lv[j - E.ls]);
-    copy_level(E, j - 1, E.pf.lv[j - 1 - E.ls], E.corr.lv[j - 1 - E.ls]);
-    prolong_level(E, E.wc_temp, E.pf, j);
-    lc(E, j, E.corr.lv[j - E.ls], 1.0, E.corr.lv[j - E.ls], 1.0, E.pf.lv[j - E.ls]);
+    interp_level(E, j, E.corr.lv[j - 1 - E.ls], E.corr.lv[j - E.ls], true);
     jacobi(E, E.corr, E.res, j, o.up_iter);
   }
   lc(E, l, u.lv[l - E.ls], 1.0, u.lv[l - E.ls], 1.0, E.corr.lv[l - E.ls]);
@@ -402,7 +482,6 @@ void v_cycle(Ell& E, const wt_solver_opts& o, MField& u, MField& f, int l, doubl
 void fmg(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
   MField& u = E.u;
   MField& f = E.f;
-  for (int l = E.ls; l <= E.le; ++l) zero_level(E, l, E.wc_mass.lv[l - E.ls]);
   std::vector<double> nrm_f(E.le - E.ls + 1);
   for (int l = E.ls; l <= E.le; ++l) {
     nrm_f[l - E.ls] = l2(E, l, f.lv[l - E.ls]);
@@ -413,7 +492,7 @@ void fmg(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
   bicgstab(E, u, f, nrm_f[0], l, o.coarse_tol, o.coarse_iter, &rep.nrm_res_final[0], &rep.iterations[0]);
   for (l = E.ls + 1; l <= E.le; ++l) {
     if (rep.nrm_res_init[l - E.ls] < o.fine_tol) continue;
-    prolong_level(E, E.wc_mass, u, l);
+    interp_level(E, l, u.lv[l - 1 - E.ls], u.lv[l - E.ls], false);
     jacobi(E, u, f, l, o.pre_iter);
     for (int iter = 1; iter <= o.max_vcycle; ++iter) {
       v_cycle(E, o, u, f, l, nrm_f[l - E.ls], rep);
@@ -426,7 +505,6 @@ void fmg(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
 void srj(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
   MField& u = E.u;
   MField& f = E.f;
-  for (int l = E.ls; l <= E.le; ++l) zero_level(E, l, E.wc_mass.lv[l - E.ls]);
   std::vector<double> nrm_f(E.le - E.ls + 1);
   for (int l = E.ls; l <= E.le; ++l) {
     nrm_f[l - E.ls] = l2(E, l, f.lv[l - E.ls]);
@@ -447,19 +525,51 @@ void srj(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
   int l = E.ls;
   bicgstab(E, u, f, nrm_f[0], l, o.coarse_tol, o.coarse_iter, &rep.nrm_res_final[0], &rep.iterations[0]);
   for (l = E.ls + 1; l <= E.le; ++l) {
-    prolong_level(E, E.wc_mass, u, l);
-    int ii = 0;
-    for (int iter = 1; iter <= max_iter; ++iter) {
-      ii = ii + 1;
-      if (ii > m) {
-        if (rep.nrm_res_final[l - E.ls] < o.fine_tol) break;
-        ii = 1;
+    interp_level(E, l, u.lv[l - 1 - E.ls], u.lv[l - E.ls], false);
+    // Sweep k and the residual norm of what sweep k-1 left come from one stencil
+    // pass over u_{k-1}.  The host reads the norms of m sweeps at a time and, when
+    // one of them reaches the tolerance, steps back to that sweep: sweeps past it
+    // are undone exactly by keeping the m states of a batch.
+    const int q = l - E.ls;
+    const unsigned g = nb(10 * E.m(l) * E.m(l));
+    const EllLev V = E.view(l);
+    double* ring[m + 1];
+    ring[0] = u.lv[q];
+    double* pool[m] = {E.tmp.lv[q], E.rr.lv[q], E.r0.lv[q], E.pp.lv[q], E.ss.lv[q], E.ap.lv[q], E.as_.lv[q], E.cc.lv[q]};
+    for (int k = 0; k < m; ++k) ring[k + 1] = pool[k];
+    int iter = 0;
+    bool done = max_iter < 1;
+    while (!done) {
+      const int nb_ = std::min(m, max_iter - iter);
+      for (int k = 0; k < nb_; ++k) {
+        // norm of ring[k] (the state after sweep iter + k) and sweep iter + k + 1 into ring[k + 1]
+        k_ell_resid_norm<<<g, TPB, 0, E.s()>>>(V, ring[k], f.lv[q], nullptr, nullptr, ring[k + 1], w[(iter + k) % m],
+                                               E.partial, E.ticket, E.scal + 8 + k, 1, nullptr);
       }
-      jacobi(E, u, f, l, 1, w[ii - 1]);
-      rep.nrm_res_final[l - E.ls] = res_err(E, f, u, nrm_f[l - E.ls], l);
-      rep.iterations[l - E.ls] = iter;
-      if (rep.nrm_res_final[l - E.ls] <= o.fine_tol) break;
+      k_ell_resid_norm<<<g, TPB, 0, E.s()>>>(V, ring[nb_], f.lv[q], nullptr, nullptr, nullptr, 0.0, E.partial, E.ticket,
+                                             E.scal + 8 + nb_, 1, nullptr);
+      double nrm[m + 1];
+      cudaMemcpyAsync(nrm, E.scal + 8, 8 * (nb_ + 1), cudaMemcpyDeviceToHost, E.s());
+      cudaStreamSynchronize(E.s());
+      int last = nb_;
+      for (int k = 1; k <= nb_; ++k) {
+        rep.nrm_res_final[q] = nrm[k] / nrm_f[q];
+        if (rep.nrm_res_final[q] <= o.fine_tol) {
+          last = k;
+          done = true;
+          break;
+        }
+      }
+      iter += last;
+      rep.iterations[q] = iter;
+      std::swap(ring[0], ring[last]);
+      if (iter >= max_iter) done = true;
     }
+    // ring[0] holds the solution; the other buffers keep roles among themselves
+    u.lv[q] = ring[0];
+    double** role[m] = {&E.tmp.lv[q], &E.rr.lv[q], &E.r0.lv[q], &E.pp.lv[q], &E.ss.lv[q], &E.ap.lv[q], &E.as_.lv[q],
+                        &E.cc.lv[q]};
+    for (int k = 0; k < m; ++k) *role[k] = ring[k + 1];
   }
 }
 
@@ -522,8 +632,7 @@ int wt_elliptic_prolong(wt_handle* h, int fine) {
   if (!h || !h->ell) return WT_ERR_STATE;
   Ell& E = *static_cast<Ell*>(h->ell);
   if (fine <= E.ls || fine > E.le) return WT_ERR_ARG;
-  for (int l = E.ls; l <= E.le; ++l) zero_level(E, l, E.wc_mass.lv[l - E.ls]);
-  prolong_level(E, E.wc_mass, E.u, fine);
+  interp_level(E, fine, E.u.lv[fine - 1 - E.ls], E.u.lv[fine - E.ls], false);
   CKE(cudaStreamSynchronize(E.s()));
   CKE(cudaGetLastError());
   return WT_OK;
@@ -668,7 +777,7 @@ int eta_after_step(wt_handle* h, Ell& E) {
     double* wc = E.eta_wc.lv[q];
     zero_level(E, l, wc);
     const int n = E.L[q - 1].n;
-    k_wc_compute<<<nb(10 * n * n), TPB, 0, E.s()>>>(E.view(l - 1), E.view(l), eta[q], wc);
+    k_wc_compute<double><<<nb(10 * n * n), TPB, 0, E.s()>>>(E.view(l - 1), E.view(l), eta[q], wc);
   }
   return eta_inverse(h, E, eta);
 }

@@ -7,155 +7,86 @@
 
 namespace {
 
-template <class T>
-__device__ __forceinline__ T rdwT(const EllLev& L, const T* __restrict__ f, int d, int i, int j) {
-  if (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1) return T(0);
-  return f[L.nsrc[nidx(L, d, i, j)]];
-}
-__device__ __forceinline__ float oaf(const EllLev& L, int d, int i, int j, int k) {
-  if (i < -2 || j < -2 || i > L.n + 1 || j > L.n + 1) return 0.f;
-  return (float)L.oa[(int64_t)(k - 1) * L.NN + nidx(L, d, i, j)];
-}
-__device__ __forceinline__ float interp_node32(const EllLev& F, const float* s, int d, int i, int j, int i1, int j1,
-                                               int i2, int j2, int i3, int j3, int i4, int j4) {
-  return (oaf(F, d, i, j, 1) * rdwT(F, s, d, i1, j1) + oaf(F, d, i, j, 2) * rdwT(F, s, d, i2, j2) +
-          oaf(F, d, i, j, 3) * rdwT(F, s, d, i3, j3) + oaf(F, d, i, j, 4) * rdwT(F, s, d, i4, j4)) *
-         F.hinvf[nidx(F, d, i, j)];
-}
-
-// FP32 restriction of a residual (wavelets + lifting) from level c+1 to c.
-__global__ void k_wc_compute32(EllLev C, EllLev F, const float* __restrict__ s, float* __restrict__ wc) {
-  const int m = C.n;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 10 * m * m) return;
-  int d, ip, jp;
-  decode(C, t, d, ip, jp, m);
-  const int i = 2 * ip, j = 2 * jp;
-  wc[nidx(F, d, i + 1, j)] = rdwT(F, s, d, i + 1, j) - interp_node32(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2);
-  wc[nidx(F, d, i + 1, j + 1)] =
-      rdwT(F, s, d, i + 1, j + 1) - interp_node32(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2);
-  wc[nidx(F, d, i, j + 1)] = rdwT(F, s, d, i, j + 1) - interp_node32(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2);
-}
-
-__global__ void k_restrict32(EllLev C, EllLev F, const float* __restrict__ sf, const float* __restrict__ wc,
-                             float* __restrict__ sc) {
-  const int m = C.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 10 * m * m) return;
-  int d, ip, jp;
-  decode(C, t, d, ip, jp, m);
-  const int64_t kp = nidx(C, d, ip, jp);
-  if (C.nsrc[kp] != kp) return;
-  const int i = 2 * ip, j = 2 * jp;
-#define W(a, b, k) (rdwT(F, wc, d, i + (a), j + (b)) * oaf(F, d, i + (a), j + (b), k))
-  const float sum = W(1, 0, 1) + W(1, 1, 2) + W(2, 1, 3) + W(1, 2, 4) + W(0, 1, 1) + W(-1, 0, 2) + W(-1, 1, 3) +
-                    W(-2, -1, 4) + W(-1, -1, 1) + W(0, -1, 2) + W(-1, -2, 3) + W(1, -1, 4);
-#undef W
-  sc[kp] = sf[nidx(F, d, i, j)] + sum * C.hinvf[kp];
-}
-
-// Interpolation of a coarse correction onto level f (zero wavelets): even
-// children copy the parent, odd children interpolate.  acc: add into dst.
-__global__ void k_interp_even32(EllLev C, EllLev F, const float* __restrict__ sc, float* __restrict__ sf) {
-  const int m = C.n + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 10 * m * m) return;
-  int d, ip, jp;
-  decode(C, t, d, ip, jp, m);
-  const int64_t kc = nidx(F, d, 2 * ip, 2 * jp);
-  if (F.nsrc[kc] != kc) return;
-  sf[kc] = sc[C.nsrc[nidx(C, d, ip, jp)]];
-}
-__global__ void k_interp_odd32(EllLev C, EllLev F, float* __restrict__ s) {
-  const int m = C.n;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 10 * m * m) return;
-  int d, ip, jp;
-  decode(C, t, d, ip, jp, m);
-  const int i = 2 * ip, j = 2 * jp;
-  float a = interp_node32(F, s, d, i + 1, j, i, j, i + 2, j, i + 2, j + 2, i, j - 2);
-  float b = interp_node32(F, s, d, i + 1, j + 1, i + 2, j + 2, i, j, i + 2, j, i, j + 2);
-  float c = interp_node32(F, s, d, i, j + 1, i, j, i, j + 2, i - 2, j, i + 2, j + 2);
-  s[nidx(F, d, i + 1, j)] = a;
-  s[nidx(F, d, i + 1, j + 1)] = b;
-  s[nidx(F, d, i, j + 1)] = c;
-}
-
-__global__ void k_add32(int64_t n, float* __restrict__ a, const float* __restrict__ b) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) a[t] += b[t];
-}
-__global__ void k_d2f(int64_t n, const double* __restrict__ a, float* __restrict__ b) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) b[t] = (float)a[t];
-}
 // u += (double) c  on the whole level (ghost copies are refreshed by reads via nsrc)
 __global__ void k_axpy_f2d(int64_t n, double* __restrict__ u, const float* __restrict__ c) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) u[t] = u[t] + (double)c[t];
 }
 
-
-void jacobi32(Ell& E, MField& u, MField& f, int l, int iters, float w = 1.f) {
+// Jacobi sweeps; the last one also adds its result to acc (the refined
+// solution) where given.
+void jacobi32(Ell& E, MField& u, MField& f, int l, int iters, double* acc = nullptr) {
   EllLev V = E.view(l);
   unsigned g = nb(10 * E.m(l) * E.m(l));
   for (int it = 0; it < iters; ++it) {
-    k_ell_op32<OP_JACOBI><<<g, TPB, 0, E.s()>>>(V, u.lvf[l - E.ls], f.lvf[l - E.ls], E.t32.lvf[l - E.ls], w);
+    k_ell_op<OP_JACOBI, float><<<g, TPB, 0, E.s()>>>(V, u.lvf[l - E.ls], f.lvf[l - E.ls], E.t32.lvf[l - E.ls], 1.f,
+                                                     it == iters - 1 ? acc : nullptr);
     std::swap(u.lvf[l - E.ls], E.t32.lvf[l - E.ls]);
   }
 }
+void jacobi32_zero(Ell& E, MField& u, MField& f, int l, int iters) {
+  const int q = l - E.ls;
+  if (iters < 1) {
+    cudaMemsetAsync(u.lvf[q], 0, 4 * E.L[q].NN, E.s());
+    return;
+  }
+  k_ell_first2<float><<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), f.lvf[q], u.lvf[q], iters > 1);
+  jacobi32(E, u, f, l, iters - 2);
+}
 
-// One FP32 V-cycle for L c = r on levels ls..le, c returned in E.c32 (level le).
-void vcycle32(Ell& E, const wt_solver_opts& o) {
-  for (int j = E.ls; j <= E.le; ++j) cudaMemsetAsync(E.c32.lvf[j - E.ls], 0, 4 * E.L[j - E.ls].NN, E.s());
+// One FP32 V-cycle for L c = r on levels ls..le, c returned in E.c32 (level le)
+// and added to acc where given.  Per level above the coarsest seven launches:
+// the first two sweeps, the residual, wavelets and restriction on the way down,
+// the interpolation and two sweeps on the way up; the coarsest level's sweeps
+// are one launch where a cluster holds it.
+void vcycle32(Ell& E, const wt_solver_opts& o, double* acc = nullptr) {
   for (int j = E.le; j >= E.ls + 1; --j) {
-    jacobi32(E, E.c32, E.r32, j, o.down_iter);
-    EllLev V = E.view(j);
-    unsigned g = nb(10 * E.m(j) * E.m(j));
-    // residual r - L c into t32 (level j), then restrict it into r32 at level j-1
-    k_ell_op32<OP_RESID><<<g, TPB, 0, E.s()>>>(V, E.c32.lvf[j - E.ls], E.r32.lvf[j - E.ls], E.u32.lvf[j - E.ls], 1.f);
+    const int q = j - E.ls;
+    jacobi32_zero(E, E.c32, E.r32, j, o.down_iter);
+    // residual r - L c into u32 (level j), then restrict it into r32 at level j-1
     EllLev C = E.view(j - 1), F = E.view(j);
-    int n = E.L[j - 1 - E.ls].n;
-    cudaMemsetAsync(E.f32.lvf[j - E.ls], 0, 4 * E.L[j - E.ls].NN, E.s());
-    k_wc_compute32<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.u32.lvf[j - E.ls], E.f32.lvf[j - E.ls]);
-    k_restrict32<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.u32.lvf[j - E.ls], E.f32.lvf[j - E.ls],
-                                                                 E.r32.lvf[j - 1 - E.ls]);
+    const int n = E.L[q - 1].n;
+    k_ell_op<OP_RESID, float><<<nb(10 * E.m(j) * E.m(j)), TPB, 0, E.s()>>>(F, E.c32.lvf[q], E.r32.lvf[q], E.u32.lvf[q],
+                                                                          1.f, nullptr);
+    k_wc_compute<float><<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.u32.lvf[q], E.f32.lvf[q]);
+    k_restrict<float><<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.u32.lvf[q], E.f32.lvf[q],
+                                                                      E.r32.lvf[q - 1]);
   }
-  jacobi32(E, E.c32, E.r32, E.ls, o.coarse_iter);
+  if (cluster_level(E, E.ls) && o.coarse_iter > 0)
+    coarse_jacobi<float>(E, E.r32.lvf[0], E.c32.lvf[0], E.t32.lvf[0], o.coarse_iter);
+  else
+    jacobi32_zero(E, E.c32, E.r32, E.ls, o.coarse_iter);
   for (int j = E.ls + 1; j <= E.le; ++j) {
-    EllLev C = E.view(j - 1), F = E.view(j);
-    int n = E.L[j - 1 - E.ls].n;
-    k_interp_even32<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.c32.lvf[j - 1 - E.ls], E.u32.lvf[j - E.ls]);
-    k_interp_odd32<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.u32.lvf[j - E.ls]);
-    int64_t NN = E.L[j - E.ls].NN;
-    k_add32<<<nb(NN), TPB, 0, E.s()>>>(NN, E.c32.lvf[j - E.ls], E.u32.lvf[j - E.ls]);
-    jacobi32(E, E.c32, E.r32, j, o.up_iter);
+    const int q = j - E.ls;
+    k_interp<float><<<nb(10 * E.m(j) * E.m(j)), TPB, 0, E.s()>>>(E.view(j - 1), E.view(j), E.c32.lvf[q - 1],
+                                                                 E.c32.lvf[q], 1);
+    jacobi32(E, E.c32, E.r32, j, o.up_iter, j == E.le ? acc : nullptr);
   }
+  // no sweep at the top took the sum (no up sweeps, or one level only)
+  const int q = E.le - E.ls;
+  if (acc && (E.le == E.ls || o.up_iter < 1))
+    k_axpy_f2d<<<nb(E.L[q].NN), TPB, 0, E.s()>>>(E.L[q].NN, acc, E.c32.lvf[q]);
 }
 
 // The same V-cycle in FP64 (WT_SOLVER_MG64): the precision-matched baseline of
 // the mixed solver, with the reference's FP64 kernels.
 void vcycle64(Ell& E, const wt_solver_opts& o) {
-  for (int j = E.ls; j <= E.le; ++j) zero_level(E, j, E.corr.lv[j - E.ls]);
   for (int j = E.le; j >= E.ls + 1; --j) {
-    jacobi(E, E.corr, E.res, j, o.down_iter);
-    op(E, OP_RESID, j, E.corr.lv[j - E.ls], E.res.lv[j - E.ls], E.au.lv[j - E.ls]);
+    const int q = j - E.ls;
+    jacobi_zero(E, E.corr, E.res, j, o.down_iter);
+    op(E, OP_RESID, j, E.corr.lv[q], E.res.lv[q], E.au.lv[q]);
     EllLev C = E.view(j - 1), F = E.view(j);
-    int n = E.L[j - 1 - E.ls].n;
-    zero_level(E, j, E.wc_temp.lv[j - E.ls]);
-    k_wc_compute<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.au.lv[j - E.ls], E.wc_temp.lv[j - E.ls]);
-    k_restrict<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.au.lv[j - E.ls], E.wc_temp.lv[j - E.ls],
-                                                                E.res.lv[j - 1 - E.ls]);
+    const int n = E.L[q - 1].n;
+    k_wc_compute<double><<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.au.lv[q], E.wc_temp.lv[q]);
+    k_restrict<double><<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.au.lv[q], E.wc_temp.lv[q],
+                                                                       E.res.lv[q - 1]);
   }
-  jacobi(E, E.corr, E.res, E.ls, o.coarse_iter);
+  if (cluster_level(E, E.ls) && o.coarse_iter > 0)
+    coarse_jacobi<double>(E, E.res.lv[0], E.corr.lv[0], E.tmp.lv[0], o.coarse_iter);
+  else
+    jacobi_zero(E, E.corr, E.res, E.ls, o.coarse_iter);
   for (int j = E.ls + 1; j <= E.le; ++j) {
-    EllLev C = E.view(j - 1), F = E.view(j);
-    int n = E.L[j - 1 - E.ls].n;
-    zero_level(E, j, E.wc_mass.lv[j - E.ls]);
-    k_prolong_even<<<nb(10 * (n + 1) * (n + 1)), TPB, 0, E.s()>>>(C, F, E.corr.lv[j - 1 - E.ls], E.wc_mass.lv[j - E.ls],
-                                                                    E.pf.lv[j - E.ls]);
-    k_prolong_odd<<<nb(10 * n * n), TPB, 0, E.s()>>>(C, F, E.pf.lv[j - E.ls], E.wc_mass.lv[j - E.ls]);
-    lc(E, j, E.corr.lv[j - E.ls], 1.0, E.corr.lv[j - E.ls], 1.0, E.pf.lv[j - E.ls]);
+    interp_level(E, j, E.corr.lv[j - 1 - E.ls], E.corr.lv[j - E.ls], true);
     jacobi(E, E.corr, E.res, j, o.up_iter);
   }
 }
@@ -173,8 +104,11 @@ int mixed_ir(Ell& E, const wt_solver_opts& o, wt_solver_report& rep, bool fp64 =
   int it;
   double err = 0.0;
   for (it = 0; it <= o.ir_max; ++it) {
-    op(E, OP_RESID, l, E.u.lv[q], E.f.lv[q], E.res.lv[q]);
-    err = l2(E, l, E.res.lv[q]) / nf;
+    // the residual, its norm and (mixed) its FP32 copy in one pass
+    k_ell_resid_norm<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(
+        E.view(l), E.u.lv[q], E.f.lv[q], fp64 ? E.res.lv[q] : nullptr, fp64 ? nullptr : E.r32.lvf[q], nullptr, 0.0,
+        E.partial, E.ticket, E.scal, 1, nullptr);
+    err = fetch(E, 0) / nf;
     if (it == 0) rep.nrm_res_init[q] = err;
     if (err <= o.ir_tol || it == o.ir_max) break;
     // The correction cycle has no host decision: it is captured once per
@@ -191,9 +125,7 @@ int mixed_ir(Ell& E, const wt_solver_opts& o, wt_solver_report& rep, bool fp64 =
           vcycle64(E, o);
           k_axpy_d<<<nb(NN), TPB, 0, E.s()>>>(NN, E.u.lv[q], E.corr.lv[q]);
         } else {
-          k_d2f<<<nb(NN), TPB, 0, E.s()>>>(NN, E.res.lv[q], E.r32.lvf[q]);
-          vcycle32(E, o);
-          k_axpy_f2d<<<nb(NN), TPB, 0, E.s()>>>(NN, E.u.lv[q], E.c32.lvf[q]);
+          vcycle32(E, o, E.u.lv[q]);
         }
       });
       if (rc != WT_OK) return rc;

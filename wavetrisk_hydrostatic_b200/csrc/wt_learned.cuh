@@ -411,10 +411,7 @@ void fcg_iteration(Ell& E, LPNet& N, const wt_solver_opts& o, int pre) {
                                                      N.partial2);
   k_lp_sum2<<<1, 256, 0, st>>>(N.partial, N.partial2, N.nbd(), N.fcg + FCG_PR, N.fcg + FCG_DELTA);
   k_fcg_step<<<lpg(ns), LP_TPB, 0, st>>>(ns, N.slot, N.fcg, N.p, N.lp, E.u.lv[q], N.r);
-  EllLev V = E.view(l);
-  const unsigned g = nb(10 * E.m(l) * E.m(l));
-  k_ell_dot<TPB><<<g, TPB, 0, st>>>(V, N.r, N.r, E.partial);
-  k_final_sum<<<1, 256, 0, st>>>(E.partial, (int)g, N.fcg + FCG_RNORM, 1, nullptr);
+  dot_to(E, l, N.r, N.r, N.fcg + FCG_RNORM, 1);
 }
 
 int fcg_launch(Ell& E, LPNet& N, const wt_solver_opts& o, int pre) {
