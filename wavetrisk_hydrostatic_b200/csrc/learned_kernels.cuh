@@ -469,80 +469,272 @@ __global__ void __launch_bounds__(NT) k_lp_aloss(int ns, const int* __restrict__
   block_partial<NT>(v, partial);
 }
 
-// Input value ci of node u for the weight gradient: FP32 (the network input)
-// or BF16 (the stored activations), node-major.
-__device__ __forceinline__ float lp_in(const float* a, int64_t i) { return a[i]; }
-__device__ __forceinline__ float lp_in(const __nv_bfloat16* a, int64_t i) { return __bfloat162float(a[i]); }
+// Two FP32 multiply-adds in one instruction (each rounded as fmaf).
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
 
-// Weight gradient of one layer: dW[t][ci][co] = sum_s dz(s)[co] *
-// in(tap_t(s))[ci], in and dz node-major.  A block stages a chunk of kChunk
-// nodes (their tap inputs A[s][t*CIN+ci] and dz) in shared memory; each
-// thread owns fixed entries of the gradient and sums them over the block's
-// chunks, then adds them once to the global gradient.
-constexpr int kChunk = 32;
-template <int CIN, int COUT, class TIn>
-__global__ void __launch_bounds__(256) k_lp_wgrad(int ns, const int* __restrict__ tap, const TIn* __restrict__ in,
-                                                  const float* __restrict__ dz, float* __restrict__ dW) {
-  constexpr int K = kTaps * CIN;             // rows of A
-  constexpr int NE = K * COUT;               // gradient entries
-  constexpr int PER = (NE + 255) / 256;      // entries per thread
-  __shared__ float A[kChunk][K];
-  __shared__ float G[kChunk][COUT];
-  float acc[PER];
+// Weight gradient of the 32 -> 32 layer: dW[t][ci][co] = sum_s dz(s)[co] *
+// h(tap_t(s))[ci], FP32 sums.  A block stages kChunk nodes (their 7 x 32 tap
+// inputs, widened to FP32, and dz) in shared memory and keeps all 224 x 32
+// entries in registers, 8 x 8 a thread, two half-blocks taking half of the
+// nodes each; the next chunk's rows are in flight while this one is summed.
+// Bound by shared-memory operand reads: 8 x 8 tiles take 64 bytes per 64
+// multiply-adds, where one entry a thread took 8 bytes a multiply-add and
+// ran 376 us at J7.
+constexpr int kChunk = 32, kWgPitch = kTaps * kC + 4;
+__global__ void __launch_bounds__(256, 2) k_lp_wgrad32(int ns, const int* __restrict__ tap,
+                                                       const uint4* __restrict__ h, const float* __restrict__ dz,
+                                                       float* __restrict__ dW) {
+  __shared__ __align__(16) float A[kChunk][kWgPitch];
+  __shared__ __align__(16) float G[kChunk][kC];
+  const int tid = threadIdx.x, half = tid / 112, r = tid - half * 112, kg = r >> 2, cg = r & 3;
+  const bool work = tid < 224;
+  unsigned long long acc[8][4];
 #pragma unroll
-  for (int r = 0; r < PER; ++r) acc[r] = 0.0f;
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
   const int nchunk = (ns + kChunk - 1) / kChunk;
-  for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
+  uint4 v[4];
+  float4 gv;
+  auto fetch = [&](int c) {
     const int s0 = c * kChunk;
-    __syncthreads();
-    for (int q = threadIdx.x; q < kChunk * K; q += 256) {
-      const int nl = q / K, k = q % K, s = s0 + nl;
-      float v = 0.0f;
-      if (s < ns) {
-        const int t = k / CIN, ci = k % CIN, u = tap[t * ns + s];
-        v = u >= 0 ? lp_in(in, (int64_t)u * CIN + ci) : 0.0f;
-      }
-      A[nl][k] = v;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = tid + 256 * q, t = e >> 7, s = s0 + ((e >> 2) & 31);
+      const int u = (t < kTaps && s < ns) ? tap[t * ns + s] : -1;
+      v[q] = u >= 0 ? h[4 * (int64_t)u + (e & 3)] : make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int q = threadIdx.x; q < kChunk * COUT; q += 256) {
-      const int nl = q / COUT, co = q % COUT, s = s0 + nl;
-      G[nl][co] = s < ns ? dz[(int64_t)s * COUT + co] : 0.0f;
-    }
+    const int s = s0 + (tid >> 3);
+    gv = s < ns ? reinterpret_cast<const float4*>(dz)[(int64_t)s * 8 + (tid & 7)] : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  int c = blockIdx.x;
+  if (c < nchunk) fetch(c);
+  for (; c < nchunk; c += gridDim.x) {
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < PER; ++r) {
-      const int e = threadIdx.x + 256 * r;
-      if (e < NE) {
-        const int k = e / COUT, co = e % COUT;
-        float a = acc[r];
-#pragma unroll 8
-        for (int nl = 0; nl < kChunk; ++nl) a = fmaf(A[nl][k], G[nl][co], a);
-        acc[r] = a;
+    for (int q = 0; q < 4; ++q) {
+      const int e = tid + 256 * q, t = e >> 7;
+      if (t < kTaps) {
+        float f[8];
+        unpack_bf16x8(v[q], f);
+        float4* to = reinterpret_cast<float4*>(&A[(e >> 2) & 31][t * kC + 8 * (e & 3)]);
+        to[0] = make_float4(f[0], f[1], f[2], f[3]);
+        to[1] = make_float4(f[4], f[5], f[6], f[7]);
+      }
+    }
+    reinterpret_cast<float4*>(&G[tid >> 3][0])[tid & 7] = gv;
+    __syncthreads();
+    if (c + (int)gridDim.x < nchunk) fetch(c + gridDim.x);
+    if (work) {
+#pragma unroll 2
+      for (int nl = 16 * half; nl < 16 * half + 16; ++nl) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&A[nl][4 * kg]);
+        const float4 a1 = *reinterpret_cast<const float4*>(&A[nl][112 + 4 * kg]);
+        const ulonglong2 g0 = *reinterpret_cast<const ulonglong2*>(&G[nl][4 * cg]);
+        const ulonglong2 g1 = *reinterpret_cast<const ulonglong2*>(&G[nl][16 + 4 * cg]);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const unsigned long long aa = pack2(a[q], a[q]);
+          acc[q][0] = ffma2(aa, g0.x, acc[q][0]);
+          acc[q][1] = ffma2(aa, g0.y, acc[q][1]);
+          acc[q][2] = ffma2(aa, g1.x, acc[q][2]);
+          acc[q][3] = ffma2(aa, g1.y, acc[q][3]);
+        }
+      }
+    }
+  }
+  // the second half's sums join the first's in shared memory, then one global addition an entry and block
+  __syncthreads();
+  float* X = &A[0][0];
+  auto entry = [&](int q, int b) {  // of the pair b of row q
+    const int k = (q < 4 ? 0 : 112) + 4 * kg + (q & 3), co = (b < 2 ? 0 : 16) + 4 * cg + 2 * (b & 1);
+    return k * kC + co;
+  };
+  if (work && half)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) unpack2(acc[q][b], X[entry(q, b)], X[entry(q, b) + 1]);
+  __syncthreads();
+  if (work && !half)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        float x, y;
+        unpack2(acc[q][b], x, y);
+        const int e = entry(q, b);
+        atomicAdd(&dW[e], x + X[e]);
+        atomicAdd(&dW[e + 1], y + X[e + 1]);
+      }
+}
+static_assert(kChunk * kWgPitch >= kTaps * kC * kC, "the gradient fits the staging buffer");
+
+// Weight gradient of the 32 -> 1 layer: dW[t][ci] = sum_s dy(s) h(tap_t(s))[ci].
+// A half-warp takes a node, a lane two channels: each tap is one coalesced read
+// of the tap's row, which is all the kernel moves (7 x 64 bytes a node).
+__global__ void __launch_bounds__(256) k_lp_wgrad_out(int ns, const int* __restrict__ tap,
+                                                      const unsigned* __restrict__ h, const float* __restrict__ dy,
+                                                      float* __restrict__ dW) {
+  __shared__ float sh[kTaps * kC];
+  const int lane = threadIdx.x & 31, sub = lane >> 4, c2 = lane & 15;
+  float ax[kTaps], ay[kTaps];
+#pragma unroll
+  for (int t = 0; t < kTaps; ++t) ax[t] = ay[t] = 0.0f;
+  const int stride = gridDim.x * 16;
+#pragma unroll 2
+  for (int s = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 2 + sub; s < ns; s += stride) {
+    const float g = dy[s];
+#pragma unroll
+    for (int t = 0; t < kTaps; ++t) {
+      const int u = tap[t * ns + s];
+      const unsigned w = u >= 0 ? h[(int64_t)u * 16 + c2] : 0u;
+      ax[t] = fmaf(__uint_as_float(w << 16), g, ax[t]);
+      ay[t] = fmaf(__uint_as_float(w & 0xffff0000u), g, ay[t]);
+    }
+  }
+  for (int q = threadIdx.x; q < kTaps * kC; q += 256) sh[q] = 0.0f;
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kTaps; ++t) {
+    ax[t] += __shfl_xor_sync(0xffffffffu, ax[t], 16);
+    ay[t] += __shfl_xor_sync(0xffffffffu, ay[t], 16);
+    if (!sub) {
+      atomicAdd(&sh[t * kC + 2 * c2], ax[t]);
+      atomicAdd(&sh[t * kC + 2 * c2 + 1], ay[t]);
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < kTaps * kC; q += 256) atomicAdd(&dW[q], sh[q]);
+}
+
+// Weight gradient of the 2 -> 32 layer: dW[t][ci][co] = sum_s dz(s)[co]
+// x(tap_t(s))[ci].  A warp takes a node, a lane one output channel; the 14 taps'
+// inputs are warp-uniform reads beside the node's coalesced dz row.
+__global__ void __launch_bounds__(256) k_lp_wgrad_in(int ns, const int* __restrict__ tap, const float2* __restrict__ x,
+                                                     const float* __restrict__ dz, float* __restrict__ dW) {
+  __shared__ float sh[kTaps * kIn * kC];
+  const int lane = threadIdx.x & 31;
+  float a0[kTaps], a1[kTaps];
+#pragma unroll
+  for (int t = 0; t < kTaps; ++t) a0[t] = a1[t] = 0.0f;
+  const int stride = gridDim.x * 8;
+#pragma unroll 2
+  for (int s = blockIdx.x * 8 + (threadIdx.x >> 5); s < ns; s += stride) {
+    const float g = dz[(int64_t)s * kC + lane];
+#pragma unroll
+    for (int t = 0; t < kTaps; ++t) {
+      const int u = tap[t * ns + s];
+      const float2 v = u >= 0 ? x[u] : make_float2(0.0f, 0.0f);
+      a0[t] = fmaf(v.x, g, a0[t]);
+      a1[t] = fmaf(v.y, g, a1[t]);
+    }
+  }
+  for (int q = threadIdx.x; q < kTaps * kIn * kC; q += 256) sh[q] = 0.0f;
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kTaps; ++t) {
+    atomicAdd(&sh[(t * kIn) * kC + lane], a0[t]);
+    atomicAdd(&sh[(t * kIn + 1) * kC + lane], a1[t]);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < kTaps * kIn * kC; q += 256) atomicAdd(&dW[q], sh[q]);
+}
+
+// Input gradient of the 32 -> 32 layer for the nodes whose inverse taps hold at
+// most one entry a tap, itap[t][u] = s with tap_t(s) = u (or -1): 256 nodes x 32
+// channels a block, 8 x 8 a thread, tap by tap through shared memory (the tap's
+// gathered dz rows, transposed, and its weights).  The entries are added in the
+// order of the list form, which takes the few other nodes (irr).
+constexpr int kIgNodes = 256, kIgPitch = kIgNodes + 1;
+__global__ void __launch_bounds__(128) k_lp_igrad32(int ns, const int* __restrict__ itap, const float* __restrict__ W,
+                                                    const float* __restrict__ dz, const uint4* __restrict__ h,
+                                                    float slope, float* __restrict__ dzin) {
+  __shared__ float A[kC][kIgPitch];
+  __shared__ __align__(16) float Wt[kC][kC];  // [co][ci]
+  const int tid = threadIdx.x, cg = tid & 3, ng = tid >> 2, u0 = blockIdx.x * kIgNodes;
+  unsigned long long acc[8][4];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
+  for (int t = 0; t < kTaps; ++t) {
+    __syncthreads();
+#pragma unroll 4
+    for (int q = tid; q < kIgNodes * 8; q += 128) {
+      const int nl = q >> 3, c4 = q & 7, u = u0 + nl;
+      const int s = u < ns ? itap[t * ns + u] : -1;
+      const float4 g = s >= 0 ? reinterpret_cast<const float4*>(dz)[(int64_t)s * 8 + c4] : make_float4(0.f, 0.f, 0.f, 0.f);
+      A[4 * c4][nl] = g.x;
+      A[4 * c4 + 1][nl] = g.y;
+      A[4 * c4 + 2][nl] = g.z;
+      A[4 * c4 + 3][nl] = g.w;
+    }
+    for (int q = tid; q < kC * kC; q += 128) Wt[q & 31][q >> 5] = W[(t * kC + (q >> 5)) * kC + (q & 31)];
+    __syncthreads();
+#pragma unroll 4
+    for (int co = 0; co < kC; ++co) {
+      const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Wt[co][4 * cg]);
+      const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(&Wt[co][16 + 4 * cg]);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float g = A[co][ng + 32 * q];
+        const unsigned long long gg = pack2(g, g);
+        acc[q][0] = ffma2(w0.x, gg, acc[q][0]);
+        acc[q][1] = ffma2(w0.y, gg, acc[q][1]);
+        acc[q][2] = ffma2(w1.x, gg, acc[q][2]);
+        acc[q][3] = ffma2(w1.y, gg, acc[q][3]);
       }
     }
   }
 #pragma unroll
-  for (int r = 0; r < PER; ++r) {
-    const int e = threadIdx.x + 256 * r;
-    if (e < NE) atomicAdd(&dW[e], acc[r]);
+  for (int q = 0; q < 8; ++q) {
+    const int u = u0 + ng + 32 * q;
+    if (u >= ns) continue;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {  // channels 16 b + 4 cg .. + 3
+      const uint2 hv = reinterpret_cast<const uint2*>(h + 4 * (int64_t)u)[4 * b + cg];
+      float x, y, z, w;
+      unpack2(acc[q][2 * b], x, y);
+      unpack2(acc[q][2 * b + 1], z, w);
+      reinterpret_cast<float4*>(dzin)[(int64_t)u * 8 + 4 * b + cg] =
+          make_float4(x * lp_dact(__uint_as_float(hv.x << 16), slope), y * lp_dact(__uint_as_float(hv.x & 0xffff0000u), slope),
+                      z * lp_dact(__uint_as_float(hv.y << 16), slope), w * lp_dact(__uint_as_float(hv.y & 0xffff0000u), slope));
+    }
   }
 }
 
 // Gradient at the input of one layer, gathered: for node u,
 //   dh(u)[ci] = sum over (s, t) with tap_t(s) = u of sum_co W[t][ci][co] dz(s)[co],
 // the pairs listed in the inverse tap table (inv[inv_ptr[u] .. inv_ptr[u+1]),
-// entry 8 s + t), then through the activation whose stored output is h(u):
+// entry 8 s + t), then through the activation whose stored output is h(u); u runs
+// over all ns nodes or over the ns listed ones:
 // dzin(u)[ci] = dh(u)[ci] * act'(h(u)[ci]).  Node-major FP32 output.
 template <int COUT>
-__global__ void __launch_bounds__(128) k_lp_igrad(int ns, const int* __restrict__ inv_ptr,
-                                                  const int* __restrict__ inv, const float* __restrict__ W,
+__global__ void __launch_bounds__(128) k_lp_igrad(int ns, const int* __restrict__ nodes,
+                                                  const int* __restrict__ inv_ptr, const int* __restrict__ inv,
+                                                  const float* __restrict__ W,
                                                   const float* __restrict__ dz, const __nv_bfloat16* __restrict__ h,
                                                   float slope, float* __restrict__ dzin) {
   __shared__ __align__(16) float sw[kTaps * kC * COUT];
   for (int q = threadIdx.x; q < kTaps * kC * COUT; q += blockDim.x) sw[q] = W[q];
   __syncthreads();
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= ns) return;
+  if (nodes) u = nodes[u];
   float acc[kC];
 #pragma unroll
   for (int ci = 0; ci < kC; ++ci) acc[ci] = 0.0f;
@@ -580,8 +772,15 @@ __global__ void __launch_bounds__(128) k_lp_igrad(int ns, const int* __restrict_
     }
   }
 #pragma unroll
-  for (int ci = 0; ci < kC; ++ci)
-    dzin[(int64_t)u * kC + ci] = acc[ci] * lp_dact(__bfloat162float(h[(int64_t)u * kC + ci]), slope);
+  for (int q = 0; q < 4; ++q) {
+    float f[8];
+    unpack_bf16x8(reinterpret_cast<const uint4*>(h)[4 * (int64_t)u + q], f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = acc[8 * q + e] * lp_dact(f[e], slope);
+    float4* to = reinterpret_cast<float4*>(dzin) + (int64_t)u * 8 + 2 * q;
+    to[0] = make_float4(f[0], f[1], f[2], f[3]);
+    to[1] = make_float4(f[4], f[5], f[6], f[7]);
+  }
 }
 
 // Adam step on the FP32 master parameters (bias-corrected; step t >= 1).
