@@ -117,35 +117,35 @@ struct MapLev {
   const int* nsrc;
 };
 
-__global__ void k_map_or(int NN, const unsigned char* __restrict__ a, const unsigned char* __restrict__ b,
-                         unsigned char* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < NN) out[x] = (unsigned char)(a[x] | (b ? b[x] : 0));
-}
-
-__global__ void k_map_dilate(MapLev L, const unsigned char* __restrict__ in, unsigned char* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= L.NN) return;
+// One hex step of a map, v(y) its value at slot y: marked if the slot's source or
+// one of the six neighbours' is.
+template <class V>
+__device__ __forceinline__ int map_dilated(const MapLev& L, int x, V v) {
   const int PP = L.P * L.P;
   const int d = x / PP, r = x - d * PP;
   const int i = r % L.P - 2, j = r / L.P - 2;
-  int v = in[__ldg(L.nsrc + x)];
+  int any = v(__ldg(L.nsrc + x));
   const int di[6] = {1, -1, 0, 0, 1, -1}, dj[6] = {0, 0, 1, -1, 1, -1};
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const int a = i + di[k], b = j + dj[k];
-    if (a >= -2 && b >= -2 && a < L.n + 2 && b < L.n + 2)
-      v |= in[__ldg(L.nsrc + (d * L.P + b + 2) * L.P + a + 2)];
+    if (a >= -2 && b >= -2 && a < L.n + 2 && b < L.n + 2) any |= v(__ldg(L.nsrc + (d * L.P + b + 2) * L.P + a + 2));
   }
-  out[x] = (unsigned char)v;
+  return any;
 }
 
-// parent slot x of level Pa is marked if one of its four children is marked
-__global__ void k_map_up(MapLev C, MapLev Pa, const unsigned char* __restrict__ cin, unsigned char* __restrict__ out) {
+// out = dilate(a | b), b may be null
+__global__ void k_map_dilate(MapLev L, const unsigned char* __restrict__ a, const unsigned char* __restrict__ b,
+                             unsigned char* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= Pa.NN) return;
+  if (x >= L.NN) return;
+  out[x] = (unsigned char)map_dilated(L, x, [&](int y) { return b ? a[y] | b[y] : a[y]; });
+}
+
+// parent slot y of level Pa is marked if one of its four children is
+__device__ __forceinline__ int map_up(const MapLev& C, const MapLev& Pa, const unsigned char* __restrict__ cin, int y) {
   const int PP = Pa.P * Pa.P;
-  const int d = x / PP, r = x - d * PP;
+  const int d = y / PP, r = y - d * PP;
   const int ip = r % Pa.P - 2, jp = r / Pa.P - 2;
   int v = 0;
 #pragma unroll
@@ -154,7 +154,14 @@ __global__ void k_map_up(MapLev C, MapLev Pa, const unsigned char* __restrict__ 
     if (a >= -2 && b >= -2 && a < C.n + 2 && b < C.n + 2)
       v |= cin[__ldg(C.nsrc + (d * C.P + b + 2) * C.P + a + 2)];
   }
-  out[x] = (unsigned char)v;
+  return v;
+}
+// out = dilate(parents of the children marked in cin)
+__global__ void k_map_up_dilate(MapLev C, MapLev Pa, const unsigned char* __restrict__ cin,
+                                unsigned char* __restrict__ out) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= Pa.NN) return;
+  out[x] = (unsigned char)map_dilated(Pa, x, [&](int y) { return map_up(C, Pa, cin, y); });
 }
 
 }  // namespace wtw
@@ -185,18 +192,34 @@ __device__ __forceinline__ bool tree_node(const TreeLev& T, int ps, int y) {
 
 // Whether a node of an existing patch lies within 2 nodes (i and j each) of
 // padded slot (d, i, j), i, j in [0, n): the patch nodes and their 2-node ring.
+// Away from the lozenge's borders the ring lies in two by two patches (ps >= 4; up
+// to three by three for ps 2).
 __device__ __forceinline__ bool tree_near(const TreeLev& T, int ps, int d, int i, int j) {
+  if (i >= 2 && j >= 2 && i < T.n - 2 && j < T.n - 2) {
+    const int np = T.n / ps, a0 = (i - 2) / ps, a1 = (i + 2) / ps, b1 = (j + 2) / ps;
+    int v = 0;
+    for (int b = (j - 2) / ps; b <= b1; ++b)
+      for (int a = a0; a <= a1; ++a) v |= T.exist[(d * np + b) * np + a];
+    return v != 0;
+  }
   for (int b = -2; b <= 2; ++b)
     for (int a = -2; a <= 2; ++a)
       if (tree_node(T, ps, (d * T.P + j + b + 2) * T.P + i + a + 2)) return true;
   return false;
 }
 
-// need &= the tree's nodes and their ring, on the owned nodes [0, n)^2 of one
-// level (the lozenge-corner regions the seed forces stay in).
-__global__ void k_need_tree(TreeLev T, int ps, unsigned char* __restrict__ need) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= T.NN || !need[x]) return;
+// need &= the tree's nodes and their ring, on the owned nodes [0, n)^2 of every
+// level of S (the lozenge-corner regions the seed forces stay in); the maps are in
+// buf[r & 1], exist[q] the patch bytes of entry q.
+struct TreeSet {
+  const unsigned char* exist[NEED_MAXL];
+};
+__global__ void k_need_tree(NeedSet S, TreeSet E, int ps, int r_) {
+  int q, x;
+  if (!need_entry(S, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, q, x)) return;
+  unsigned char* __restrict__ need = S.L[q].buf[r_ & 1];
+  if (!need[x]) return;
+  const TreeLev T{S.L[q].n, S.L[q].P, S.L[q].NN, S.L[q].nsrc, E.exist[q]};
   const int PP = T.P * T.P;
   const int d = x / PP, r = x - d * PP;
   const int i = r % T.P - 2, j = r / T.P - 2, n = T.n;
@@ -211,11 +234,13 @@ __global__ void k_need_tree(TreeLev T, int ps, unsigned char* __restrict__ need)
 // children within 2 nodes of the coincident child is a node of an existing
 // patch of the child level, so that the state after the step is complete on
 // the tree.  Own-source parent slots only (the kernels read through nsrc).
+// k_map_tree_par takes recpar's last dilation (of in) with it.
 __global__ void k_map_tree_par(MapLev Lp, TreeLev Tc, int ps, const unsigned char* __restrict__ in,
-                               unsigned char* __restrict__ out) {
+                               unsigned char* __restrict__ recpar, unsigned char* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= Lp.NN) return;
-  unsigned char v = in[x];
+  unsigned char v = (unsigned char)map_dilated(Lp, x, [&](int y) { return in[y]; });
+  recpar[x] = v;
   if (!v && __ldg(Lp.nsrc + x) == x) {
     const int PP = Lp.P * Lp.P;
     const int d = x / PP, r = x - d * PP;
@@ -240,47 +265,52 @@ namespace wtw {
 // scan of the counts, then each block writes its entries at its offset.
 constexpr int LIST_B = 1024;
 
-// Candidates of a level's node list: every padded slot x, on where
-// need[nsrc[x]] is set.
-struct NodeCand {
-  int NN;
-  const int* nsrc;
-  const unsigned char* map;
-  __device__ __forceinline__ int n() const { return NN; }
-  __device__ __forceinline__ bool on(int t, int& x) const {
-    x = t;
-    return map[__ldg(nsrc + t)] != 0;
-  }
+// Every list of a build in one launch a pass.  Candidates of a level's node list
+// (parent 0): every padded slot x, on where map[nsrc[x]] is set; of a parent
+// level's list (parent 1): the slots of [0, n]^2.
+constexpr int LIST_MAX = 2 * NEED_MAXL;
+struct ListSet {
+  int nl;
+  int bstart[LIST_MAX + 1];  // first block of each list
+  int parent[LIST_MAX], n[LIST_MAX];
+  const int* nsrc[LIST_MAX];
+  const unsigned char* map[LIST_MAX];
+  int* ids[LIST_MAX];
+  int* count[LIST_MAX];
 };
-// Candidates of a parent level's list: the slots of [0, np]^2, on where
-// rec[nsrc[x]] is set.
-struct ParentCand {
-  int np, P;
-  const int* nsrc;
-  const unsigned char* map;
-  __device__ __forceinline__ int n() const { return 10 * (np + 1) * (np + 1); }
-  __device__ __forceinline__ bool on(int t, int& x) const {
-    const int m = np + 1, d = t / (m * m), r = t - d * m * m;
-    const int jp = r / m, ip = r - jp * m;
+__device__ __forceinline__ int list_of(const ListSet& S, int b) {
+  int q = 0;
+  while (b >= S.bstart[q + 1]) ++q;
+  return q;
+}
+__device__ __forceinline__ bool list_on(const ListSet& S, int q, int t, int& x) {
+  const int n = S.n[q], P = n + 4, m = n + 1;
+  if (S.parent[q]) {
+    if (t >= 10 * m * m) return false;
+    const int d = t / (m * m), r = t - d * m * m, jp = r / m, ip = r - jp * m;
     x = (d * P + jp + 2) * P + ip + 2;
-    return map[__ldg(nsrc + x)] != 0;
+  } else {
+    if (t >= 10 * P * P) return false;
+    x = t;
   }
-};
+  return S.map[q][__ldg(S.nsrc[q] + x)] != 0;
+}
 
-template <class Cand>
-__global__ void __launch_bounds__(LIST_B) k_list_count(Cand c, int* __restrict__ bcnt) {
-  const int t = blockIdx.x * LIST_B + threadIdx.x;
+__global__ void __launch_bounds__(LIST_B) k_list_count(ListSet S, int* __restrict__ bcnt) {
+  const int q = list_of(S, blockIdx.x);
   int x;
-  const bool on = t < c.n() && c.on(t, x);
+  const bool on = list_on(S, q, (blockIdx.x - S.bstart[q]) * LIST_B + threadIdx.x, x);
   const int k = __syncthreads_count(on);
   if (threadIdx.x == 0) bcnt[blockIdx.x] = k;
 }
 
-// Exclusive scan of nb block counts into boff, the total into *count (one block).
-__global__ void __launch_bounds__(LIST_B) k_list_scan(int nb, const int* __restrict__ bcnt, int* __restrict__ boff,
-                                                      int* __restrict__ count) {
+// Exclusive scan of each list's block counts into boff, the total into *count (one
+// block a list).
+__global__ void __launch_bounds__(LIST_B) k_list_scan(ListSet S, const int* __restrict__ bcnt, int* __restrict__ boff) {
   __shared__ int part[LIST_B];
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, l = blockIdx.x, nb = S.bstart[l + 1] - S.bstart[l];
+  bcnt += S.bstart[l];
+  boff += S.bstart[l];
   const int run = (nb + LIST_B - 1) / LIST_B;
   const int a = min(nb, t * run), b = min(nb, a + run);
   int c = 0;
@@ -298,22 +328,21 @@ __global__ void __launch_bounds__(LIST_B) k_list_scan(int nb, const int* __restr
     boff[q] = w;
     w += bcnt[q];
   }
-  if (t == LIST_B - 1) *count = part[t];
+  if (t == LIST_B - 1) *S.count[l] = part[t];
 }
 
-template <class Cand>
-__global__ void __launch_bounds__(LIST_B) k_list_write(Cand c, const int* __restrict__ boff, int* __restrict__ ids) {
+__global__ void __launch_bounds__(LIST_B) k_list_write(ListSet S, const int* __restrict__ boff) {
   __shared__ int wsum[LIST_B / 32];
-  const int t = blockIdx.x * LIST_B + threadIdx.x;
+  const int l = list_of(S, blockIdx.x);
   int x = 0;
-  const bool on = t < c.n() && c.on(t, x);
+  const bool on = list_on(S, l, (blockIdx.x - S.bstart[l]) * LIST_B + threadIdx.x, x);
   const unsigned m = __ballot_sync(0xffffffffu, on);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) wsum[w] = __popc(m);
   __syncthreads();
   int before = 0;
   for (int q = 0; q < w; ++q) before += wsum[q];
-  if (on) ids[boff[blockIdx.x] + before + __popc(m & ((1u << lane) - 1))] = x;
+  if (on) S.ids[l][boff[blockIdx.x] + before + __popc(m & ((1u << lane) - 1))] = x;
 }
 
 }  // namespace wtw

@@ -188,12 +188,15 @@ __device__ __forceinline__ int ncode(const WLev& C, int d, int i, int j) {
   if (!inr(C, i, j)) return -1;
   return __ldg(C.nsrc + nid(C, d, i, j));
 }
+// As we / wn of wavelet_layers.cuh: no branch, read-only loads (the child's fields).
 __device__ __forceinline__ double fe(const double* __restrict__ f, int c) {
-  if (c < 0) return 0.0;
-  const double v = f[c >> 1];
-  return (c & 1) ? -v : v;
+  const double v = __ldg(f + (max(c, 0) >> 1));
+  return c < 0 ? 0.0 : (c & 1) ? -v : v;
 }
-__device__ __forceinline__ double fn(const double* __restrict__ f, int c) { return c < 0 ? 0.0 : f[c]; }
+__device__ __forceinline__ double fn(const double* __restrict__ f, int c) {
+  const double v = __ldg(f + max(c, 0));
+  return c < 0 ? 0.0 : v;
+}
 
 __device__ __forceinline__ void sm_build(SmTerm& t, const WLev& C, int d, const RInd& r, const int a3[3],
                                          const int p3[3], const int m3[3], int i0, int j0, int i1, int j1, bool pos) {

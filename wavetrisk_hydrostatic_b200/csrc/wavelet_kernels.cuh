@@ -34,21 +34,28 @@ struct ParentList {
 // (parent, group of lpt layers): items group-major as parent_of's, strided by
 // the grid; f(d, ip, jp, k0, k1) for the listed parents of [0, m)^2 (m = n or
 // n + 1 of the parent level, whose padded side is np + 4).
-template <class F>
+// With REP, each (group, parent) comes REP times, f's last argument 0 .. REP-1
+// (slower than the parents).
+template <int REP, class F>
 __device__ __forceinline__ void for_parents(int np, int m, int nz, int lpt, const ParentList& PL, F f) {
   const int cnt = __ldg(PL.count);
   const int ng = (nz + lpt - 1) / lpt;
   const int P = np + 4, PP = P * P;
-  const int64_t tot = (int64_t)cnt * ng;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-    const int g = (int)(t / cnt), e = (int)(t - (int64_t)g * cnt);
+  // fewer than 2^32 (the level's fields take 40 bytes for each); one grid stride past it does not wrap below tot
+  const unsigned tot = (unsigned)cnt * ng * REP;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += gridDim.x * blockDim.x) {
+    const int gr = (int)(t / (unsigned)cnt), e = (int)(t - (unsigned)gr * cnt), g = gr / REP;
     const int x = __ldg(PL.ids + e);
     const int d = x / PP, r = x - d * PP;
     const int ip = r % P - 2, jp = r / P - 2;
     if (ip < 0 || jp < 0 || ip >= m || jp >= m) continue;
     const int k0 = g * lpt;
-    f(d, ip, jp, k0, min(nz, k0 + lpt));
+    f(d, ip, jp, k0, min(nz, k0 + lpt), gr - g * REP);
   }
+}
+template <class F>
+__device__ __forceinline__ void for_parents(int np, int m, int nz, int lpt, const ParentList& PL, F f) {
+  for_parents<1>(np, m, nz, lpt, PL, [&](int d, int ip, int jp, int k0, int k1, int) { f(d, ip, jp, k0, k1); });
 }
 
 // The parent (d, ip, jp) of work-list entry x (a padded slot of a parent
@@ -339,6 +346,39 @@ __device__ __forceinline__ bool node_of(int m, int st, int& d, int& i, int& j) {
   return true;
 }
 
+// The masks of several levels for the sweeps that stay on a level: one launch over
+// all of them (thread t belongs to the level q with start[q] <= t < start[q+1]).
+constexpr int MS_MAXL = 16;
+struct MaskSet {
+  int nl;
+  int start[MS_MAXL + 1];
+  int n[MS_MAXL];
+  int* mask_n[MS_MAXL];
+  int* mask_e[MS_MAXL];
+};
+__device__ __forceinline__ WLev mask_level(const MaskSet& S, int q) {
+  WLev g{};
+  g.n = S.n[q];
+  g.P = g.n + 4;
+  g.NN = 10 * g.P * g.P;
+  g.mask_n = S.mask_n[q];
+  g.mask_e = S.mask_e[q];
+  return g;
+}
+// nodes [st, n - 1 + add + st]^2 of the thread's level
+__device__ __forceinline__ bool mask_node(const MaskSet& S, int add, int st, int& q, int& d, int& i, int& j) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= S.start[S.nl]) return false;
+  q = 0;
+  while (t >= S.start[q + 1]) ++q;
+  const int m = S.n[q] + add, x = t - S.start[q];
+  d = x / (m * m);
+  const int r = x - d * m * m;
+  j = r / m + st;
+  i = r % m + st;
+  return true;
+}
+
 // serial comm_masks_mpi (src/comm.f90:531-553): node and edge masks to their
 // ghost copies (the tables have no chains, so the copy order is immaterial).
 // The mask ghost copy of every level in one launch (comm_masks): thread t
@@ -469,10 +509,14 @@ __global__ void k_mask_tol_y(WLev L, int nz, int st, int en, const double* __res
   }
 }
 
-__global__ void k_mask_zero(WLev g) {  // init_masks_zero on one level
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < g.NN) g.mask_n[t] = ZERO;
-  if (t < 3 * g.NN) g.mask_e[t] = ZERO;
+__global__ void k_mask_zero(MaskSet S) {  // init_masks_zero, padded levels
+  int q, d, i, j;
+  if (!mask_node(S, 4, -2, q, d, i, j)) return;
+  const WLev g = mask_level(S, q);
+  const int x = nid(g, d, i, j);
+  g.mask_n[x] = ZERO;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) g.mask_e[e * g.NN + x] = ZERO;
 }
 
 // mask_parent_nodes (parents [0, np]) and mask_parent_edges (parents [0, np))
@@ -480,38 +524,40 @@ __global__ void k_mask_parent(WLev Pa, WLev C) {
   int d, ip, jp;
   if (!node_of(Pa.n + 1, 0, d, ip, jp)) return;
   const int i = 2 * ip, j = 2 * jp;
-  if (mn(C, d, i + 1, j) == TOLRNZ || mn(C, d, i + 1, j + 1) == TOLRNZ || mn(C, d, i, j + 1) == TOLRNZ ||
-      mn(C, d, i - 1, j) == TOLRNZ || mn(C, d, i - 1, j - 1) == TOLRNZ || mn(C, d, i, j - 1) == TOLRNZ) {
+  if (mn(C, d, i + 1, j) == TOLRNZ | mn(C, d, i + 1, j + 1) == TOLRNZ | mn(C, d, i, j + 1) == TOLRNZ |
+      mn(C, d, i - 1, j) == TOLRNZ | mn(C, d, i - 1, j - 1) == TOLRNZ | mn(C, d, i, j - 1) == TOLRNZ) {
     sn(Pa, d, ip, jp, TOLRNZ);
     sn(C, d, i, j, TOLRNZ);
   }
-  if (ip == Pa.n || jp == Pa.n) return;
+  if (ip == Pa.n | jp == Pa.n) return;
   auto T = [&](int e, int a, int b) { return me(C, e, d, a, b) == TOLRNZ; };
-  if (T(RT, i, j) || T(RT, i + 1, j) || T(DG, i, j - 1) || T(DG, i + 1, j) || T(UP, i + 1, j) || T(UP, i + 1, j - 1))
+  if (T(RT, i, j) | T(RT, i + 1, j) | T(DG, i, j - 1) | T(DG, i + 1, j) | T(UP, i + 1, j) | T(UP, i + 1, j - 1))
     se(Pa, RT, d, ip, jp, TOLRNZ);
-  if (T(RT, i, j + 1) || T(RT, i + 1, j + 1) || T(DG, i, j) || T(DG, i + 1, j + 1) || T(UP, i + 1, j + 1) || T(UP, i + 1, j))
+  if (T(RT, i, j + 1) | T(RT, i + 1, j + 1) | T(DG, i, j) | T(DG, i + 1, j + 1) | T(UP, i + 1, j + 1) | T(UP, i + 1, j))
     se(Pa, DG, d, ip, jp, TOLRNZ);
-  if (T(RT, i, j + 1) || T(RT, i - 1, j + 1) || T(DG, i, j + 1) || T(DG, i - 1, j) || T(UP, i, j) || T(UP, i, j + 1))
+  if (T(RT, i, j + 1) | T(RT, i - 1, j + 1) | T(DG, i, j + 1) | T(DG, i - 1, j) | T(UP, i, j) | T(UP, i, j + 1))
     se(Pa, UP, d, ip, jp, TOLRNZ);
 }
 
 // mask_adj_same_scale_nodes_edges, nodes [0, n]
-__global__ void k_mask_adj_same(WLev g) {
-  int d, i, j;
-  if (!node_of(g.n + 1, 0, d, i, j)) return;
-  if (mn(g, d, i + 1, j) == TOLRNZ || mn(g, d, i + 1, j + 1) == TOLRNZ || mn(g, d, i, j + 1) == TOLRNZ ||
-      mn(g, d, i - 1, j) == TOLRNZ || mn(g, d, i - 1, j - 1) == TOLRNZ || mn(g, d, i, j - 1) == TOLRNZ)
+__global__ void k_mask_adj_same(MaskSet S) {
+  int q, d, i, j;
+  if (!mask_node(S, 1, 0, q, d, i, j)) return;
+  const WLev g = mask_level(S, q);
+  if (mn(g, d, i + 1, j) == TOLRNZ | mn(g, d, i + 1, j + 1) == TOLRNZ | mn(g, d, i, j + 1) == TOLRNZ |
+      mn(g, d, i - 1, j) == TOLRNZ | mn(g, d, i - 1, j - 1) == TOLRNZ | mn(g, d, i, j - 1) == TOLRNZ)
     sn(g, d, i, j, ADJSPACE);
   auto T = [&](int e, int a, int b) { return me(g, e, d, a, b) == TOLRNZ; };
-  if (T(DG, i, j) || T(UP, i, j - 1) || T(DG, i, j - 1) || T(UP, i + 1, j)) se(g, RT, d, i, j, ADJSPACE);
-  if (T(UP, i, j) || T(RT, i, j) || T(UP, i + 1, j) || T(RT, i, j + 1)) se(g, DG, d, i, j, ADJSPACE);
-  if (T(DG, i, j) || T(RT, i - 1, j) || T(DG, i - 1, j) || T(RT, i, j + 1)) se(g, UP, d, i, j, ADJSPACE);
+  if (T(DG, i, j) | T(UP, i, j - 1) | T(DG, i, j - 1) | T(UP, i + 1, j)) se(g, RT, d, i, j, ADJSPACE);
+  if (T(UP, i, j) | T(RT, i, j) | T(UP, i + 1, j) | T(RT, i, j + 1)) se(g, DG, d, i, j, ADJSPACE);
+  if (T(DG, i, j) | T(RT, i - 1, j) | T(DG, i - 1, j) | T(RT, i, j + 1)) se(g, UP, d, i, j, ADJSPACE);
 }
 
 // mask_restrict_flux, nodes [0, n)
-__global__ void k_mask_restrict_flux(WLev g) {
-  int d, i, j;
-  if (!node_of(g.n, 0, d, i, j)) return;
+__global__ void k_mask_restrict_flux(MaskSet S) {
+  int q, d, i, j;
+  if (!mask_node(S, 0, 0, q, d, i, j)) return;
+  const WLev g = mask_level(S, q);
   if (mn(g, d, i, j) >= ADJSPACE) {
     se(g, RT, d, i, j, RESTRCT);
     se(g, DG, d, i, j, RESTRCT);
@@ -523,73 +569,78 @@ __global__ void k_mask_restrict_flux(WLev g) {
   }
 }
 
-// mask_adj_child, parents [0, np]
+// set_at_least without a look at the old value: where a thread sets dozens of
+// masks, each look would wait for memory before the next
+__device__ __forceinline__ void snr(const WLev& g, int d, int i, int j, int typ) {
+  if (inr(g, i, j)) atomicMax(g.mask_n + nid(g, d, i, j), typ);
+}
+__device__ __forceinline__ void ser(const WLev& g, int e, int d, int i, int j, int typ) {
+  if (inr(g, i, j)) atomicMax(g.mask_e + e * g.NN + nid(g, d, i, j), typ);
+}
+
+// mask_adj_child, parents [0, np].  The parent masks the tests read (>= ADJSPACE,
+// which the sweep's own writes of RESTRCT cannot reach) come first, together.
 __global__ void k_mask_adj_child(WLev Pa, WLev C) {
   int d, ip, jp;
   if (!node_of(Pa.n + 1, 0, d, ip, jp)) return;
   const int i = 2 * ip, j = 2 * jp;
-  auto PE = [&](int e, int a, int b, int typ) { return me(Pa, e, d, a, b) >= typ; };
-  if (mn(Pa, d, ip, jp) >= TOLRNZ) {
+  const int n0 = mn(Pa, d, ip, jp), nN = mn(Pa, d, ip, jp + 1), nNE = mn(Pa, d, ip + 1, jp + 1), nE = mn(Pa, d, ip + 1, jp);
+  const int u0 = me(Pa, UP, d, ip, jp), uS = me(Pa, UP, d, ip, jp - 1), uE = me(Pa, UP, d, ip + 1, jp);
+  const int g0 = me(Pa, DG, d, ip, jp), gSW = me(Pa, DG, d, ip - 1, jp - 1), gW = me(Pa, DG, d, ip - 1, jp),
+            gS = me(Pa, DG, d, ip, jp - 1);
+  const int r0 = me(Pa, RT, d, ip, jp), rW = me(Pa, RT, d, ip - 1, jp), rN = me(Pa, RT, d, ip, jp + 1);
+  if (n0 >= TOLRNZ) {
     const int nb[13][2] = {{0, 0},  {1, 0},  {1, 1}, {0, 1}, {-1, 0},  {-1, -1}, {0, -1},
                            {-1, 1}, {1, -1}, {2, 1}, {1, 2}, {-1, -2}, {-2, -1}};
-    for (int q = 0; q < 13; ++q) sn(C, d, i + nb[q][0], j + nb[q][1], ADJZONE);
-    se(Pa, UP, d, ip, jp, RESTRCT);
-    se(Pa, DG, d, ip, jp, RESTRCT);
-    se(Pa, RT, d, ip, jp, RESTRCT);
+#pragma unroll
+    for (int q = 0; q < 13; ++q) snr(C, d, i + nb[q][0], j + nb[q][1], ADJZONE);
+    ser(Pa, UP, d, ip, jp, RESTRCT);
+    ser(Pa, DG, d, ip, jp, RESTRCT);
+    ser(Pa, RT, d, ip, jp, RESTRCT);
   } else {
-    if (mn(Pa, d, ip, jp + 1) >= TOLRNZ) {
-      sn(C, d, i, j + 1, ADJZONE);
-      se(Pa, UP, d, ip, jp, RESTRCT);
+    if (nN >= TOLRNZ) {
+      snr(C, d, i, j + 1, ADJZONE);
+      ser(Pa, UP, d, ip, jp, RESTRCT);
     }
-    if (mn(Pa, d, ip + 1, jp + 1) >= TOLRNZ) {
-      sn(C, d, i + 1, j + 1, ADJZONE);
-      se(Pa, DG, d, ip, jp, RESTRCT);
+    if (nNE >= TOLRNZ) {
+      snr(C, d, i + 1, j + 1, ADJZONE);
+      ser(Pa, DG, d, ip, jp, RESTRCT);
     }
-    if (mn(Pa, d, ip + 1, jp) >= TOLRNZ) {
-      sn(C, d, i + 1, j, ADJZONE);
-      se(Pa, RT, d, ip, jp, RESTRCT);
+    if (nE >= TOLRNZ) {
+      snr(C, d, i + 1, j, ADJZONE);
+      ser(Pa, RT, d, ip, jp, RESTRCT);
     }
   }
-  if (PE(UP, ip, jp, TOLRNZ)) {
-    sn(C, d, i, j + 1, ADJZONE);
-    if (PE(UP, ip, jp - 1, TOLRNZ)) sn(C, d, i, j, ADJZONE);
+  const bool tu = u0 >= TOLRNZ, tg = g0 >= TOLRNZ, tr = r0 >= TOLRNZ, tuS = uS >= TOLRNZ, tuE = uE >= TOLRNZ,
+             tgSW = gSW >= TOLRNZ, tgW = gW >= TOLRNZ, tgS = gS >= TOLRNZ, trW = rW >= TOLRNZ, trN = rN >= TOLRNZ;
+  if (tu) snr(C, d, i, j + 1, ADJZONE);
+  if (tg) snr(C, d, i + 1, j + 1, ADJZONE);
+  if (tr) snr(C, d, i + 1, j, ADJZONE);
+  if ((tu & tuS) | (tg & tgSW) | (tr & trW)) snr(C, d, i, j, ADJZONE);
+  if (tu | tg | trW | tgW | trN) {
+    ser(C, UP, d, i, j, ADJZONE);
+    ser(C, UP, d, i, j + 1, ADJZONE);
   }
-  if (PE(DG, ip, jp, TOLRNZ)) {
-    sn(C, d, i + 1, j + 1, ADJZONE);
-    if (PE(DG, ip - 1, jp - 1, TOLRNZ)) sn(C, d, i, j, ADJZONE);
+  if (tg | tu | tr | tuE | trN) {
+    ser(C, DG, d, i, j, ADJZONE);
+    ser(C, DG, d, i + 1, j + 1, ADJZONE);
   }
-  if (PE(RT, ip, jp, TOLRNZ)) {
-    sn(C, d, i + 1, j, ADJZONE);
-    if (PE(RT, ip - 1, jp, TOLRNZ)) sn(C, d, i, j, ADJZONE);
+  if (tr | tg | tuS | tgS | tuE) {
+    ser(C, RT, d, i, j, ADJZONE);
+    ser(C, RT, d, i + 1, j, ADJZONE);
   }
-  if (PE(UP, ip, jp, TOLRNZ) || PE(DG, ip, jp, TOLRNZ) || PE(RT, ip - 1, jp, TOLRNZ) || PE(DG, ip - 1, jp, TOLRNZ) ||
-      PE(RT, ip, jp + 1, TOLRNZ)) {
-    se(C, UP, d, i, j, ADJZONE);
-    se(C, UP, d, i, j + 1, ADJZONE);
+  if (tu | tg | trN) {
+    ser(C, RT, d, i, j + 1, ADJZONE);
+    ser(C, DG, d, i, j + 1, ADJZONE);
+    ser(C, UP, d, i + 1, j + 1, ADJZONE);
   }
-  if (PE(DG, ip, jp, TOLRNZ) || PE(UP, ip, jp, TOLRNZ) || PE(RT, ip, jp, TOLRNZ) || PE(UP, ip + 1, jp, TOLRNZ) ||
-      PE(RT, ip, jp + 1, TOLRNZ)) {
-    se(C, DG, d, i, j, ADJZONE);
-    se(C, DG, d, i + 1, j + 1, ADJZONE);
+  if (tr | tg | tuE) {
+    ser(C, UP, d, i + 1, j, ADJZONE);
+    ser(C, DG, d, i + 1, j, ADJZONE);
+    ser(C, RT, d, i + 1, j + 1, ADJZONE);
   }
-  if (PE(RT, ip, jp, TOLRNZ) || PE(DG, ip, jp, TOLRNZ) || PE(UP, ip, jp - 1, TOLRNZ) || PE(DG, ip, jp - 1, TOLRNZ) ||
-      PE(UP, ip + 1, jp, TOLRNZ)) {
-    se(C, RT, d, i, j, ADJZONE);
-    se(C, RT, d, i + 1, j, ADJZONE);
-  }
-  if (PE(UP, ip, jp, TOLRNZ) || PE(DG, ip, jp, TOLRNZ) || PE(RT, ip, jp + 1, TOLRNZ)) {
-    se(C, RT, d, i, j + 1, ADJZONE);
-    se(C, DG, d, i, j + 1, ADJZONE);
-    se(C, UP, d, i + 1, j + 1, ADJZONE);
-  }
-  if (PE(RT, ip, jp, TOLRNZ) || PE(DG, ip, jp, TOLRNZ) || PE(UP, ip + 1, jp, TOLRNZ)) {
-    se(C, UP, d, i + 1, j, ADJZONE);
-    se(C, DG, d, i + 1, j, ADJZONE);
-    se(C, RT, d, i + 1, j + 1, ADJZONE);
-  }
-  if (PE(RT, ip, jp, ADJSPACE) || PE(DG, ip, jp, ADJSPACE) || PE(UP, ip, jp, ADJSPACE) || PE(RT, ip - 1, jp, ADJSPACE) ||
-      PE(DG, ip - 1, jp - 1, ADJSPACE) || PE(UP, ip, jp - 1, ADJSPACE))
-    sn(Pa, d, ip, jp, RESTRCT);
+  if ((r0 >= ADJSPACE) | (g0 >= ADJSPACE) | (u0 >= ADJSPACE) | (rW >= ADJSPACE) | (gSW >= ADJSPACE) | (uS >= ADJSPACE))
+    snr(Pa, d, ip, jp, RESTRCT);
 }
 
 // mask_edges_if_both_nodes, nodes [0, n)
@@ -609,17 +660,17 @@ __global__ void k_mask_edges_consist(WLev Pa, WLev C) {
   if (!node_of(Pa.n + 1, 0, d, ip, jp)) return;
   const int i = 2 * ip, j = 2 * jp;
   auto A = [&](int e, int a, int b) { return me(C, e, d, a, b) >= ADJZONE; };
-  if (A(RT, i, j) || A(RT, i + 1, j) || A(DG, i, j - 1) || A(DG, i + 1, j) || A(UP, i + 1, j - 1) || A(UP, i + 1, j)) {
+  if (A(RT, i, j) | A(RT, i + 1, j) | A(DG, i, j - 1) | A(DG, i + 1, j) | A(UP, i + 1, j - 1) | A(UP, i + 1, j)) {
     se(C, RT, d, i, j, ADJZONE);
     se(C, RT, d, i + 1, j, ADJZONE);
     se(Pa, RT, d, ip, jp, ADJZONE);
   }
-  if (A(RT, i, j + 1) || A(RT, i + 1, j + 1) || A(DG, i, j) || A(DG, i + 1, j + 1) || A(UP, i + 1, j) || A(UP, i + 1, j + 1)) {
+  if (A(RT, i, j + 1) | A(RT, i + 1, j + 1) | A(DG, i, j) | A(DG, i + 1, j + 1) | A(UP, i + 1, j) | A(UP, i + 1, j + 1)) {
     se(C, DG, d, i, j, ADJZONE);
     se(C, DG, d, i + 1, j + 1, ADJZONE);
     se(Pa, DG, d, ip, jp, ADJZONE);
   }
-  if (A(RT, i - 1, j + 1) || A(RT, i, j + 1) || A(DG, i - 1, j) || A(DG, i, j + 1) || A(UP, i, j) || A(UP, i, j + 1)) {
+  if (A(RT, i - 1, j + 1) | A(RT, i, j + 1) | A(DG, i - 1, j) | A(DG, i, j + 1) | A(UP, i, j) | A(UP, i, j + 1)) {
     se(C, UP, d, i, j, ADJZONE);
     se(C, UP, d, i, j + 1, ADJZONE);
     se(Pa, UP, d, ip, jp, ADJZONE);
@@ -632,14 +683,14 @@ __global__ void k_mask_edges_consist2(WLev Pa, WLev C) {
   if (!node_of(Pa.n, 0, d, ip, jp)) return;
   const int i = 2 * ip, j = 2 * jp;
   auto A = [&](int e, int a, int b) { return me(C, e, d, i + a, j + b) >= ADJZONE; };
-  if (A(RT, -2, -2) || A(RT, 0, -2) || A(RT, 0, 2) || A(RT, 2, 2) || A(DG, -2, -2) || A(DG, 0, -2) || A(DG, 0, 0) ||
-      A(DG, 2, 0) || A(UP, 0, -2) || A(UP, 2, -2) || A(UP, 0, 0) || A(UP, 2, 0))
+  if (A(RT, -2, -2) | A(RT, 0, -2) | A(RT, 0, 2) | A(RT, 2, 2) | A(DG, -2, -2) | A(DG, 0, -2) | A(DG, 0, 0) |
+      A(DG, 2, 0) | A(UP, 0, -2) | A(UP, 2, -2) | A(UP, 0, 0) | A(UP, 2, 0))
     se(Pa, RT, d, ip, jp, ADJZONE);
-  if (A(RT, -2, 0) || A(RT, 0, 0) || A(RT, 0, 2) || A(RT, 2, 2) || A(DG, 0, -2) || A(DG, -2, 0) || A(DG, 2, 0) ||
-      A(DG, 0, 2) || A(UP, 0, -2) || A(UP, 0, 0) || A(UP, 2, 0) || A(UP, 2, 2))
+  if (A(RT, -2, 0) | A(RT, 0, 0) | A(RT, 0, 2) | A(RT, 2, 2) | A(DG, 0, -2) | A(DG, -2, 0) | A(DG, 2, 0) |
+      A(DG, 0, 2) | A(UP, 0, -2) | A(UP, 0, 0) | A(UP, 2, 0) | A(UP, 2, 2))
     se(Pa, DG, d, ip, jp, ADJZONE);
-  if (A(RT, 0, 0) || A(RT, 0, 2) || A(RT, -2, 0) || A(RT, -2, 2) || A(DG, 0, 2) || A(DG, 0, 0) || A(DG, -2, -2) ||
-      A(DG, -2, 0) || A(UP, 2, 0) || A(UP, 2, 2) || A(UP, -2, -2) || A(UP, -2, 0))
+  if (A(RT, 0, 0) | A(RT, 0, 2) | A(RT, -2, 0) | A(RT, -2, 2) | A(DG, 0, 2) | A(DG, 0, 0) | A(DG, -2, -2) |
+      A(DG, -2, 0) | A(UP, 2, 0) | A(UP, 2, 2) | A(UP, -2, -2) | A(UP, -2, 0))
     se(Pa, UP, d, ip, jp, ADJZONE);
 }
 
@@ -660,9 +711,10 @@ __global__ void k_mask_prolong_adj(WLev Pa, WLev C) {
 }
 
 // mask_node_trsk with div_grad_stencil (no Laplacian diffusion), nodes [-2, n+1]
-__global__ void k_mask_trsk(WLev g) {
-  int d, i, j;
-  if (!node_of(g.n + 4, -2, d, i, j)) return;
+__global__ void k_mask_trsk(MaskSet S) {
+  int l, d, i, j;
+  if (!mask_node(S, 4, -2, l, d, i, j)) return;
+  const WLev g = mask_level(S, l);
   if (mn(g, d, i, j) < ADJZONE) return;
   const int nb[7][2] = {{0, 0}, {1, 0}, {1, 1}, {0, 1}, {-1, 0}, {-1, -1}, {0, -1}};
   for (int q = 0; q < 7; ++q) sn(g, d, i + nb[q][0], j + nb[q][1], TRSK);
@@ -676,21 +728,23 @@ __global__ void k_mask_trsk(WLev g) {
 
 // check_child_required (src/refine_patch.f90:289-327): one flag per (lozenge,
 // parent patch of side ps, child quadrant c = 0 NE, 1 SE, 2 SW, 3 NW).
+// A warp per flag tests the quadrant's nodes and ring side by side.
 __global__ void k_child_required(WLev g, int ps, unsigned char* __restrict__ out) {
   const int np = g.n / ps;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= 10 * np * np * 4) return;
   const int c = t % 4, r = t / 4;
   const int pi = r % np, pj = (r / np) % np, d = r / (np * np);
   const int ox = (c == 0 || c == 1) ? ps / 2 : 0, oy = (c == 0 || c == 3) ? ps / 2 : 0;
+  const int side = ps / 2 + 4;
   bool req = false;
-  for (int jj = -2; jj <= ps / 2 + 1 && !req; ++jj)
-    for (int ii = -2; ii <= ps / 2 + 1 && !req; ++ii) {
-      const int i = pi * ps + ox + ii, j = pj * ps + oy + jj;
-      req = mn(g, d, i, j) >= ADJZONE || me(g, RT, d, i, j) >= RESTRCT || me(g, DG, d, i, j) >= RESTRCT ||
-            me(g, UP, d, i, j) >= RESTRCT;
-    }
-  out[t] = req ? 1 : 0;
+  for (int q = lane; q < side * side; q += 32) {
+    const int i = pi * ps + ox + q % side - 2, j = pj * ps + oy + q / side - 2;
+    req = req | (mn(g, d, i, j) >= ADJZONE) | (me(g, RT, d, i, j) >= RESTRCT) | (me(g, DG, d, i, j) >= RESTRCT) |
+          (me(g, UP, d, i, j) >= RESTRCT);
+  }
+  req = __any_sync(0xffffffffu, req);
+  if (lane == 0) out[t] = req ? 1 : 0;
 }
 
 }  // namespace wtw

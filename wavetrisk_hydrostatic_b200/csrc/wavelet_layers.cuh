@@ -31,23 +31,32 @@ __device__ __forceinline__ int wn_code(const WLev& L, int d, int i, int j) {
 __device__ __forceinline__ int we_code(const WLev& L, int e, int d, int i, int j) {
   return inr(L, i, j) ? __ldg(L.esrc + e * L.NN + nid(L, d, i, j)) : -1;
 }
-__device__ __forceinline__ double wn(const double* __restrict__ f, int c) { return c < 0 ? 0.0 : f[c]; }
+// No branch (an absent value reads slot 0 and is dropped) and read-only loads: a
+// kernel writes no slot that it reads through these, so that the loads of several
+// layers or edges may pass its stores and be in flight together.
+__device__ __forceinline__ double wn(const double* __restrict__ f, int c) {
+  const double v = __ldg(f + max(c, 0));
+  return c < 0 ? 0.0 : v;
+}
 __device__ __forceinline__ double we(const double* __restrict__ f, int c) {
-  if (c < 0) return 0.0;
-  const double v = f[c >> 1];
-  return (c & 1) ? -v : v;
+  const double v = __ldg(f + (max(c, 0) >> 1));
+  return c < 0 ? 0.0 : (c & 1) ? -v : v;
 }
 
 // Parent (d, ip, jp) of [0, m)^2 and layer range [k0, k1) of this thread: the
 // layers are split into groups of lpt (grid: 10 m^2 threads per group, group
 // slowest), trading the once-per-thread setup against the number of threads.
-__device__ __forceinline__ bool parent_of(int m, int nz, int lpt, int& d, int& ip, int& jp, int& k0, int& k1) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t per = (int64_t)10 * m * m;
+template <int REP>
+__device__ __forceinline__ bool parent_of(int m, int nz, int lpt, int& d, int& ip, int& jp, int& k0, int& k1, int& rep) {
+  // fewer than 2^32 threads: 3 (10 m^2) nz / lpt, the level's fields taking 40 bytes for each
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned per = 10u * m * m;
   const int ng = (nz + lpt - 1) / lpt;
-  if (t >= per * ng) return false;
-  const int g = (int)(t / per);
-  const int r0 = (int)(t - (int64_t)g * per);
+  const int gr = (int)(t / per);
+  if (gr >= ng * REP) return false;
+  const int r0 = (int)(t - gr * per);
+  const int g = gr / REP;
+  rep = gr - g * REP;
   d = r0 / (m * m);
   const int r = r0 - d * m * m;
   jp = r / m;
@@ -55,6 +64,10 @@ __device__ __forceinline__ bool parent_of(int m, int nz, int lpt, int& d, int& i
   k0 = g * lpt;
   k1 = min(nz, k0 + lpt);
   return true;
+}
+__device__ __forceinline__ bool parent_of(int m, int nz, int lpt, int& d, int& ip, int& jp, int& k0, int& k1) {
+  int rep;
+  return parent_of<1>(m, nz, lpt, d, ip, jp, k0, k1, rep);
 }
 
 // Whether the inverse transform rebuilds parent (d, ip, jp) of level Pa: every
@@ -281,61 +294,70 @@ __device__ __forceinline__ double outer_eval(const OuterInterp& O, const double*
 // leaves out the pairs whose slots hold 0 already) and compress_vector's rule
 // (0 where the slot's own mask is below ADJZONE) is applied to them, after the
 // pentagon corrections in the corner parents.
+// A thread takes one of the parent's three edges (edge group slower than the
+// parents, so that a warp stays on one edge); a corner parent's first thread takes
+// all three and the corrections.
 template <int CMP>
 __global__ void __launch_bounds__(128, WL_MINB_OUTER) k_velo_wc_outer_l(WLev Pa, WLev C, int nz, int lpt, ParentList PL) {
-  auto body = [&](int d, int ip, int jp, int k0, int k1) {
+  auto edge = [&](int d, int ip, int jp, int k0, int k1, int e, bool corner) {
     const int i = 2 * ip, j = 2 * jp;
-    const bool corner = (ip == 0 || ip == Pa.n - 1) && (jp == 0 || jp == Pa.n - 1);
-    for (int e = 0; e < 3; ++e) {
-      const int a1 = i + c_end_pt[e][0][0], b1 = j + c_end_pt[e][0][1];
-      const int a2 = i + c_end_pt[e][1][0], b2 = j + c_end_pt[e][1][1];
-      const int x2 = e * C.NN + nid(C, d, a2, b2), x1 = e * C.NN + nid(C, d, a1, b1);
-      if (me(C, e, d, a2, b2) < ADJZONE) {
-        if (CMP == 1)
-          for (int k = k0; k < k1; ++k) {
-            C.wv[(int64_t)k * 3 * C.NN + x2] = 0.0;
-            C.wv[(int64_t)k * 3 * C.NN + x1] = 0.0;
-          }
-        else if (CMP == 2 && me(C, e, d, a1, b1) >= ADJZONE)  // a kept slot that the pair leaves at 0
-          for (int k = k0; k < k1; ++k) C.wv[(int64_t)k * 3 * C.NN + x1] = 0.0;
-        continue;
-      }
-      const bool keep1 = CMP == 0 || corner || me(C, e, d, a1, b1) >= ADJZONE;
-      OuterInterp O;
-      outer_interp(O, Pa, C, d, ip, jp, a2, b2, e);
-      const int cv = we_code(C, e, d, a2, b2);
-      for (int k = k0; k < k1; ++k) {
-        const double* vp = Pa.sv + (int64_t)k * 3 * Pa.NN;
-        const double* v = C.sv + (int64_t)k * 3 * C.NN;
-        double* wc = C.wv + (int64_t)k * 3 * C.NN;
-        double t0;
-        const double u = outer_eval(O, vp, t0);
-        const double w = we(v, cv) - u;
-        wc[x2] = w;
-        wc[x1] = keep1 ? -w : 0.0;
-      }
+    const int a1 = i + c_end_pt[e][0][0], b1 = j + c_end_pt[e][0][1];
+    const int a2 = i + c_end_pt[e][1][0], b2 = j + c_end_pt[e][1][1];
+    const int x2 = e * C.NN + nid(C, d, a2, b2), x1 = e * C.NN + nid(C, d, a1, b1);
+    const int m2 = me(C, e, d, a2, b2), m1 = me(C, e, d, a1, b1);
+    if (m2 < ADJZONE) {
+      if (CMP == 1)
+        for (int k = k0; k < k1; ++k) {
+          C.wv[(int64_t)k * 3 * C.NN + x2] = 0.0;
+          C.wv[(int64_t)k * 3 * C.NN + x1] = 0.0;
+        }
+      else if (CMP == 2 && m1 >= ADJZONE)  // a kept slot that the pair leaves at 0
+        for (int k = k0; k < k1; ++k) C.wv[(int64_t)k * 3 * C.NN + x1] = 0.0;
+      return;
     }
-    if (corner) {
-      for (int k = k0; k < k1; ++k)
-        penta_compute(Pa, C, Pa.sv + (int64_t)k * 3 * Pa.NN, C.wv + (int64_t)k * 3 * C.NN, d, ip, jp);
-      if (CMP)
-        for (int e = 0; e < 3; ++e)
-  #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int a = i + c_end_pt[e][h][0], b = j + c_end_pt[e][h][1];
-            if (me(C, e, d, a, b) >= ADJZONE) continue;
-            const int x = e * C.NN + nid(C, d, a, b);
-            for (int k = k0; k < k1; ++k) C.wv[(int64_t)k * 3 * C.NN + x] = 0.0;
-          }
+    const bool keep1 = CMP == 0 || corner || m1 >= ADJZONE;
+    OuterInterp O;
+    outer_interp(O, Pa, C, d, ip, jp, a2, b2, e);
+    const int cv = we_code(C, e, d, a2, b2);
+    for (int k = k0; k < k1; ++k) {
+      const double* vp = Pa.sv + (int64_t)k * 3 * Pa.NN;
+      const double* v = C.sv + (int64_t)k * 3 * C.NN;
+      double* wc = C.wv + (int64_t)k * 3 * C.NN;
+      double t0;
+      const double u = outer_eval(O, vp, t0);
+      const double w = we(v, cv) - u;
+      wc[x2] = w;
+      wc[x1] = keep1 ? -w : 0.0;
     }
   };
+  auto body = [&](int d, int ip, int jp, int k0, int k1, int e) {
+    const bool corner = (ip == 0 || ip == Pa.n - 1) && (jp == 0 || jp == Pa.n - 1);
+    if (!corner) {
+      edge(d, ip, jp, k0, k1, e, false);
+      return;
+    }
+    if (e) return;
+    const int i = 2 * ip, j = 2 * jp;
+    for (int q = 0; q < 3; ++q) edge(d, ip, jp, k0, k1, q, true);
+    for (int k = k0; k < k1; ++k)
+      penta_compute(Pa, C, Pa.sv + (int64_t)k * 3 * Pa.NN, C.wv + (int64_t)k * 3 * C.NN, d, ip, jp);
+    if (CMP)
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int a = i + c_end_pt[q][h][0], b = j + c_end_pt[q][h][1];
+          if (me(C, q, d, a, b) >= ADJZONE) continue;
+          const int x = q * C.NN + nid(C, d, a, b);
+          for (int k = k0; k < k1; ++k) C.wv[(int64_t)k * 3 * C.NN + x] = 0.0;
+        }
+  };
   if (PL.ids) {
-    for_parents(Pa.n, Pa.n, nz, lpt, PL, body);
+    for_parents<3>(Pa.n, Pa.n, nz, lpt, PL, body);
     return;
   }
-  int d, ip, jp, k0, k1;
-  if (!parent_of(Pa.n, nz, lpt, d, ip, jp, k0, k1)) return;
-  body(d, ip, jp, k0, k1);
+  int d, ip, jp, k0, k1, e;
+  if (!parent_of<3>(Pa.n, nz, lpt, d, ip, jp, k0, k1, e)) return;
+  body(d, ip, jp, k0, k1, e);
 }
 
 // Interp_inner_velo (src/wavelet.f90:1005-1062) of parent (ip, jp): parent

@@ -51,25 +51,35 @@ unsigned pgrid(K kernel, int threads, unsigned dense) {
 }
 const ParentList kNoList{nullptr, nullptr};
 
-// Blocks of LIST_B candidates of the largest level (the list compaction's scratch).
-size_t mx_nn_blocks(wt_handle* h) {
-  size_t mx = 0;
-  for (int l = h->level_start; l <= h->level_end; ++l) mx = std::max(mx, (size_t)h->at(l).NN);
-  return (mx + LIST_B - 1) / LIST_B;
+inline int list_blocks(int64_t n) { return (int)((n + LIST_B - 1) / LIST_B); }
+// Blocks of every node and parent list together (the list compaction's scratch).
+size_t all_list_blocks(wt_handle* h) {
+  size_t b = 0;
+  for (int l = h->level_start; l <= h->level_end; ++l) b += 2 * (size_t)list_blocks(h->at(l).NN);
+  return b;
 }
 
-// An ascending work list of the candidates c into ids, its count into *count
-// (stream-ordered; scratch: the context's block counts and offsets).
-template <class Cand>
-void build_list(wt_handle* h, const Cand& c, int n, int* ids, int* count) {
+void add_list(ListSet& S, int parent, const DevLevel& D, const unsigned char* map, int* ids, int* count) {
+  const int q = S.nl++;
+  S.parent[q] = parent;
+  S.n[q] = D.n;
+  S.nsrc[q] = D.nsrc;
+  S.map[q] = map;
+  S.ids[q] = ids;
+  S.count[q] = count;
+  S.bstart[q + 1] = S.bstart[q] + list_blocks(parent ? (int64_t)10 * (D.n + 1) * (D.n + 1) : D.NN);
+}
+// The ascending work lists of S, their counts on the device (stream-ordered).
+void build_lists(wt_handle* h, const ListSet& S) {
+  if (S.nl == 0) return;
   WavCtx* W = ctx(h);
-  const int nb = (n + LIST_B - 1) / LIST_B;
   int* bcnt = W->lscr;
   int* boff = W->lscr + W->lscr_n / 2;
   cudaStream_t s = h->stream;
-  k_list_count<<<nb, LIST_B, 0, s>>>(c, bcnt);
-  k_list_scan<<<1, LIST_B, 0, s>>>(nb, bcnt, boff, count);
-  k_list_write<<<nb, LIST_B, 0, s>>>(c, boff, ids);
+  const unsigned nb = (unsigned)S.bstart[S.nl];
+  k_list_count<<<nb, LIST_B, 0, s>>>(S, bcnt);
+  k_list_scan<<<S.nl, LIST_B, 0, s>>>(S, bcnt, boff);
+  k_list_write<<<nb, LIST_B, 0, s>>>(S, boff);
 }
 
 #define CKW(x)                                  \
@@ -173,7 +183,8 @@ void launch_velo_wc(wt_handle* h, int l, cudaStream_t s, cudaStream_t si) {
   const int np = h->at(l).n, nz = h->nz;
   const unsigned g = nbl((int64_t)10 * np * np, nz);
   const ParentList PL = CMP == 2 ? wt_level_plist(h, l) : kNoList;
-  k_velo_wc_outer_l<CMP><<<PL.ids ? pgrid(k_velo_wc_outer_l<CMP>, TPBL, g) : g, TPBL, 0, s>>>(
+  const unsigned g3 = nbl((int64_t)30 * np * np, nz);  // a thread per edge
+  k_velo_wc_outer_l<CMP><<<PL.ids ? pgrid(k_velo_wc_outer_l<CMP>, TPBL, g3) : g3, TPBL, 0, s>>>(
       view(h, l), view(h, l + 1), nz, lpt_for(nz), PL);
   k_velo_wc_inner_l<CMP><<<PL.ids ? pgrid(k_velo_wc_inner_l<CMP>, TPBL, g) : g, TPBL, 0, si>>>(
       view(h, l), view(h, l + 1), nz, lpt_for(nz), PL);
@@ -361,7 +372,7 @@ int wt_wavelet_setup(wt_handle* h) {
     CKW(W->alloc(&W->need[1], tot));
     CKW(W->alloc(&W->list, tot));
     CKW(W->alloc(&W->list_cnt, W->L.size()));
-    W->lscr_n = 2 * (mx_nn_blocks(h) + 1);
+    W->lscr_n = 2 * all_list_blocks(h);
     CKW(W->alloc(&W->lscr, W->lscr_n));
     size_t ptot = 0, mx = 0;
     W->rec_off.assign(W->L.size(), 0);
@@ -597,6 +608,25 @@ void mask_tol(wt_handle* h, int l, int st, int en, int level_fill) {
                                                                                      W->tree_ps);
 }
 inline unsigned nodes_blocks(int m) { return nb((int64_t)10 * m * m); }
+// The masks of levels a .. b with (n + add)^2 threads a lozenge each.
+MaskSet mask_set(wt_handle* h, int a, int b, int add) {
+  MaskSet S{};
+  for (int l = a; l <= b; ++l) {
+    const int q = S.nl++, m = h->at(l).n + add;
+    const WavLevel& V = ctx(h)->L[l - h->level_start];
+    S.n[q] = h->at(l).n;
+    S.mask_n[q] = V.mask_n;
+    S.mask_e[q] = V.mask_e;
+    S.start[q + 1] = S.start[q] + 10 * m * m;
+  }
+  return S;
+}
+template <class K>
+void mask_sweep(wt_handle* h, K kernel, int a, int b, int add) {
+  if (a > b) return;
+  const MaskSet S = mask_set(h, a, b, add);
+  kernel<<<nb(S.start[S.nl]), TPB, 0, h->stream>>>(S);
+}
 }  // namespace
 
 extern "C" {
@@ -635,7 +665,7 @@ static int mask_phase1(wt_handle* h, int level_fill, int max_level, int patch_si
   const int ls = h->level_start;
   cudaStream_t s = h->stream;
   const bool child_required = dreq != nullptr;
-  for (int l = ls + 1; l <= le; ++l) k_mask_zero<<<nb(3 * h->at(l).NN), TPB, 0, s>>>(view(h, l));
+  mask_sweep(h, k_mask_zero, ls + 1, le, 4);
   // mask_active
   auto tol = [&](int l, int st, int en) { mask_tol(h, l, st, en, level_fill); };
   tol(le, 0, 1);
@@ -643,19 +673,17 @@ static int mask_phase1(wt_handle* h, int level_fill, int max_level, int patch_si
   for (int l = le - 1; l >= ls; --l) {
     tol(l, -1, 2);
     k_mask_parent<<<nodes_blocks(h->at(l).n + 1), TPB, 0, s>>>(view(h, l), view(h, l + 1));
-    comm_masks(h);
+    comm_masks(h);  // the last one is also mask_active's own at its end
   }
+  mask_sweep(h, k_mask_adj_same, ls, le, 1);
   comm_masks(h);
-  for (int l = ls; l <= le; ++l) k_mask_adj_same<<<nodes_blocks(h->at(l).n + 1), TPB, 0, s>>>(view(h, l));
-  comm_masks(h);
-  for (int l = ls; l <= std::min(le, max_level - 1); ++l)
-    k_mask_restrict_flux<<<nodes_blocks(h->at(l).n), TPB, 0, s>>>(view(h, l));
+  mask_sweep(h, k_mask_restrict_flux, ls, std::min(le, max_level - 1), 0);
   comm_masks(h);
   if (child_required) {
     int64_t o = 0;
     for (int l = ls; l <= req_hi; ++l) {
       const int64_t cnt = (int64_t)10 * (h->at(l).n / patch_size) * (h->at(l).n / patch_size) * 4;
-      k_child_required<<<nb(cnt), TPB, 0, s>>>(view(h, l), patch_size, dreq + o);
+      k_child_required<<<nb(32 * cnt), TPB, 0, s>>>(view(h, l), patch_size, dreq + o);
       o += cnt;
     }
   }
@@ -710,7 +738,7 @@ static int mask_phase2(wt_handle* h, int le) {
   if (ls + 1 <= le) k_mask_nodes_all<<<nodes_blocks(h->at(ls + 1).n + 1), TPB, 0, s>>>(view(h, ls + 1));
   comm_masks(h);
   // mask_trsk
-  for (int l = ls; l <= le; ++l) k_mask_trsk<<<nodes_blocks(h->at(l).n + 4), TPB, 0, s>>>(view(h, l));
+  mask_sweep(h, k_mask_trsk, ls, le, 4);
   CKW(cudaGetLastError());
   ctx(h)->zero_ok = false;  // new masks: compress_wavelets has not run under them
   return wt_level_need_build(h);
@@ -769,10 +797,11 @@ int wt_level_need_build(wt_handle* h) {
     const DevLevel& D = h->at(l);
     return TreeLev{D.n, D.P, (int)D.NN, D.nsrc, W->tree + W->tree_off[l - h->level_start]};
   };
-  if (tree)
-    for (int l = h->level_start + 1; l <= h->level_end; ++l)
-      k_need_tree<<<nb(h->at(l).NN), TPB, 0, s>>>(tl(l), W->tree_ps,
-                                                  W->need[NEED_R & 1] + W->need_off[l - h->level_start]);
+  if (tree) {
+    TreeSet E{};
+    for (int q = 1; q < S.nl; ++q) E.exist[q] = W->tree + W->tree_off[q];
+    k_need_tree<<<g, TPB, 0, s>>>(S, E, W->tree_ps, NEED_R);
+  }
   // parents rebuilt by the intermediate stages' inverse transforms, finest first
   auto ml = [&](int l) {
     const DevLevel& D = h->at(l);
@@ -785,30 +814,26 @@ int wt_level_need_build(wt_handle* h) {
     const unsigned char* nc = W->need[NEED_R & 1] + W->need_off[c - h->level_start];
     const unsigned char* rc = c < h->level_end ? W->recpar + W->rec_off[c - h->level_start] : nullptr;
     unsigned char* rp = W->recpar + W->rec_off[l - h->level_start];
-    k_map_or<<<nb(Lc.NN), TPB, 0, s>>>(Lc.NN, nc, rc, A);
-    k_map_dilate<<<nb(Lc.NN), TPB, 0, s>>>(Lc, A, B);
-    k_map_dilate<<<nb(Lc.NN), TPB, 0, s>>>(Lc, B, A);  // rec(c)
-    k_map_up<<<nb(Lp.NN), TPB, 0, s>>>(Lc, Lp, A, B);
-    k_map_dilate<<<nb(Lp.NN), TPB, 0, s>>>(Lp, B, A);
-    k_map_dilate<<<nb(Lp.NN), TPB, 0, s>>>(Lp, A, rp);  // recpar(l)
-    if (tree && W->recfin)
-      k_map_tree_par<<<nb(Lp.NN), TPB, 0, s>>>(Lp, tl(c), W->tree_ps, rp, W->recfin + W->rec_off[l - h->level_start]);
+    k_map_dilate<<<nb(Lc.NN), TPB, 0, s>>>(Lc, nc, rc, B);
+    k_map_dilate<<<nb(Lc.NN), TPB, 0, s>>>(Lc, B, nullptr, A);  // rec(c)
+    k_map_up_dilate<<<nb(Lp.NN), TPB, 0, s>>>(Lc, Lp, A, B);
+    if (tree && W->recfin)  // recpar(l), and with it recfin(l)
+      k_map_tree_par<<<nb(Lp.NN), TPB, 0, s>>>(Lp, tl(c), W->tree_ps, B, rp, W->recfin + W->rec_off[l - h->level_start]);
+    else
+      k_map_dilate<<<nb(Lp.NN), TPB, 0, s>>>(Lp, B, nullptr, rp);
   }
-  // with a patch tree, the parent levels' work lists from recfin
+  // the parent levels' work lists from recfin (patch tree) and those of the levels above level_start
+  ListSet T{};
   if (tree && W->recfin)
     for (int l = h->level_start; l < h->level_end; ++l) {
-      const int q = l - h->level_start, m = h->at(l).n + 1;
-      const DevLevel& D = h->at(l);
-      build_list(h, ParentCand{D.n, D.P, D.nsrc, W->recfin + W->rec_off[q]}, 10 * m * m, W->plist_par + W->rec_off[q],
-                 W->plist_cnt + q);
+      const int q = l - h->level_start;
+      add_list(T, 1, h->at(l), W->recfin + W->rec_off[q], W->plist_par + W->rec_off[q], W->plist_cnt + q);
     }
-  // work lists of the levels above level_start
   for (int l = h->level_start + 1; l <= h->level_end; ++l) {
     const int q = l - h->level_start;
-    const DevLevel& D = h->at(l);
-    build_list(h, NodeCand{(int)D.NN, D.nsrc, W->need[NEED_R & 1] + W->need_off[q]}, (int)D.NN,
-               W->list + W->need_off[q], W->list_cnt + q);
+    add_list(T, 0, h->at(l), W->need[NEED_R & 1] + W->need_off[q], W->list + W->need_off[q], W->list_cnt + q);
   }
+  build_lists(h, T);
   CKW(cudaGetLastError());
   W->need_ok = true;
   W->recfin_ok = tree && W->recfin;
