@@ -23,6 +23,7 @@
 #pragma once
 #include <cstdint>
 
+#include "trisk_kernels.cuh"
 #include "trisk_read.cuh"
 #include "trisk_types.cuh"
 

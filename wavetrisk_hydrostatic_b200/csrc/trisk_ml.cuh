@@ -125,13 +125,15 @@ __device__ __forceinline__ void trend_ml_node(const LevelDev& L, int nz, const T
       const double th0 = th[id], thE = th[idE], thNE = th[idNE], thN = th[idN];
       const double* __restrict__ B = io.bern + ko;
       const double* __restrict__ F = io.phik + ko;
-      const double gB0 = (B[idE] - B[id]) / len3[0], gB1 = (B[id] - B[idNE]) / len3[1],
-                   gB2 = (B[idN] - B[id]) / len3[2];
+      const double y0 = 1.0 / len3[0], y1 = 1.0 / len3[1], y2 = 1.0 / len3[2];
+      const double gB0 = div_by(B[idE] - B[id], len3[0], y0), gB1 = div_by(B[id] - B[idNE], len3[1], y1),
+                   gB2 = div_by(B[idN] - B[id], len3[2], y2);
       const double xE = -F[idE], x0 = -F[id], xNE = -F[idNE], xN = -F[idN];
-      const double gE0 = (xE - x0) / len3[0], gE1 = (x0 - xNE) / len3[1], gE2 = (xN - x0) / len3[2];
-      dv3[0] = s[0] / len3[0] - gB0 - interp(th0, thE) * gE0;
-      dv3[1] = s[1] / len3[1] - gB1 - interp(th0, thNE) * gE1;
-      dv3[2] = s[2] / len3[2] - gB2 - interp(th0, thN) * gE2;
+      const double gE0 = div_by(xE - x0, len3[0], y0), gE1 = div_by(x0 - xNE, len3[1], y1),
+                   gE2 = div_by(xN - x0, len3[2], y2);
+      dv3[0] = div_by(s[0], len3[0], y0) - gB0 - interp(th0, thE) * gE0;
+      dv3[1] = div_by(s[1], len3[1], y1) - gB1 - interp(th0, thNE) * gE1;
+      dv3[2] = div_by(s[2], len3[2], y2) - gB2 - interp(th0, thN) * gE2;
     }
     if (io.dv) {
 #pragma unroll

@@ -42,35 +42,51 @@ __device__ __forceinline__ bool layer_node(const LevelDev& L, int nz, int& k, in
   return true;
 }
 
-// Grid of a persistent kernel: the blocks of NODE_TILE threads the device
+// Grid of a persistent kernel: the blocks of `threads` threads the device
 // keeps resident at once (never more than `dense`, the blocks of the dense
 // launch it replaces).  Host code.
 template <class K>
-inline unsigned persistent_grid(K kernel, unsigned dense) {
+inline unsigned persistent_grid(K kernel, unsigned dense, int threads = NODE_TILE) {
   int dev = 0, sms = 0, per = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, NODE_TILE, 0) != cudaSuccess || per < 1)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0) != cudaSuccess || per < 1)
     return dense;
   const unsigned g = (unsigned)sms * (unsigned)per;
   return g < dense ? g : dense;
 }
 
-// Work-list items: (chunk of NODE_TILE entries, layer) layer-fastest as in
-// the dense launches; a persistent kernel strides w over [0, list_items) by the
-// grid and takes entry (k, id, i, j) of item w where list_entry says so.
+// Work-list items: (chunk of TILE entries, layer) layer-fastest as in the dense
+// launches; a persistent kernel strides w over [0, list_items) by the grid and
+// takes entry (k, id, i, j) of item w where list_entry says so.
+template <int TILE = NODE_TILE>
 __device__ __forceinline__ int64_t list_items(int cnt, int nz) {
-  return (int64_t)((cnt + NODE_TILE - 1) / NODE_TILE) * nz;
+  return (int64_t)((cnt + TILE - 1) / TILE) * nz;
 }
+template <int TILE = NODE_TILE>
 __device__ __forceinline__ bool list_entry(const LevelDev& L, int nz, const NodeList& W, int cnt, int64_t w, int& k,
                                            int& id, int& i, int& j) {
   const int chunk = (int)(w / nz);
   k = (int)(w - (int64_t)chunk * nz);
-  const int e = chunk * NODE_TILE + threadIdx.x;
+  const int e = chunk * TILE + threadIdx.x;
   if (e >= cnt) return false;
   id = __ldg(W.ids + e);
   node_ij(L, id, i, j);
   return true;
+}
+
+// a / b from y = RN(1 / b) (__drcp_rn or 1.0 / b), correctly rounded: the quotient
+// estimate a y is within two units in the last place, one residual correction
+// makes it faithful and, by Markstein's theorem (P. Markstein, IBM J. Res. Dev.
+// 34(1), 1990), the second rounds it as the division does, short of underflow in
+// the residual (|a| below 2^-960 or so).  A zero, infinite or NaN estimate is returned
+// as it is, with its sign.  Five dependent operations replace a division's some
+// fifteen instructions wherever quotients share a divisor.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = fma(fma(-b, q0, a), y, q0);
+  const double q2 = fma(fma(-b, q1, a), y, q1);
+  return ((unsigned)__double2hiint(q0) & 0x7ff00000u) - 0x00100000u < 0x7fe00000u ? q2 : q0;
 }
 
 // Readers of the state through the ghost remap.
@@ -106,6 +122,15 @@ __device__ __forceinline__ void weights5(const LevelDev& L, int id, int offs, do
   for (int q = 0; q < 5; ++q) wgt[q] = 0.5 - wgt[q] * hinv;
   w[0] = wgt[0]; w[1] = -wgt[1]; w[2] = wgt[2]; w[3] = -wgt[3]; w[4] = wgt[4];
 }
+
+// The ten edges (edge, node offset) of Qperp at the RT, DG and UP edge of a node, in
+// the reference's order of summation.
+#define WT_QPERP_RT(X) X(0, DG, 0, 0) X(1, UP, 0, 0) X(2, RT, -1, 0) X(3, DG, -1, -1) X(4, UP, 0, -1) \
+                       X(5, DG, 0, -1) X(6, UP, 1, -1) X(7, RT, 1, 0) X(8, DG, 1, 0) X(9, UP, 1, 0)
+#define WT_QPERP_DG(X) X(0, UP, 0, 0) X(1, RT, -1, 0) X(2, DG, -1, -1) X(3, UP, 0, -1) X(4, RT, 0, 0) \
+                       X(5, UP, 1, 0) X(6, RT, 1, 1) X(7, DG, 1, 1) X(8, UP, 1, 1) X(9, RT, 0, 1)
+#define WT_QPERP_UP(X) X(0, RT, -1, 0) X(1, DG, -1, -1) X(2, UP, 0, -1) X(3, RT, 0, 0) X(4, DG, 0, 0) \
+                       X(5, RT, 0, 1) X(6, DG, 0, 1) X(7, UP, 0, 1) X(8, RT, -1, 1) X(9, DG, -1, 0)
 
 // Qperp (src/ops.f90:834-901): the TRiSK Coriolis term of the three edges of
 // node id from the mass flux hm and qe of one layer (ghost edges of hm read

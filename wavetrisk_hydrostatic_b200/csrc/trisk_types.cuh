@@ -49,6 +49,20 @@ struct Step1Maps {
   CUtensorMap len, ped, part, cor;  // plane = edge orientation / area part / triangle
 };
 
+// Tensor maps of the pipelined single-level trend (trisk_pipe.cuh): FP64 fluxes
+// (TrendMapsD) or FP32 ones (TrendMapsF: hfm, hft, qe, theta, ke in FP32).
+// A state and what step1 reads beside it (PipeStateMaps).
+struct PipeStateMaps {
+  CUtensorMap mass, temp, velo, mean_m, mean_t, phik, pterm;
+};
+struct TrendMapsD {
+  CUtensorMap hfm, hft, qe, theta, bern, phik;
+};
+struct TrendMapsF {
+  CUtensorMap hfm, hft, qe, theta, ke;
+  CUtensorMap phik, pterm;
+};
+
 // Inputs and outputs of the trend kernels (trisk_kernels.cuh, trisk_tma.cuh).
 struct TrendIO {
   const double* __restrict__ theta;  // Theta/rho of the stage state at [0, n]^2 (k_step1)
@@ -72,6 +86,14 @@ struct TrendIO {
 
 struct Phys {
   double grav, ref_density, p_top;
+};
+
+// Ghost copies, (destination, signed source) pairs of what the pipelined kernels read:
+// nodes and edges of [-1, n+1]^2 of a state, edges of [-1, n]^2 of the fluxes (the
+// first n_f of the list).
+struct GhostLists {
+  const int2 *nodes, *edges;
+  int n_nodes, n_edges, n_f;
 };
 
 }  // namespace wtk

@@ -12,6 +12,7 @@
 #include "../../include/wavetrisk_gpu.h"
 #include "trisk_kernels.cuh"
 #include "trisk_mixed.cuh"
+#include "trisk_pipe.cuh"
 #include "trisk_tma.cuh"
 #include "wt_handle.cuh"
 
@@ -66,17 +67,21 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return encode;
 }
 
-// Tensor map of a top-level field of `planes` planes of NN doubles.
-static bool top_map(wt_handle* h, CUtensorMap* m, const double* base, int planes) {
+// Tensor map of a top-level field of `planes` planes of NN values (double or
+// float), boxes of bx x by nodes.
+template <class T>
+static bool top_map(wt_handle* h, CUtensorMap* m, const T* base, int planes, int bx = TB_X, int by = TB_Y) {
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return false;
   const DevLevel& D = h->top();
+  const cuuint64_t sz = sizeof(T);
   const cuuint64_t dims[4] = {(cuuint64_t)D.P, (cuuint64_t)D.P, 10, (cuuint64_t)planes};
-  const cuuint64_t strides[3] = {(cuuint64_t)D.P * 8, (cuuint64_t)D.P * D.P * 8, (cuuint64_t)D.NN * 8};
-  const cuuint32_t box[4] = {(cuuint32_t)TB_X, (cuuint32_t)TB_Y, 1, 1};
+  const cuuint64_t strides[3] = {(cuuint64_t)D.P * sz, (cuuint64_t)D.P * D.P * sz, (cuuint64_t)D.NN * sz};
+  const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, 1, 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
-  return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(base), dims, strides, box, elem,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  return encode(m, sz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                const_cast<T*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -84,10 +89,10 @@ static bool top_map(wt_handle* h, CUtensorMap* m, const double* base, int planes
 static bool step1_maps(wt_handle* h, const double* m, const double* t, const double* v, Step1Maps* S) {
   const DevLevel& D = h->top();
   const int nz = h->nz;
-  return top_map(h, &S->mass, m, nz) && top_map(h, &S->temp, t, nz) && top_map(h, &S->velo, v, 3 * nz) &&
-         top_map(h, &S->mean_m, h->mean_m, nz) && top_map(h, &S->mean_t, h->mean_t, nz) &&
-         top_map(h, &S->len, D.len, 3) && top_map(h, &S->ped, D.pedlen, 3) && top_map(h, &S->part, D.part, 6) &&
-         top_map(h, &S->cor, D.coriolis, 2);
+  auto mk = [&](CUtensorMap* map, const double* base, int planes) { return top_map(h, map, base, planes); };
+  return mk(&S->mass, m, nz) && mk(&S->temp, t, nz) && mk(&S->velo, v, 3 * nz) && mk(&S->mean_m, h->mean_m, nz) &&
+         mk(&S->mean_t, h->mean_t, nz) && mk(&S->len, D.len, 3) && mk(&S->ped, D.pedlen, 3) &&
+         mk(&S->part, D.part, 6) && mk(&S->cor, D.coriolis, 2);
 }
 
 int wt_make_step1_maps(wt_handle* h, const double* m, const double* t, const double* v, wtk::Step1Maps* out) {
@@ -107,26 +112,87 @@ int wt_make_trend_maps(wt_handle* h, const double* hfm, const double* hft, const
   return ok ? WT_OK : WT_ERR_CUDA;
 }
 
+// Tensor maps and launch limits of the TMA-staged kernels on the top level.
 static int make_trend_maps(wt_handle* h) {
   const DevLevel& D = h->top();
-  auto mk = [&](CUtensorMap* m, const double* base, int planes) { return top_map(h, m, base, planes); };
-  TrendMaps& M = h->maps;
   const int nz = h->nz;
-  bool ok = mk(&M.hfm, h->hfm, 3 * nz) && mk(&M.hft, h->hft, 3 * nz) && mk(&M.qe, h->qe, 3 * nz) &&
-                  mk(&M.theta, h->theta, nz) && mk(&M.bern, h->bern, nz) && mk(&M.phik, h->phik, nz) &&
-                  mk(&M.part, D.part, 6) && mk(&M.hinv, D.hex_inv, 1);
+  auto mk = [&](CUtensorMap* m, const double* base, int planes) {
+    return top_map(h, m, base, planes, PBX, PipeTile::BY);
+  };
+  TrendMapsD& M = h->pmaps;
+  bool ok = step1_maps(h, h->mass, h->temp, h->velo, &h->s1maps) && mk(&M.hfm, h->hfm, 3 * nz) &&
+            mk(&M.hft, h->hft, 3 * nz) && mk(&M.qe, h->qe, 3 * nz) && mk(&M.theta, h->theta, nz) &&
+            mk(&M.bern, h->bern, nz) && mk(&M.phik, h->phik, nz);
   double* SM[3] = {h->mass, h->m1, h->m2};
   double* ST[3] = {h->temp, h->t1, h->t2};
   double* SV[3] = {h->velo, h->v1, h->v2};
-  for (int b = 0; b < 3 && ok; ++b) ok = step1_maps(h, SM[b], ST[b], SV[b], &h->s1maps[b]);
+  for (int b = 0; b < 3 && ok; ++b) {
+    PipeStateMaps& S = h->p1maps[b];
+    ok = mk(&S.mass, SM[b], nz) && mk(&S.temp, ST[b], nz) && mk(&S.velo, SV[b], 3 * nz) && mk(&S.mean_m, h->mean_m, nz) &&
+         mk(&S.mean_t, h->mean_t, nz) && mk(&S.phik, h->phik, nz) && mk(&S.pterm, h->pterm, nz);
+  }
   if (!ok) {
     std::fprintf(stderr, "wavetrisk_gpu: tensor map encoding failed\n");
     return WT_ERR_CUDA;
   }
-  CK(cudaFuncSetAttribute(k_step1_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, STEP1_TMA_SMEM));
-  CK(cudaFuncSetAttribute(k_trend_tma<MODE_RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, TREND_TMA_SMEM));
-  CK(cudaFuncSetAttribute(k_trend_tma<MODE_TREND>, cudaFuncAttributeMaxDynamicSharedMemorySize, TREND_TMA_SMEM));
-  CK(cudaFuncSetAttribute(k_trend_tma<MODE_ML>, cudaFuncAttributeMaxDynamicSharedMemorySize, TREND_TMA_SMEM));
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&h->pipe_slots, cudaDevAttrMultiProcessorCount, dev));  // one block a SM
+  const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  CK(cudaFuncSetAttribute(k_step1_tma, smem, STEP1_TMA_SMEM));
+  CK(cudaFuncSetAttribute(k_trend_tma, smem, TREND_TMA_SMEM));
+  CK(cudaFuncSetAttribute(k_step1_pipe<double>, smem, Step1Pipe<double>::SMEM));
+  CK(cudaFuncSetAttribute(k_step1_pipe<float>, smem, Step1Pipe<float>::SMEM));
+  CK(cudaFuncSetAttribute(k_trend_pipe<double, MODE_RK>, smem, TrendPipe<double, MODE_RK>::SMEM));
+  CK(cudaFuncSetAttribute(k_trend_pipe<double, MODE_TREND>, smem, TrendPipe<double, MODE_TREND>::SMEM));
+  CK(cudaFuncSetAttribute(k_trend_pipe<float, MODE_RK>, smem, TrendPipe<float, MODE_RK>::SMEM));
+  CK(cudaFuncSetAttribute(k_trend_pipe<float, MODE_TREND>, smem, TrendPipe<float, MODE_TREND>::SMEM));
+  return WT_OK;
+}
+
+// The pipelined kernels' ghost lists of the top level, from its halo lists and remaps.
+static int make_ghost_lists(wt_handle* h, const DevLevel& D, const std::vector<int2>& hn, const std::vector<int3>& he,
+                            const std::vector<int>& nsrc, const std::vector<int>& esrc) {
+  std::vector<int2> nodes, edges, outer;
+  const int NN = (int)D.NN, P = D.P;
+  auto within = [&](int x, int hi) {  // node slot x lies in [-1, hi]^2
+    const int r = x % (P * P), i = r % P - 2, j = r / P - 2;
+    return i >= -1 && j >= -1 && i <= hi && j <= hi;
+  };
+  for (const int2& e : hn)
+    if (nsrc[e.x] != e.x && within(e.x, D.n + 1)) nodes.push_back(make_int2(e.x, 2 * nsrc[e.x]));
+  for (const int3& e : he) {
+    const int x = e.x % NN;
+    if (esrc[e.x] == 2 * e.x || !within(x, D.n + 1)) continue;
+    (within(x, D.n) ? edges : outer).push_back(make_int2(e.x, esrc[e.x]));
+  }
+  h->ghosts.n_f = (int)edges.size();
+  edges.insert(edges.end(), outer.begin(), outer.end());
+  int2 *dn = nullptr, *de = nullptr;
+  CK(cudaMalloc(&dn, sizeof(int2) * std::max<size_t>(1, nodes.size())));
+  h->ghosts.nodes = dn;
+  CK(cudaMalloc(&de, sizeof(int2) * std::max<size_t>(1, edges.size())));
+  h->ghosts.edges = de;
+  CK(cudaMemcpy(dn, nodes.data(), sizeof(int2) * nodes.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(de, edges.data(), sizeof(int2) * edges.size(), cudaMemcpyHostToDevice));
+  h->ghosts.n_nodes = (int)nodes.size();
+  h->ghosts.n_edges = (int)edges.size();
+  return WT_OK;
+}
+
+// Trend input maps of the FP32 flux arrays.
+static int make_f32_maps(wt_handle* h) {
+  const int nz = h->nz;
+  TrendMapsF& M = h->fmaps;
+  auto mk = [&](CUtensorMap* m, const float* base, int planes) { return top_map(h, m, base, planes, FBX, PipeTile::BY); };
+  const bool ok = mk(&M.hfm, h->hfm32, 3 * nz) && mk(&M.hft, h->hft32, 3 * nz) && mk(&M.qe, h->qe32, 3 * nz) &&
+                  mk(&M.theta, h->theta32, nz) && mk(&M.ke, h->ke32, nz) &&
+                  top_map(h, &M.phik, h->phik, nz, PBX, PipeTile::BY) &&
+                  top_map(h, &M.pterm, h->pterm, nz, PBX, PipeTile::BY);
+  if (!ok) {
+    std::fprintf(stderr, "wavetrisk_gpu: tensor map encoding failed\n");
+    return WT_ERR_CUDA;
+  }
   return WT_OK;
 }
 
@@ -145,6 +211,14 @@ int wt_create(const wt_grid_desc* desc, wt_handle** out) {
   const int nlev = desc->level_end - desc->level_start + 1;
   h->lev.resize(nlev);
   int rc = WT_OK;
+  // Kernel family: TMA-staged tiles from n = 64 up; below that the tiles are mostly
+  // empty and the L1 kernels are faster (J5 x 8, 100 steps: 10.4 ms against 11.4).
+  // WAVETRISK_TREND_KERNEL=tma|plain forces either.
+  h->trend_variant = desc->level_end >= 6 ? 0 : 1;
+  if (const char* tv = std::getenv("WAVETRISK_TREND_KERNEL")) {
+    if (std::strcmp(tv, "tma") == 0) h->trend_variant = 0;
+    if (std::strcmp(tv, "plain") == 0) h->trend_variant = 1;
+  }
   for (int q = 0; q < nlev && rc == WT_OK; ++q) {
     const wt_level_desc& ld = desc->levels[q];
     DevLevel& D = h->lev[q];
@@ -197,16 +271,7 @@ int wt_create(const wt_grid_desc* desc, wt_handle** out) {
     if ((e = cudaMalloc(&D.esrc, sizeof(int) * 3 * NN)) != cudaSuccess) { rc = wt_handle_fail("remap", e); break; }
     cudaMemcpy(D.nsrc, nsrc.data(), sizeof(int) * NN, cudaMemcpyHostToDevice);
     cudaMemcpy(D.esrc, esrc.data(), sizeof(int) * 3 * NN, cudaMemcpyHostToDevice);
-  }
-  if (rc == WT_OK) {
-    // Kernel pair: TMA-staged tiles from n = 64 up; below that the 32-wide tiles
-    // are mostly empty (n + 1 = 33 nodes per row at J5) and the L1 kernels are
-    // faster.  WAVETRISK_TREND_KERNEL=tma|plain forces either pair.
-    h->trend_variant = (h->top().n >= 64) ? 0 : 1;
-    if (const char* tv = std::getenv("WAVETRISK_TREND_KERNEL")) {
-      if (std::strcmp(tv, "tma") == 0) h->trend_variant = 0;
-      if (std::strcmp(tv, "plain") == 0) h->trend_variant = 1;
-    }
+    if (h->trend_variant == 0 && D.level == h->level_end && (rc = make_ghost_lists(h, D, hn, he, nsrc, esrc))) break;
   }
   if (rc == WT_OK) {
     // Prognostic state and RK/trend work arrays on level_end.
@@ -258,6 +323,8 @@ int wt_destroy(wt_handle* h) {
   for (float* p : arrays32)
     if (p) cudaFree(p);
   h->release_extra();
+  cudaFree(const_cast<int2*>(h->ghosts.nodes));
+  cudaFree(const_cast<int2*>(h->ghosts.edges));
   if (h->dflag) cudaFree(h->dflag);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -282,6 +349,7 @@ int wt_set_flux_precision(wt_handle* h, int bits) {
       if (e == cudaSuccess) e = cudaMemset(*arrays[q], 0, sizeof(float) * sizes[q]);
       if (e != cudaSuccess) return wt_handle_fail("flux fp32 arrays", e);
     }
+    if (int rc = make_f32_maps(h)) return rc;
   }
   if (h->graph_exec) {
     cudaGraphExecDestroy(h->graph_exec);
@@ -405,10 +473,64 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   (void)halo_first;
   // block b: layer b % nz of node chunk b / nz (layer_node in trisk_kernels.cuh)
   const unsigned chunks = blocks_for(D.NN, NODE_TILE);
+  const bool pipe = h->trend_variant == 0;  // pipelined tiles (trisk_pipe.cuh)
+  const unsigned cb = blocks_for(D.NN, COL_TILE);
+  const unsigned gb = pipe ? ghost_blocks(h->ghosts.n_nodes + h->ghosts.n_edges, nz, COL_TILE) : 0;
   TB(1);
-  k_column<<<chunks, NODE_TILE, 0, s>>>(L, h->ph, nz, m, t, h->mean_m, h->mean_t, h->phik, h->pterm, nullptr);
+  if (pipe)
+    k_column_halo<<<cb + gb, COL_TILE, 0, s>>>(L, h->ph, nz, gb, h->ghosts, m, t, v, h->mean_m, h->mean_t,
+                                                              h->phik, h->pterm);
+  else
+    k_column<<<cb, COL_TILE, 0, s>>>(L, h->ph, nz, m, t, h->mean_m, h->mean_t, h->phik, h->pterm, nullptr);
   TE(1);
-  if (h->flux_bits == 32) {  // FP32 flux stencils, FP64 trends and sub-step (trisk_mixed.cuh)
+  double* dm = mode == MODE_RK ? om : h->dm;
+  double* dt = mode == MODE_RK ? ot : h->dt;
+  double* dv = mode == MODE_RK ? ov : h->dv;
+  const bool f32 = h->flux_bits == 32;
+  if (pipe) {
+    const int sb = (m == h->m1) ? 1 : (m == h->m2) ? 2 : 0;  // which state buffer the stage reads
+    auto grid = [&](int nodes) {
+      PipeGrid G{(nodes + PX - 1) / PX, (nodes + PY - 1) / PY, 0, 0, 0};
+      const int tiles = G.nbx * G.nby * 10;
+      G.group = pipe_group(tiles, nz, h->pipe_slots);
+      G.ngroups = (nz + G.group - 1) / G.group;
+      G.items = tiles * G.ngroups;
+      return G;
+    };
+    const PipeGrid g1 = grid(D.n + 1), g2 = grid(D.P);
+    const unsigned b1 = std::min(g1.items, h->pipe_slots), b2 = std::min(g2.items, h->pipe_slots);
+    TB(2);
+    if (f32)
+      k_step1_pipe<float><<<b1, Step1Pipe<float>::BLOCK, Step1Pipe<float>::SMEM, s>>>(
+          L, nz, g1, Step1Res<float>{h->qe32, h->hfm32, h->hft32, h->ke32, h->theta32}, h->dflag, h->tma_inject, h->p1maps[sb]);
+    else
+      k_step1_pipe<double><<<b1, Step1Pipe<double>::BLOCK, Step1Pipe<double>::SMEM, s>>>(
+          L, nz, g1, Step1Res<double>{h->qe, h->hfm, h->hft, h->bern, h->theta}, h->dflag, h->tma_inject, h->p1maps[sb]);
+    const unsigned nc = corner_blocks(nz), nb = border_blocks(D.n, nz), ng = ghost_blocks(h->ghosts.n_f, nz, GHOST_TILE);
+    if (f32)
+      k_step1_border<float><<<nc + nb + ng, GHOST_TILE, 0, s>>>(L, nz, nc, nb, m, v, h->mean_m, h->qe32, h->ghosts,
+                                                                h->hfm32, h->hft32);
+    else
+      k_step1_border<double><<<nc + nb + ng, GHOST_TILE, 0, s>>>(L, nz, nc, nb, m, v, h->mean_m, h->qe, h->ghosts,
+                                                                 h->hfm, h->hft);
+    TE(2);
+    TB(5);
+    if (f32) {
+      const TrendPipeIO io{dm, dt, dv, hstep};
+      const auto k = mode == MODE_RK ? k_trend_pipe<float, MODE_RK> : k_trend_pipe<float, MODE_TREND>;
+      const int smem = mode == MODE_RK ? TrendPipe<float, MODE_RK>::SMEM : TrendPipe<float, MODE_TREND>::SMEM;
+      k<<<b2, TrendPipe<float, MODE_RK>::BLOCK, smem, s>>>(L, nz, g2, io, h->dflag, h->tma_inject, h->fmaps, h->p1maps[0]);
+    } else {
+      const TrendPipeIO io{dm, dt, dv, hstep};
+      const auto k = mode == MODE_RK ? k_trend_pipe<double, MODE_RK> : k_trend_pipe<double, MODE_TREND>;
+      const int smem = mode == MODE_RK ? TrendPipe<double, MODE_RK>::SMEM : TrendPipe<double, MODE_TREND>::SMEM;
+      k<<<b2, TrendPipe<double, MODE_RK>::BLOCK, smem, s>>>(L, nz, g2, io, h->dflag, h->tma_inject, h->pmaps, h->p1maps[0]);
+    }
+    TE(5);
+    CK(cudaGetLastError());
+    return WT_OK;
+  }
+  if (f32) {  // FP32 flux stencils, FP64 trends and sub-step (trisk_mixed.cuh)
     TB(2);
     k_step1_f32<<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, m, t, v, h->mean_m, h->mean_t,
                                                    Step1OutF{h->qe32, h->hfm32, h->hft32, h->ke32, h->theta32});
@@ -429,49 +551,30 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   }
   Step1Out so{h->qe, h->hfm, h->hft, h->bern, h->theta};
   TB(2);
-  if (h->trend_variant == 0) {
-    const int sb = (m == h->m1) ? 1 : (m == h->m2) ? 2 : 0;  // which state buffer the stage reads
-    const int nbx = (D.n + 1 + TT_X - 1) / TT_X, nby = (D.n + 1 + TT_Y - 1) / TT_Y;
-    const unsigned nblk = (unsigned)(nz * nbx * nby * 10);
-    k_step1_tma<<<nblk, TT_X * TT_Y, STEP1_TMA_SMEM, s>>>(L, nz, nbx, nby, m, t, v, h->mean_m, h->phik, h->pterm, so,
-                                                           h->dflag, h->tma_inject, h->s1maps[sb], nullptr);
-  } else {
-    k_step1<<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, m, t, v, h->mean_m, h->mean_t, h->phik, h->pterm, so, nullptr);
-  }
+  k_step1<<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, m, t, v, h->mean_m, h->mean_t, h->phik, h->pterm, so, nullptr);
   TE(2);
   TrendIO io{};
   io.theta = h->theta; io.qe = h->qe; io.hfm = h->hfm; io.hft = h->hft; io.bern = h->bern; io.phik = h->phik;
   io.base_m = bm; io.base_t = bt; io.base_v = bv; io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
   io.dm = h->dm; io.dtt = h->dt; io.dv = h->dv;
   TB(5);
-  if (h->trend_variant == 0) {
-    const int nbx = (D.P + TT_X - 1) / TT_X, nby = (D.P + TT_Y - 1) / TT_Y;
-    const unsigned nblk = (unsigned)(nz * nbx * nby * 10);
-    if (mode == MODE_RK)
-      k_trend_tma<MODE_RK><<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, s>>>(L, nz, nbx, nby, io, h->dflag, h->tma_inject,
-                                                                     h->maps);
-    else
-      k_trend_tma<MODE_TREND><<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, s>>>(L, nz, nbx, nby, io, h->dflag, h->tma_inject,
-                                                                        h->maps);
-  } else {
-    if (mode == MODE_RK)
-      k_trend<MODE_RK><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
-    else
-      k_trend<MODE_TREND><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
-  }
+  if (mode == MODE_RK)
+    k_trend<MODE_RK><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
+  else
+    k_trend<MODE_TREND><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
   TE(5);
   CK(cudaGetLastError());
   return WT_OK;
 }
 
-// k_trend_tma<MODE_ML> on the top level: the multi-level trend of the finest
+// k_trend_tma on the top level: the multi-level trend of the finest
 // level with the RK sub-step, its inputs read through the maps M.
 int wt_level_trend_ml_tma(wt_handle* h, const wtk::TrendIO& io, const wtk::TrendMaps& M, cudaStream_t stream) {
   const DevLevel& D = h->top();
   const int nz = h->nz;
   const int nbx = (D.P + TT_X - 1) / TT_X, nby = (D.P + TT_Y - 1) / TT_Y;
   const unsigned nblk = (unsigned)(nz * nbx * nby * 10);
-  k_trend_tma<MODE_ML><<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, stream ? stream : h->stream>>>(D.view(), nz, nbx, nby, io,
+  k_trend_tma<<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, stream ? stream : h->stream>>>(D.view(), nz, nbx, nby, io,
                                                                                            h->dflag, h->tma_inject, M);
   CK(cudaGetLastError());
   return WT_OK;
@@ -485,17 +588,17 @@ int wt_level_step1(wt_handle* h, int level, const double* m, const double* t, co
   const LevelDev L = D.view();
   const int nz = h->nz;
   cudaStream_t s = stream ? stream : h->stream;
-  const unsigned chunks = blocks_for(D.NN, NODE_TILE);
   Step1Out so{qe, hfm, hft, bern, theta};
+  const unsigned chunks = blocks_for(D.NN, NODE_TILE);
   if (list && list->ids) {  // the needed slots only, persistent blocks over the level's work list
-    k_column_list<<<persistent_grid(k_column_list, chunks), NODE_TILE, 0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t,
-                                                                               phik, pterm, *list);
+    k_column_list<<<persistent_grid(k_column_list, blocks_for(D.NN, COL_TILE), COL_TILE), COL_TILE, 0, s>>>(
+        L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, *list);
     k_step1_list<<<persistent_grid(k_step1_list, chunks * nz), NODE_TILE, 0, s>>>(L, nz, m, t, v, mean_m, mean_t,
                                                                                   phik, pterm, so, *list);
     CK(cudaGetLastError());
     return WT_OK;
   }
-  k_column<<<chunks, NODE_TILE, 0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, need);
+  k_column<<<blocks_for(D.NN, COL_TILE), COL_TILE, 0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, need);
   if (maps && level == h->level_end && h->trend_variant == 0) {
     const int nbx = (D.n + 1 + TT_X - 1) / TT_X, nby = (D.n + 1 + TT_Y - 1) / TT_Y;
     const unsigned nblk = (unsigned)(nz * nbx * nby * 10);

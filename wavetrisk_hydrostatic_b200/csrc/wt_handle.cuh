@@ -51,11 +51,17 @@ struct wt_handle {
   double *dm = nullptr, *dt = nullptr, *dv = nullptr;
   double *qe = nullptr, *hfm = nullptr, *hft = nullptr, *bern = nullptr, *phik = nullptr, *pterm = nullptr;
   double* theta = nullptr;  // Theta/rho of the stage state, written by k_step1
-  wtk::TrendMaps maps{};    // tensor maps of the trend inputs (TMA-staged trend kernel)
-  wtk::Step1Maps s1maps[3]{};  // step1 input maps for the state buffers (mass,temp,velo), (m1,t1,v1), (m2,t2,v2)
+  wtk::Step1Maps s1maps{};  // k_step1_tma's input maps of the state (mass, temp, velo) (hierarchy)
+  // the single-level stepper's pipelined kernels (trisk_pipe.cuh): step1 inputs of the state buffers (mass, temp,
+  // velo), (m1, t1, v1), (m2, t2, v2), trend inputs, geometry, and the blocks the device keeps resident
+  wtk::GhostLists ghosts{};
+  wtk::PipeStateMaps p1maps[3]{};
+  wtk::TrendMapsD pmaps{};
+  wtk::TrendMapsF fmaps{};
+  int pipe_slots = 0;
   int* dflag = nullptr;     // device error flag: 1 = a kernel's staged copies did not complete
   int tma_inject = 0;       // test only: the TMA kernels take their wait-timeout path
-  int trend_variant = 0;    // 0: TMA-staged k_step1_tma/k_trend_tma, 1: k_step1/k_trend (loads through L1)
+  int trend_variant = 0;    // 0: TMA-staged kernels, 1: k_step1/k_trend (loads through L1)
   // WT_TUNE_FLUX_PRECISION: 64 (default) or 32, the FP32 step1 of the
   // single-level stepper (trisk_mixed.cuh) with its FP32 results below
   int flux_bits = 64;
@@ -96,7 +102,7 @@ void wt_trend_ml_release(wt_handle* h);
 // level's geometry), for k_trend_tma; WT_ERR_STATE unless the TMA variant is on.
 int wt_make_trend_maps(wt_handle* h, const double* hfm, const double* hft, const double* qe, const double* theta,
                        const double* bern, const double* phik, wtk::TrendMaps* M);
-// k_trend_tma<MODE_ML> on the top level (stream: the handle's when null).
+// k_trend_tma on the top level (stream: the handle's when null).
 int wt_level_trend_ml_tma(wt_handle* h, const wtk::TrendIO& io, const wtk::TrendMaps& M, cudaStream_t stream);
 int wt_level_step1(wt_handle* h, int level, const double* m, const double* t, const double* v, const double* mean_m,
                    const double* mean_t, double* phik, double* pterm, double* qe, double* hfm, double* hft,

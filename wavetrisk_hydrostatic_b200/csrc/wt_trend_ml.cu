@@ -196,23 +196,43 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
   // side streams (parallel branches of a captured graph).  The phase timer
   // keeps them on the handle's stream so that its events bracket them.
   const bool concurrent = tm == nullptr && h->level_end > h->level_start;
+  // column + step1 of level l on the handle's stream (s null) or a side stream
+  auto step1 = [&](int l, cudaStream_t s) -> int {
+    const int q = l - h->level_start;
+    MLLevel& V = M->L[q];
+    double *mm, *mt;
+    if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_MASS, &mm)) return rc;
+    if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_TEMP, &mt)) return rc;
+    const wtk::Step1Maps* maps = nullptr;
+    if (l == h->level_end && h->trend_variant == 0) {
+      if (S.m[q] == h->mass && S.t[q] == h->temp && S.v[q] == h->velo) {
+        maps = &h->s1maps;
+      } else if (S.m[q] == V.m1 && S.t[q] == V.t1 && S.v[q] == V.v1) {
+        if (!M->q1maps_ok) {
+          if (int rc = wt_make_step1_maps(h, V.m1, V.t1, V.v1, &M->q1maps)) return rc;
+          M->q1maps_ok = true;
+        }
+        maps = &M->q1maps;
+      }
+    }
+    const wtk::NodeList wl = list(l);
+    return wt_level_step1(h, l, S.m[q], S.t[q], S.v[q], mm, mt, V.phik, V.pterm, V.qe, V.hfm, V.hft, V.bern, V.theta,
+                          maps, s, need(l), &wl);
+  };
   if (concurrent) {
+    // The finest level first: a graph's launch hands its branches to the device in
+    // the order of their capture, and this one heads the critical chain.
     CKM(cudaEventRecord(M->fork, h->stream));
-    for (int l = h->level_start; l < h->level_end; ++l) {
+    if (int rc = step1(h->level_end, nullptr)) return rc;
+    CKM(cudaEventRecord(M->s1top, h->stream));
+    for (int l = h->level_end - 1; l >= h->level_start; --l) {
       const int q = l - h->level_start;
-      MLLevel& V = M->L[q];
-      double *mm, *mt;
-      if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_MASS, &mm)) return rc;
-      if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_TEMP, &mt)) return rc;
       if (after_inverse) {
         if (int rc = wt_level_ready_wait(h, l, M->side[q])) return rc;
       } else {
         CKM(cudaStreamWaitEvent(M->side[q], M->fork, 0));
       }
-      const wtk::NodeList wl = list(l);
-      if (int rc = wt_level_step1(h, l, S.m[q], S.t[q], S.v[q], mm, mt, V.phik, V.pterm, V.qe, V.hfm, V.hft, V.bern,
-                                  V.theta, nullptr, M->side[q], need(l), &wl))
-        return rc;
+      if (int rc = step1(l, M->side[q])) return rc;
       CKM(cudaEventRecord(M->done[q], M->side[q]));
     }
   }
@@ -220,31 +240,12 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
     const int q = l - h->level_start;
     MLLevel& V = M->L[q];
     const DevLevel& D = h->at(l);
-    if (concurrent && l < h->level_end) {
-      CKM(cudaStreamWaitEvent(h->stream, M->done[q], 0));
+    if (concurrent) {
+      if (l < h->level_end) CKM(cudaStreamWaitEvent(h->stream, M->done[q], 0));
     } else {
-      double *mm, *mt;
-      if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_MASS, &mm)) return rc;
-      if (int rc = wt_level_mean(h, l, WT_FIELD_MEAN_TEMP, &mt)) return rc;
       PB(tm);
-      const wtk::Step1Maps* maps = nullptr;
-      if (l == h->level_end && h->trend_variant == 0) {
-        if (S.m[q] == h->mass && S.t[q] == h->temp && S.v[q] == h->velo) {
-          maps = &h->s1maps[0];
-        } else if (S.m[q] == V.m1 && S.t[q] == V.t1 && S.v[q] == V.v1) {
-          if (!M->q1maps_ok) {
-            if (int rc = wt_make_step1_maps(h, V.m1, V.t1, V.v1, &M->q1maps)) return rc;
-            M->q1maps_ok = true;
-          }
-          maps = &M->q1maps;
-        }
-      }
-      const wtk::NodeList wl = list(l);
-      if (int rc = wt_level_step1(h, l, S.m[q], S.t[q], S.v[q], mm, mt, V.phik, V.pterm, V.qe, V.hfm, V.hft,
-                                  V.bern, V.theta, maps, nullptr, need(l), &wl))
-        return rc;
+      if (int rc = step1(l, nullptr)) return rc;
       PE(tm, l == h->level_end ? PH_STEP1_TOP : PH_STEP1_COARSE);
-      if (concurrent) CKM(cudaEventRecord(M->s1top, h->stream));
     }
     wtk::TrendML io{};
     const int *mask_n, *mask_e;
