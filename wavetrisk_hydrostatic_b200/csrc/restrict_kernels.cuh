@@ -338,8 +338,8 @@ __device__ __forceinline__ double sm_eval_s(const int (*si)[32], const double (*
 
 // flux_cpt_restr of up to two fluxes (mass, Theta: fp0/fp1 from the child's
 // fc0/fc1 and dscalar dc0/dc1) on the restricted parent edges (mask_e >=
-// RESTRCT).  Block (32, ny): 32 consecutive parent edges of the plan, ny
-// threads per edge taking layers y, y + ny, ...; blocks without a restricted
+// RESTRCT).  Block (32, 2 ny): 32 consecutive parent edges of the plan, ny
+// threads per edge and flux taking layers y, y + ny, ...; blocks without a restricted
 // edge return before staging.  With a work list (PL), persistent blocks take
 // 32 of the listed parents' edges at a time.  Same expression trees and operand order as
 // part_coarse_flux + coarse_flux + interp_flux of the reference.
@@ -348,38 +348,35 @@ __device__ __forceinline__ void restr_flux_one(const WLev& P, int nz, const int 
                                                double* __restrict__ fp1, const double* __restrict__ fc0,
                                                const double* __restrict__ fc1, const double* __restrict__ dc0,
                                                const double* __restrict__ dc1, int NNc) {
-  const int y = threadIdx.y, ny = blockDim.y;
+  const int y = threadIdx.y / 2, ny = blockDim.y / 2, f = threadIdx.y % 2;
   const bool pa = (e & 1) != 0, pb = ((e + 1) & 1) != 0;
   const int64_t so = (int64_t)e * P.NN + nid(P, d, ip, jp);
   const double ar0 = sd[12][x], ar1 = sd[13][x], o0 = sd[14][x], o1 = sd[15][x], o2 = sd[16][x], o3 = sd[17][x];
+  double* __restrict__ fp = f == 0 ? fp0 : fp1;
+  if (!fp) return;
   for (int k = y; k < nz; k += ny) {
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      double* __restrict__ fp = f == 0 ? fp0 : fp1;
-      if (!fp) continue;
-      const double* __restrict__ h = (f == 0 ? fc0 : fc1) + (int64_t)3 * k * NNc;
-      const double* __restrict__ ds = (f == 0 ? dc0 : dc1) + (int64_t)k * NNc;
-      const double sma = sm_eval_s(si, sd, 0, 0, x, pa, h), smb = sm_eval_s(si, sd, 9, 6, x, pb, h);
-      double tp = fe(h, si[18][x]) * ar0;
-      tp = tp + fe(h, si[19][x]) * ar1;
-      tp = tp - (fe(h, si[20][x]) + fe(h, si[21][x])) * ar1;
-      tp = tp - (fe(h, si[22][x]) + fe(h, si[23][x])) * ar0;
-      tp = tp + o2 * fn(ds, si[24][x]);
-      tp = tp - o3 * fn(ds, si[26][x]);
-      tp = tp - o0 * fn(ds, si[25][x]);
-      tp = tp + o1 * fn(ds, si[27][x]);
-      const double dmz = fn(ds, si[28][x]), dpz = fn(ds, si[29][x]);
-      double tc = sd[18][x] * (dpz - dmz);
-      tc = tc + sd[19][x] * (fn(ds, si[32][x]) - dmz);
-      tc = tc + sd[20][x] * (fn(ds, si[31][x]) - dmz);
-      tc = tc + sd[21][x] * (dpz - fn(ds, si[33][x]));
-      tc = tc + sd[22][x] * (dpz - fn(ds, si[30][x]));
-      fp[(int64_t)3 * k * P.NN + so] = tp + tc + sma + smb;
-    }
+    const double* __restrict__ h = (f == 0 ? fc0 : fc1) + (int64_t)3 * k * NNc;
+    const double* __restrict__ ds = (f == 0 ? dc0 : dc1) + (int64_t)k * NNc;
+    const double sma = sm_eval_s(si, sd, 0, 0, x, pa, h), smb = sm_eval_s(si, sd, 9, 6, x, pb, h);
+    double tp = fe(h, si[18][x]) * ar0;
+    tp = tp + fe(h, si[19][x]) * ar1;
+    tp = tp - (fe(h, si[20][x]) + fe(h, si[21][x])) * ar1;
+    tp = tp - (fe(h, si[22][x]) + fe(h, si[23][x])) * ar0;
+    tp = tp + o2 * fn(ds, si[24][x]);
+    tp = tp - o3 * fn(ds, si[26][x]);
+    tp = tp - o0 * fn(ds, si[25][x]);
+    tp = tp + o1 * fn(ds, si[27][x]);
+    const double dmz = fn(ds, si[28][x]), dpz = fn(ds, si[29][x]);
+    double tc = sd[18][x] * (dpz - dmz);
+    tc = tc + sd[19][x] * (fn(ds, si[32][x]) - dmz);
+    tc = tc + sd[20][x] * (fn(ds, si[31][x]) - dmz);
+    tc = tc + sd[21][x] * (dpz - fn(ds, si[33][x]));
+    tc = tc + sd[22][x] * (dpz - fn(ds, si[30][x]));
+    fp[(int64_t)3 * k * P.NN + so] = tp + tc + sma + smb;
   }
 }
 
-__global__ void __launch_bounds__(256) k_restr_flux3(WLev P, int m, int nz, const int* __restrict__ pi,
+__global__ void __launch_bounds__(512, 2) k_restr_flux3(WLev P, int m, int nz, const int* __restrict__ pi,
                                                      const double* __restrict__ pd, double* __restrict__ fp0,
                                                      double* __restrict__ fp1, const double* __restrict__ fc0,
                                                      const double* __restrict__ fc1, const double* __restrict__ dc0,

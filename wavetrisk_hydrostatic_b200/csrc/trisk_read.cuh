@@ -105,6 +105,14 @@ struct Rd {
     const double v = f[c >> 1];
     return (c & 1) ? -v : v;
   }
+  // The slot e() reads, for use over several layers; its sign goes into the factor a
+  // that the value is multiplied by (exact).
+  __device__ __forceinline__ int ex(int slot, double& a) const {
+    if (direct) return slot;
+    const int c = __ldg(esrc + slot);
+    if (c & 1) a = -a;
+    return c >> 1;
+  }
 };
 
 __device__ __forceinline__ void weights5(const LevelDev& L, int id, int offs, double w[5]) {  // get_weights

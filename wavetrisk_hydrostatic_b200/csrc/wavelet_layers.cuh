@@ -564,24 +564,23 @@ __device__ __forceinline__ void stage_plan(int (*si)[32], double (*sd)[32], cons
     }
 }
 
-// Interp_outer_velo of edge e of staged parent x (outer_eval's expression).
-__device__ __forceinline__ double outer_eval_s(const int (*si)[32], const double (*sd)[32], int e, int x,
+// Interp_outer_velo of the staged edge of parent x (outer_eval's expression).
+__device__ __forceinline__ double outer_eval_s(const int (*si)[32], const double (*sd)[32], int x,
                                                const double* __restrict__ vp, double& t0) {
-  const int b = e * 14, w = e * 9;
   double t[9];
-  t[0] = we(vp, si[b + 0][x]);
-  t[1] = we(vp, si[b + 1][x]);
-  t[2] = we(vp, si[b + 2][x]);
-  t[3] = we(vp, si[b + 3][x]);
-  t[4] = we(vp, si[b + 4][x]);
-  t[5] = we(vp, si[b + 5][x]) - we(vp, si[b + 6][x]);
-  t[6] = we(vp, si[b + 7][x]) - we(vp, si[b + 8][x]);
-  t[7] = we(vp, si[b + 9][x]) - we(vp, si[b + 10][x]);
-  t[8] = we(vp, si[b + 11][x]) - we(vp, si[b + 12][x]);
+  t[0] = we(vp, si[0][x]);
+  t[1] = we(vp, si[1][x]);
+  t[2] = we(vp, si[2][x]);
+  t[3] = we(vp, si[3][x]);
+  t[4] = we(vp, si[4][x]);
+  t[5] = we(vp, si[5][x]) - we(vp, si[6][x]);
+  t[6] = we(vp, si[7][x]) - we(vp, si[8][x]);
+  t[7] = we(vp, si[9][x]) - we(vp, si[10][x]);
+  t[8] = we(vp, si[11][x]) - we(vp, si[12][x]);
   t0 = t[0];
   double sum = 0.0;
 #pragma unroll
-  for (int q = 0; q < 9; ++q) sum = sum + sd[w + q][x] * t[q];
+  for (int q = 0; q < 9; ++q) sum = sum + sd[q][x] * t[q];
   return sum;
 }
 
@@ -626,59 +625,89 @@ __device__ __forceinline__ void gather_plan(int (*si)[32], double (*sd)[32], con
     }
 }
 
-// Reconstruct_outer_velo of the staged parent x of the block (d, ip, jp).
+// Reconstruct_outer_velo of edge e of the block's parent x (d, ip, jp), its plan row
+// staged.  The pentagon correction needs a corner parent's three edges: the thread of
+// its first edge does them all, the other two from the plan itself (u).
 __device__ __forceinline__ void recon_outer_one(const WLev& Pa, const WLev& C, int nz, const int (*si)[32],
-                                                const double (*sd)[32], int x, int d, int ip, int jp) {
+                                                const double (*sd)[32], const int* __restrict__ pi,
+                                                const double* __restrict__ pd, int64_t ne, int64_t u, int x, int d,
+                                                int ip, int jp, int e) {
   const int np = Pa.n, y = threadIdx.y, ny = blockDim.y;
   const int i = 2 * ip, j = 2 * jp;
-  for (int e = 0; e < 3; ++e) {
-    const int a1 = i + c_end_pt[e][0][0], b1 = j + c_end_pt[e][0][1];
-    const int a2 = i + c_end_pt[e][1][0], b2 = j + c_end_pt[e][1][1];
-    const int x2 = e * C.NN + nid(C, d, a2, b2), x1 = e * C.NN + nid(C, d, a1, b1);
-    const int cw = si[e * 14 + 13][x];
+  const bool corner = (ip == 0 || ip == np - 1) && (jp == 0 || jp == np - 1);
+  if (corner && e) return;
+  const auto slots = [&](int q, int& x1, int& x2) {
+    x1 = q * C.NN + nid(C, d, i + c_end_pt[q][0][0], j + c_end_pt[q][0][1]);
+    x2 = q * C.NN + nid(C, d, i + c_end_pt[q][1][0], j + c_end_pt[q][1][1]);
+  };
+  int x1, x2;
+  slots(e, x1, x2);
+  const int cw = si[13][x];
+#pragma unroll 2
+  for (int k = y; k < nz; k += ny) {
+    const double* vp = Pa.sv + (int64_t)k * 3 * Pa.NN;
+    const double* wc = C.wv + (int64_t)k * 3 * C.NN;
+    double* v = C.sv + (int64_t)k * 3 * C.NN;
+    double t0;
+    const double uu = outer_eval_s(si, sd, x, vp, t0);
+    const double v2 = uu + we(wc, cw);
+    v[x2] = v2;
+    v[x1] = 2.0 * t0 - v2;
+  }
+  if (!corner) return;
+  for (int q = 1; q < 3; ++q) {
+    OuterInterp O;
+#pragma unroll
+    for (int c = 0; c < 13; ++c) O.c[c] = __ldg(pi + (q * 14 + c) * ne + u);
+#pragma unroll
+    for (int c = 0; c < 9; ++c) O.w[c] = __ldg(pd + (q * 9 + c) * ne + u);
+    const int cq = __ldg(pi + (q * 14 + 13) * ne + u);
+    slots(q, x1, x2);
     for (int k = y; k < nz; k += ny) {
-      const double* vp = Pa.sv + (int64_t)k * 3 * Pa.NN;
-      const double* wc = C.wv + (int64_t)k * 3 * C.NN;
       double* v = C.sv + (int64_t)k * 3 * C.NN;
       double t0;
-      const double uu = outer_eval_s(si, sd, e, x, vp, t0);
-      const double v2 = uu + we(wc, cw);
+      const double uu = outer_eval(O, Pa.sv + (int64_t)k * 3 * Pa.NN, t0);
+      const double v2 = uu + we(C.wv + (int64_t)k * 3 * C.NN, cq);
       v[x2] = v2;
       v[x1] = 2.0 * t0 - v2;
     }
   }
-  if ((ip == 0 || ip == np - 1) && (jp == 0 || jp == np - 1))
-    for (int k = y; k < nz; k += ny)
-      penta_reconstruct(Pa, C, Pa.sv + (int64_t)k * 3 * Pa.NN, C.sv + (int64_t)k * 3 * C.NN, d, ip, jp);
+  for (int k = y; k < nz; k += ny)
+    penta_reconstruct(Pa, C, Pa.sv + (int64_t)k * 3 * Pa.NN, C.sv + (int64_t)k * 3 * C.NN, d, ip, jp);
 }
 
 // Reconstruct_outer_velo (src/wavelet.f90:954-976) from the outer plan,
-// parents [0, np]^2, then Reconstruct_velo_penta by the corner parents.  With
-// a work list (PL), persistent blocks take 32 listed parents at a time.
-__global__ void __launch_bounds__(256) k_recon_outer_p(WLev Pa, WLev C, int nz, const int* __restrict__ pi,
+// parents [0, np]^2, then Reconstruct_velo_penta by the corner parents.  A block
+// takes 32 parents' edges e (the three edges of 32 parents are consecutive blocks);
+// with a work list (PL), persistent blocks take such items of the listed parents.
+// An edge a thread instead of three: at the coarse levels of a hierarchy, fewer
+// blocks than SMs, the launch is one thread's chain of dependent reads.
+__global__ void __launch_bounds__(256, 3) k_recon_outer_p(WLev Pa, WLev C, int nz, const int* __restrict__ pi,
                                                        const double* __restrict__ pd,
                                                        const unsigned char* __restrict__ rec, ParentList PL) {
-  __shared__ int si[OP_NI][32];
-  __shared__ double sd[OP_ND][32];
+  __shared__ int si[14][32];
+  __shared__ double sd[9][32];
   const int np = Pa.n, m = np + 1;
   const int64_t ne = (int64_t)10 * m * m;
   const int x = threadIdx.x;
   if (PL.ids) {
     const int cnt = __ldg(PL.count);
-    for (int c = blockIdx.x; c < (cnt + 31) / 32; c += gridDim.x) {
-      const int e = c * 32 + x;
+    for (int c = blockIdx.x; c < 3 * ((cnt + 31) / 32); c += gridDim.x) {
+      const int e = c % 3, r = c / 3 * 32 + x;
       int d = 0, ip = 0, jp = 0;
-      bool live = e < cnt && list_parent(Pa.n, __ldg(PL.ids + e), m, d, ip, jp) && rebuilt(rec, Pa, d, ip, jp);
+      bool live = r < cnt && list_parent(Pa.n, __ldg(PL.ids + r), m, d, ip, jp) && rebuilt(rec, Pa, d, ip, jp);
       if (__syncthreads_or(live)) {
-        gather_plan<OP_NI, OP_ND>(si, sd, pi, pd, ne, ((int64_t)d * m + jp) * m + ip, live);
+        const int64_t u = ((int64_t)d * m + jp) * m + ip;
+        gather_plan<14, 9>(si, sd, pi + e * 14 * ne, pd + e * 9 * ne, ne, u, live);
         __syncthreads();
-        if (live) recon_outer_one(Pa, C, nz, si, sd, x, d, ip, jp);
+        if (live) recon_outer_one(Pa, C, nz, si, sd, pi, pd, ne, u, x, d, ip, jp, e);
       }
       __syncthreads();
     }
     return;
   }
-  const int64_t u0 = (int64_t)blockIdx.x * 32;
+  const int e = blockIdx.x % 3;
+  const int64_t u0 = (int64_t)(blockIdx.x / 3) * 32;
   int d = 0, ip = 0, jp = 0;
   bool live = u0 + x < ne;
   if (live) {
@@ -686,10 +715,10 @@ __global__ void __launch_bounds__(256) k_recon_outer_p(WLev Pa, WLev C, int nz, 
     live = rebuilt(rec, Pa, d, ip, jp);
   }
   if (!__syncthreads_or(live)) return;
-  stage_plan<OP_NI, OP_ND>(si, sd, pi, pd, ne, u0, (int)min((int64_t)32, ne - u0));
+  stage_plan<14, 9>(si, sd, pi + e * 14 * ne, pd + e * 9 * ne, ne, u0, (int)min((int64_t)32, ne - u0));
   __syncthreads();
   if (!live) return;
-  recon_outer_one(Pa, C, nz, si, sd, x, d, ip, jp);
+  recon_outer_one(Pa, C, nz, si, sd, pi, pd, ne, u0 + x, x, d, ip, jp, e);
 }
 
 // target edges of the inner plan: UP(i+1,j) DG(i+1,j) RT(i+1,j+1) RT(i,j+1) DG(i,j+1) UP(i+1,j+1)

@@ -132,7 +132,7 @@ int wt_level_after_step(wt_handle* h, double* const* m, double* const* t, double
 // [level_start, level_end), wt_level_wav_finish, unbind.
 void wt_level_wav_bind(wt_handle* h, double* const* m, double* const* t, double* const* v);
 void wt_level_wav_unbind(wt_handle* h);
-int wt_level_wav_forward_pair(wt_handle* h, int level);
+int wt_level_wav_forward_pair(wt_handle* h, int level, cudaStream_t velo = nullptr);
 // mode 0: the inverse rebuilds every parent; 1: only the parents of
 // wt_level_rec (an intermediate RK stage, whose state the next stage reads only
 // where needed); 2: those of wt_level_rec_final (the step's last inverse).

@@ -43,6 +43,11 @@ struct MLCtx {
   // (they need both levels' step1 and the finer restriction, not the trends)
   cudaStream_t rs = nullptr;
   std::vector<cudaEvent_t> rsd;
+  // the velocity trends, level by level on their own stream, each after its level's
+  // fluxes (flx)
+  cudaStream_t vs = nullptr;
+  std::vector<cudaEvent_t> flx;
+  int edge_slots = 1;  // resident blocks of k_trend_ml_velo
   cudaEvent_t s1top = nullptr;
 };
 
@@ -86,6 +91,10 @@ int ensure(wt_handle* h) {
   CKM(cudaDeviceGetStreamPriorityRange(&least, &greatest));
   const int medium = greatest < least ? greatest + 1 : greatest;
   CKM(cudaStreamCreateWithPriority(&M->rs, cudaStreamNonBlocking, greatest));
+  CKM(cudaStreamCreateWithPriority(&M->vs, cudaStreamNonBlocking, medium));
+  M->flx.resize(M->L.size());
+  for (cudaEvent_t& e : M->flx) CKM(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  M->edge_slots = (int)wtk::persistent_grid(wtk::k_trend_ml_velo, ~0u, wtk::EDGE_BLOCK);
   for (int l = h->level_start; l < h->level_end; ++l) {
     cudaStream_t s;
     cudaEvent_t e, r;
@@ -108,7 +117,9 @@ void wt_trend_ml_release(wt_handle* h) {
   for (cudaEvent_t e : M->done) cudaEventDestroy(e);
   for (cudaEvent_t e : M->rsd) cudaEventDestroy(e);
   for (cudaStream_t s : M->side) cudaStreamDestroy(s);
+  for (cudaEvent_t e : M->flx) cudaEventDestroy(e);
   if (M->rs) cudaStreamDestroy(M->rs);
+  if (M->vs) cudaStreamDestroy(M->vs);
   if (M->fork) cudaEventDestroy(M->fork);
   if (M->s1top) cudaEventDestroy(M->s1top);
   for (void* p : M->allocs) cudaFree(p);
@@ -265,7 +276,6 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
       if (int rc = wt_level_restrict_flux(h, l, V.hfm, V.hft, C.hfm, C.hft, C.dm, C.dt, nz)) return rc;
       if (concurrent) {
         CKM(cudaEventRecord(M->rsd[q], rs));
-        CKM(cudaStreamWaitEvent(h->stream, M->rsd[q], 0));
       }
       PE(tm, PH_RESTRICT);
       const int *mask_n_c, *mask_e_c;
@@ -286,12 +296,28 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
       io.th1 = th1;
     }
     io.need = need(l);
+    // The scalars follow on the handle's stream, towards the next restriction; the
+    // velocity on its own, after this level's fluxes and restricted Bernoulli and Exner.
+    cudaStream_t vs = concurrent ? M->vs : h->stream;
+    // It is released with the next restriction, whose stream has the higher priority:
+    // released earlier, its blocks held the SMs while the restriction waited.
+    const auto velo_after = [&]() -> int {
+      if (!concurrent) return WT_OK;
+      CKM(cudaEventRecord(M->flx[q], h->stream));
+      CKM(cudaStreamWaitEvent(vs, M->flx[q], 0));
+      if (l < h->level_end) CKM(cudaStreamWaitEvent(vs, M->rsd[q], 0));
+      return WT_OK;
+    };
     const unsigned chunks = (unsigned)((D.NN + wtk::NODE_TILE - 1) / wtk::NODE_TILE);
+    const unsigned echunks = (unsigned)((D.NN + wtk::EDGE_TILE - 1) / wtk::EDGE_TILE);
     PB(tm);
     const wtk::NodeList wl = list(l);
     if (wl.ids) {  // the needed slots only, persistent blocks over the level's work list
-      wtk::k_trend_ml_list<<<wtk::persistent_grid(wtk::k_trend_ml_list, chunks * nz), wtk::NODE_TILE, 0,
-                             h->stream>>>(D.view(), nz, io, wl);
+      wtk::k_trend_ml_scal_list<<<wtk::persistent_grid(wtk::k_trend_ml_scal_list, chunks * nz), wtk::NODE_TILE, 0,
+                                  h->stream>>>(D.view(), nz, io, wl);
+      if (int rc = velo_after()) return rc;
+      wtk::k_trend_ml_velo_list<<<wtk::persistent_grid(wtk::k_trend_ml_velo_list, echunks * nz, wtk::EDGE_BLOCK),
+                                  wtk::EDGE_BLOCK, 0, vs>>>(D.view(), nz, io, wl);
     } else if (l == h->level_end && M->tmaps_ok && base && dest) {  // TMA-staged, the same arithmetic
       wtk::TrendIO t{};
       t.theta = V.theta; t.qe = V.qe; t.hfm = V.hfm; t.hft = V.hft; t.bern = V.bern; t.phik = V.phik;
@@ -300,13 +326,21 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
       t.dm = V.dm; t.dtt = V.dt; t.mask_n = mask_n; t.src = V.src; t.need = io.need;
       t.grad = io.grad; t.th1 = io.th1;
       if (int rc = wt_level_trend_ml_tma(h, t, M->tmaps, nullptr)) return rc;
+      if (int rc = velo_after()) return rc;
     } else {
-      wtk::k_trend_ml<<<chunks * nz, wtk::NODE_TILE, 0, h->stream>>>(D.view(), nz, io);
+      wtk::k_trend_ml_scal<<<chunks * nz, wtk::NODE_TILE, 0, h->stream>>>(D.view(), nz, io);
+      if (int rc = velo_after()) return rc;
+      const int lpt = wtk::layer_group(echunks, nz, M->edge_slots);
+      wtk::k_trend_ml_velo<<<echunks * ((nz + lpt - 1) / lpt), wtk::EDGE_BLOCK, 0, vs>>>(D.view(), nz, lpt, io);
     }
     PE(tm, l == h->level_end ? PH_TREND_TOP : PH_TREND_COARSE);
     CKM(cudaGetLastError());
     if (wav && dest && l < h->level_end)
-      if (int rc = wt_level_wav_forward_pair(h, l)) return rc;
+      if (int rc = wt_level_wav_forward_pair(h, l, vs)) return rc;
+  }
+  if (concurrent) {
+    CKM(cudaEventRecord(M->fork, M->vs));
+    CKM(cudaStreamWaitEvent(h->stream, M->fork, 0));
   }
   return WT_OK;
 }

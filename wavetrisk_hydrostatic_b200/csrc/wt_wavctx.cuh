@@ -47,7 +47,7 @@ struct WavCtx {
   // beside the coarser levels' trend)
   cudaStream_t side[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  std::vector<cudaEvent_t> fork;  // per level pair: its forward wavelets may start
+  std::vector<cudaEvent_t> fork, fork_v;  // per level pair: its forward wavelets may start
   // per level: its state is complete in the last inverse transform (velocity
   // chain on the handle's stream, scalar chain on side[0])
   std::vector<cudaEvent_t> ready_v, ready_s;

@@ -218,7 +218,7 @@ void inverse(wt_handle* h, int partial = 0) {
         P, C, np, nz, lpt_for(nz), rec, PL);
     cudaEventRecord(W->ready_s[q], sa);
     const WavLevel& V = W->L[l - h->level_start];
-    k_recon_outer_p<<<PL.ids ? pgrid(k_recon_outer_p, pt, plan_grid(par1)) : plan_grid(par1), pb, 0, s>>>(
+    k_recon_outer_p<<<PL.ids ? pgrid(k_recon_outer_p, pt, 3 * plan_grid(par1)) : 3 * plan_grid(par1), pb, 0, s>>>(
         P, C, nz, V.op_i, V.op_d, rec, PL);
     k_recon_inner_p<<<PL.ids ? pgrid(k_recon_inner_p, pt, plan_grid(par0)) : plan_grid(par0), pb, 0, s>>>(
         P, C, nz, V.ip_i, V.ip_d, rec, PL);
@@ -265,11 +265,14 @@ void wt_level_wav_unbind(wt_handle* h) {
 // are written on the handle's stream: the scalar, inner and outer velocity
 // wavelets run on three side streams forked here.  The arrays must be clean
 // (wt_level_clean_wavelets) before the first pair of a WT_after_step.
-int wt_level_wav_forward_pair(wt_handle* h, int l) {
+int wt_level_wav_forward_pair(wt_handle* h, int l, cudaStream_t vs) {
   WavCtx* W = ctx(h);
-  cudaEvent_t f = W->fork[l - h->level_start];
+  const size_t q = l - h->level_start;
+  cudaEvent_t f = W->fork[q], fv = f;
   CKW(cudaEventRecord(f, h->stream));
-  for (int k = 1; k < 4; ++k) CKW(cudaStreamWaitEvent(W->side[k], f, 0));
+  if (vs && vs != h->stream) CKW(cudaEventRecord(fv = W->fork_v[q], vs));
+  CKW(cudaStreamWaitEvent(W->side[3], f, 0));
+  for (int k = 1; k < 3; ++k) CKW(cudaStreamWaitEvent(W->side[k], fv, 0));
   if (W->zero_ok) {
     launch_scalar_wc<2>(h, l, W->side[3]);
     launch_velo_wc<2>(h, l, W->side[2], W->side[1]);
@@ -312,7 +315,7 @@ void wt_wavelet_release(wt_handle* h) {
   if (!h || !h->wav) return;
   for (cudaEvent_t e : ctx(h)->ev)
     if (e) cudaEventDestroy(e);
-  for (auto* v : {&ctx(h)->fork, &ctx(h)->ready_v, &ctx(h)->ready_s})
+  for (auto* v : {&ctx(h)->fork, &ctx(h)->fork_v, &ctx(h)->ready_v, &ctx(h)->ready_s})
     for (cudaEvent_t e : *v)
       if (e) cudaEventDestroy(e);
   for (cudaStream_t s : ctx(h)->side)
@@ -419,9 +422,10 @@ int wt_wavelet_setup(wt_handle* h) {
   for (int k = 1; k < 4; ++k) CKW(cudaStreamCreateWithPriority(&W->side[k], cudaStreamNonBlocking, least));
   for (cudaEvent_t& e : W->ev) CKW(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   W->fork.assign(W->L.size(), nullptr);
+  W->fork_v.assign(W->L.size(), nullptr);
   W->ready_v.assign(W->L.size(), nullptr);
   W->ready_s.assign(W->L.size(), nullptr);
-  for (auto* v : {&W->fork, &W->ready_v, &W->ready_s})
+  for (auto* v : {&W->fork, &W->fork_v, &W->ready_v, &W->ready_s})
     for (cudaEvent_t& e : *v) CKW(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   zero_wavelets(h);
   CKW(cudaStreamSynchronize(h->stream));
@@ -1015,7 +1019,7 @@ int restrict_flux(wt_handle* h, int level, double* par0, double* par1, const dou
   if (!V.rf_pi) return WT_ERR_ARG;
   const int m = h->at(level).n;
   const int64_t ne = (int64_t)3 * 10 * m * m;
-  const dim3 blk(32, std::min(nz, 8));
+  const dim3 blk(32, 2 * std::min(nz, 8));
   const ParentList PL = wt_level_plist(h, level);
   const unsigned dense = (unsigned)((ne + 31) / 32);
   k_restr_flux3<<<PL.ids ? pgrid(k_restr_flux3, (int)(blk.x * blk.y), dense) : dense, blk, 0, h->stream>>>(
