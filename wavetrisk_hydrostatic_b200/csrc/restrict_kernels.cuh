@@ -433,30 +433,38 @@ __global__ void __launch_bounds__(512, 2) k_restr_flux3(WLev P, int m, int nz, c
   restr_flux_one(P, nz, si, sd, x, d, ip, jp, e, fp0, fp1, fc0, fc1, dc0, dc1, NNc);
 }
 
-// scalar_cpt_restr over parents [0, n]^2, every layer (with a work list, its
-// parents only, persistent threads).
-__global__ void k_restr_scalar(WLev P, WLev C, int nz, ParentList PL) {
-  const int m = P.n + 1;
+// scalar_cpt_restr of one or two fields (b null: one) over parents [0, n]^2, every
+// layer (with a work list, its parents only, persistent threads).  A thread takes a
+// parent in RS_K layers: the mask, the list entry and the indices serve them all.
+constexpr int RS_K = 4;
+__device__ __forceinline__ void restr_scalar_one(const WLev& P, const WLev& C, int nz, int k0, int d, int ip, int jp,
+                                                 double* pb, const double* __restrict__ cb) {
+  const int idp = nid(P, d, ip, jp), idc = nid(C, d, 2 * ip, 2 * jp);
+  if (P.mask_n[idp] < M_RESTRCT) return;
+#pragma unroll
+  for (int q = 0; q < RS_K; ++q)
+    if (k0 + q < nz) {
+      const int64_t o = (int64_t)(k0 + q) * P.NN + idp, c = (int64_t)(k0 + q) * C.NN + idc;
+      P.scal[o] = __ldg(C.scal + c);
+      if (pb) pb[o] = __ldg(cb + c);
+    }
+}
+__global__ void k_restr_scalar(WLev P, WLev C, int nz, double* pb, const double* __restrict__ cb, ParentList PL) {
+  const int m = P.n + 1, groups = (nz + RS_K - 1) / RS_K;
+  const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (PL.ids) {
-    const int cnt = __ldg(PL.count);
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)cnt * nz;
-         t += (int64_t)gridDim.x * blockDim.x) {
-      const int k = (int)(t / cnt), e = (int)(t - (int64_t)k * cnt);
+    const unsigned cnt = __ldg(PL.count);
+    for (unsigned t = t0; t < cnt * groups; t += gridDim.x * blockDim.x) {
+      const int g = t / cnt, e = t - g * cnt;
       int d, ip, jp;
-      if (!list_parent(P.n, __ldg(PL.ids + e), m, d, ip, jp)) continue;
-      const int idp = nid(P, d, ip, jp);
-      if (P.mask_n[idp] >= M_RESTRCT)
-        P.scal[(int64_t)k * P.NN + idp] = C.scal[(int64_t)k * C.NN + nid(C, d, 2 * ip, 2 * jp)];
+      if (list_parent(P.n, __ldg(PL.ids + e), m, d, ip, jp)) restr_scalar_one(P, C, nz, g * RS_K, d, ip, jp, pb, cb);
     }
     return;
   }
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)nz * 10 * m * m) return;
-  const int ip = (int)(t % m), jp = (int)((t / m) % m), d = (int)((t / ((int64_t)m * m)) % 10);
-  const int k = (int)(t / ((int64_t)10 * m * m));
-  const int idp = nid(P, d, ip, jp);
-  if (P.mask_n[idp] >= M_RESTRCT)
-    P.scal[(int64_t)k * P.NN + idp] = C.scal[(int64_t)k * C.NN + nid(C, d, 2 * ip, 2 * jp)];
+  const unsigned per = 10u * m * m;
+  if (t0 >= per * groups) return;
+  const int g = t0 / per, r = t0 - g * per, d = r / (m * m), jp = r / m - d * m, ip = r % m;
+  restr_scalar_one(P, C, nz, g * RS_K, d, ip, jp, pb, cb);
 }
 
 // flux_cpt_restr over parents [0, n)^2, every layer.

@@ -247,7 +247,7 @@ int wt_u_update_multi(wt_handle* h, double dt, double theta1) {
     const DevLevel& D = h->at(l);
     const int m = D.n + 1;
     if (l < h->level_end)
-      if (int rc = wt_level_restrict_scalar(h, l, V.eta_w, B->L[l + 1 - h->level_start].eta_w, 1)) return rc;
+      if (int rc = wt_level_restrict_scalar(h, l, V.eta_w, B->L[l + 1 - h->level_start].eta_w, nullptr, nullptr, 1)) return rc;
     double *ms, *v, *mm;
     level_state(h, l, &ms, &v, &mm);
     wtb::k_grad_eta_update<true><<<nb(10 * m * m), TPB, 0, h->stream>>>(D.view(), h->nz, h->ph.grav, V.eta_w,
@@ -319,7 +319,7 @@ int wt_level_grad_eta(wt_handle* h, const double** grad) {
     const DevLevel& D = h->at(l);
     const int m = D.n + 1;
     if (l < h->level_end)
-      if (int rc = wt_level_restrict_scalar(h, l, V.eta_w, B->L[l + 1 - h->level_start].eta_w, 1)) return rc;
+      if (int rc = wt_level_restrict_scalar(h, l, V.eta_w, B->L[l + 1 - h->level_start].eta_w, nullptr, nullptr, 1)) return rc;
     wtb::k_grad_eta_update<true><<<nb(10 * m * m), TPB, 0, h->stream>>>(D.view(), 0, h->ph.grav, V.eta_w, 0.0,
                                                                        V.grad, nullptr);
     grad[l - h->level_start] = V.grad;

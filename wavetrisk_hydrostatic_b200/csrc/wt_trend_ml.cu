@@ -271,8 +271,8 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
         CKM(cudaStreamWaitEvent(rs, M->done[q], 0));
         CKM(cudaStreamWaitEvent(rs, l + 1 == h->level_end ? M->s1top : M->done[q + 1], 0));
       }
-      if (int rc = wt_level_restrict_scalar(h, l, V.bern, C.bern, nz, rs)) return rc;
-      if (int rc = wt_level_restrict_scalar(h, l, V.phik, C.phik, nz, rs)) return rc;  // exner = -Phi_k
+      // the Bernoulli function and exner = -Phi_k
+      if (int rc = wt_level_restrict_scalar(h, l, V.bern, C.bern, V.phik, C.phik, nz, rs)) return rc;
       if (int rc = wt_level_restrict_flux(h, l, V.hfm, V.hft, C.hfm, C.hft, C.dm, C.dt, nz)) return rc;
       if (concurrent) {
         CKM(cudaEventRecord(M->rsd[q], rs));

@@ -998,15 +998,16 @@ int wt_wt_after_step(wt_handle* h) {
 
 }  // extern "C"
 
-int wt_level_restrict_scalar(wt_handle* h, int level, double* par, const double* chd, int nz, cudaStream_t stream) {
+int wt_level_restrict_scalar(wt_handle* h, int level, double* par, const double* chd, double* par1, const double* chd1,
+                             int nz, cudaStream_t stream) {
   WLev P = view(h, level), C = view(h, level + 1);
   P.scal = par;
   C.scal = const_cast<double*>(chd);
   const int m = h->at(level).n + 1;
   const ParentList PL = wt_level_plist(h, level);
-  const unsigned dense = nb((int64_t)nz * 10 * m * m);
-  k_restr_scalar<<<PL.ids ? pgrid(k_restr_scalar, TPB, dense) : dense, TPB, 0, stream ? stream : h->stream>>>(P, C, nz,
-                                                                                                              PL);
+  const unsigned dense = nb((int64_t)((nz + RS_K - 1) / RS_K) * 10 * m * m);
+  k_restr_scalar<<<PL.ids ? pgrid(k_restr_scalar, TPB, dense) : dense, TPB, 0, stream ? stream : h->stream>>>(
+      P, C, nz, par1, chd1, PL);
   CKW(cudaGetLastError());
   return WT_OK;
 }
@@ -1053,8 +1054,8 @@ int restrict_pair(wt_handle* h, int level, std::initializer_list<int> fields) {
 int wt_restrict_scalar(wt_handle* h, int level) {
   if (int rc = restrict_pair(h, level, {WT_WORK_SCALAR})) return rc;
   const int m = h->at(level).n + 1;
-  k_restr_scalar<<<nb((int64_t)h->nz * 10 * m * m), TPB, 0, h->stream>>>(view(h, level), view(h, level + 1), h->nz,
-                                                                          kNoList);
+  k_restr_scalar<<<nb((int64_t)((h->nz + RS_K - 1) / RS_K) * 10 * m * m), TPB, 0, h->stream>>>(
+      view(h, level), view(h, level + 1), h->nz, nullptr, nullptr, kNoList);
   CKW(cudaGetLastError());
   CKW(cudaStreamSynchronize(h->stream));
   return WT_OK;
