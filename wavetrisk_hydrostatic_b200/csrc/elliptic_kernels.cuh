@@ -15,6 +15,8 @@
 #pragma once
 #include <cstdint>
 
+#include "div_by.cuh"
+
 namespace wte {
 
 enum { RT = 0, DG = 1, UP = 2 };
@@ -24,6 +26,7 @@ struct EllLev {
   int64_t NN;
   const double* __restrict__ len;   // 3*NN
   const double* __restrict__ ped;   // 3*NN
+  const double* __restrict__ rlen;  // 3*NN reciprocals of len (div_by)
   const double* __restrict__ hinv;  // NN
   const double* __restrict__ oa;    // 4*NN overlap areas a(1..4)
   const double* __restrict__ Ie;    // 3*NN interp(csq(a), csq(b)) of each edge's own stencil
@@ -77,10 +80,15 @@ __device__ __forceinline__ int border_index(int n, int d, int i, int j) {
   return d * border_nodes(n) + b;
 }
 
+__global__ void k_recip(int64_t n, const double* __restrict__ a, double* __restrict__ y) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) y[k] = 1.0 / a[k];
+}
+
 // Flux of one edge (step1 itype 2, src/ops.f90:202-216):
 // interp(csq0, csq1) * (q1/phi1 - q0/phi0) / len * pedlen with phi = 1.
 __device__ __forceinline__ double ell_edge(const EllLev& L, int slot, double dq) {
-  return L.Ie[slot] * dq / L.len[slot] * L.ped[slot];
+  return wtk::div_by(L.Ie[slot] * dq, L.len[slot], L.rlen[slot]) * L.ped[slot];
 }
 __device__ __forceinline__ float ell_edge(const EllLev& L, int slot, float dq) { return L.Kf[slot] * dq; }
 
@@ -256,8 +264,8 @@ __global__ void k_ell_lc(EllLev L, double* __restrict__ s, double a1, const doub
 // shuffle order); the partials are added in a fixed order by 256 threads, so a
 // sum has the same bits whichever kernel forms it.
 __device__ __forceinline__ double ell_weigh(const EllLev& L, int i, int j, double x) {
-  const int wi = (i > 0 && i < L.n && i % L.nd == 0) ? 2 : 1;
-  const int wj = (j > 0 && j < L.n && j % L.nd == 0) ? 2 : 1;
+  const int wi = (i > 0 && i < L.n && (i & (L.nd - 1)) == 0) ? 2 : 1;  // nd is a power of two
+  const int wj = (j > 0 && j < L.n && (j & (L.nd - 1)) == 0) ? 2 : 1;
   double v = x;
   if (wi * wj >= 2) v = v + x;
   if (wi * wj == 4) v = v + x + x;
@@ -286,18 +294,26 @@ __device__ __forceinline__ double ell_finish(double v, int mode, const double* d
   return v;
 }
 
-// The partial of this block into partial[]; the last block of the grid to
-// arrive (ticket, which it resets) adds them all and writes *out.  One launch a
-// reduction instead of two; blocks of 256 threads.
-__device__ __forceinline__ void ell_reduce(double v, double* partial, unsigned* ticket, double* out, int mode,
+// Sums over the nodes [0, n]^2 by resident blocks: value(t) of node t, chunk c (nodes
+// 256 c .. 256 c + 255) into partial[c], chunks strided over the grid; the last block
+// to arrive (ticket, which it resets) adds the partials and writes *out.  One launch
+// a reduction instead of two, and one fence and one ticket a resident block, not a
+// chunk (2580 at J8: k_ell_resid_norm 39 -> 35 us).
+constexpr int RED_PER_SM = 4;  // resident blocks of 256 threads
+template <class F>
+__device__ __forceinline__ void ell_reduce(int nodes, F value, double* partial, unsigned* ticket, double* out, int mode,
                                            const double* den) {
-  __shared__ double sh[8];
+  __shared__ double sh[2][8];
   __shared__ bool last;
   auto bar = [] { __syncthreads(); };
-  const int tid = threadIdx.x;
-  v = ell_sum256(v, sh, tid, bar);
+  const int tid = threadIdx.x, chunks = (nodes + 255) / 256;
+  int par = 0;  // a chunk's warp sums are read while the next chunk's are written
+  for (int c = blockIdx.x; c < chunks; c += gridDim.x, par ^= 1) {
+    const int t = c * 256 + tid;
+    const double v = ell_sum256(t < nodes ? value(t) : 0.0, sh[par], tid, bar);
+    if (tid == 0) partial[c] = v;
+  }
   if (tid == 0) {
-    partial[blockIdx.x] = v;
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
@@ -305,27 +321,27 @@ __device__ __forceinline__ void ell_reduce(double v, double* partial, unsigned* 
   if (!last) return;
   __threadfence();
   double a = 0.0;
-  for (int k = tid; k < (int)gridDim.x; k += 256) a += __ldcg(partial + k);
-  a = ell_sum256(a, sh, tid, bar);
+  for (int k = tid; k < chunks; k += 256) a += __ldcg(partial + k);
+  a = ell_sum256(a, sh[0], tid, bar);
   if (tid == 0) {
     *out = ell_finish(a, mode, den);
     *ticket = 0;
   }
 }
 
-__global__ void __launch_bounds__(256) k_ell_dot(EllLev L, const double* __restrict__ a, const double* __restrict__ b,
-                                                 double* partial, unsigned* ticket, double* out, int mode,
-                                                 const double* den) {
+__global__ void __launch_bounds__(256, RED_PER_SM)
+    k_ell_dot(EllLev L, const double* __restrict__ a, const double* __restrict__ b, double* partial, unsigned* ticket,
+              double* out, int mode, const double* den) {
   const int m = L.n + 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (t < 10 * m * m) {
-    int d, i, j;
-    decode(L, t, d, i, j, m);
-    const int s = L.nsrc[nidx(L, d, i, j)];
-    v = ell_weigh(L, i, j, a[s] * b[s]);
-  }
-  ell_reduce(v, partial, ticket, out, mode, den);
+  ell_reduce(
+      10 * m * m,
+      [&](int t) {
+        int d, i, j;
+        decode(L, t, d, i, j, m);
+        const int s = L.nsrc[nidx(L, d, i, j)];
+        return ell_weigh(L, i, j, a[s] * b[s]);
+      },
+      partial, ticket, out, mode, den);
 }
 
 // r = f - L(u), its weighted norm into *out (mode, den) and, where given, r
@@ -333,37 +349,36 @@ __global__ void __launch_bounds__(256) k_ell_dot(EllLev L, const double* __restr
 // u + w r / diag.  A copy of another node takes the residual of its source, as
 // the sum over stored values would.  One stencil pass instead of residual, dot
 // and conversion passes.
-__global__ void __launch_bounds__(256, 4) k_ell_resid_norm(EllLev L, const double* __restrict__ u,
-                                                        const double* __restrict__ f, double* __restrict__ r64,
-                                                        float* __restrict__ r32, double* __restrict__ next, double w,
-                                                        double* partial, unsigned* ticket, double* out, int mode,
-                                                        const double* den) {
+__global__ void __launch_bounds__(256, RED_PER_SM)
+    k_ell_resid_norm(EllLev L, const double* __restrict__ u, const double* __restrict__ f, double* __restrict__ r64,
+                     float* __restrict__ r32, double* __restrict__ next, double w, double* partial, unsigned* ticket,
+                     double* out, int mode, const double* den) {
   const int m = L.n + 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (t < 10 * m * m) {
-    int d, i, j;
-    decode(L, t, d, i, j, m);
-    const int id = nidx(L, d, i, j);
-    const bool inner = ell_inner(L, i, j);
-    int s = id, sd = d, si = i, sj = j;
-    if (!inner) {
-      s = L.nsrc[id];
-      const int row = s / L.P;
-      si = s - row * L.P - 2;
-      sd = row / L.P;
-      sj = row - sd * L.P - 2;
-    }
-    const double uc = u[s], fs = f[s];
-    const double r = fs - ell_lo(L, [&](int x) { return u[x]; }, s, sd, si, sj, inner || ell_inner(L, si, sj), uc);
-    if (s == id) {
-      if (r64) r64[id] = r;
-      if (r32) r32[id] = (float)r;
-      if (next) next[id] = uc + w * r / L.diag[id];
-    }
-    v = ell_weigh(L, i, j, r * r);
-  }
-  ell_reduce(v, partial, ticket, out, mode, den);
+  ell_reduce(
+      10 * m * m,
+      [&](int t) {
+        int d, i, j;
+        decode(L, t, d, i, j, m);
+        const int id = nidx(L, d, i, j);
+        const bool inner = ell_inner(L, i, j);
+        int s = id, sd = d, si = i, sj = j;
+        if (!inner) {
+          s = L.nsrc[id];
+          const int row = s / L.P;
+          si = s - row * L.P - 2;
+          sd = row / L.P;
+          sj = row - sd * L.P - 2;
+        }
+        const double uc = u[s], fs = f[s];
+        const double r = fs - ell_lo(L, [&](int x) { return u[x]; }, s, sd, si, sj, inner || ell_inner(L, si, sj), uc);
+        if (s == id) {
+          if (r64) r64[id] = r;
+          if (r32) r32[id] = (float)r;
+          if (next) next[id] = uc + w * r / L.diag[id];
+        }
+        return ell_weigh(L, i, j, r * r);
+      },
+      partial, ticket, out, mode, den);
 }
 
 // ---------------------------------------------------------- cluster kernels ----

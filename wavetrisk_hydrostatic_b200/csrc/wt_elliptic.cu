@@ -36,7 +36,7 @@ struct MField {
 struct ELevelDev {
   int level = 0, n = 0, P = 0, nd = 1;
   int64_t NN = 0;
-  double *Ie = nullptr, *diag = nullptr;
+  double *Ie = nullptr, *diag = nullptr, *rlen = nullptr;
   int *nsrc = nullptr, *esrc = nullptr, *bt = nullptr;
   float *Kf = nullptr, *hinvf = nullptr, *diagf = nullptr, *oaf = nullptr;
 };
@@ -52,6 +52,7 @@ struct Ell {
   bool eta_wc_valid = false;
   MField u32, f32, r32, c32, t32;  // FP32 V-cycle work
   double* partial = nullptr;
+  int sms = 1;  // multiprocessors
   unsigned* ticket = nullptr;  // arrivals of a reduction's blocks (0 between launches)
   double* clpart = nullptr;    // partial sums of the cluster kernels
   double* scal = nullptr;      // device scalars
@@ -66,7 +67,7 @@ struct Ell {
     const DevLevel& D = const_cast<wt_handle*>(h)->at(l);
     const ELevelDev& E = L[l - ls];
     const auto magic = [](int m) { return ((1ull << 40) + m - 1) / m; };
-    return EllLev{D.n, D.P, E.nd, D.NN, D.len, D.pedlen, D.hex_inv, D.overl_a, E.Ie, E.diag, E.nsrc, E.esrc,
+    return EllLev{D.n, D.P, E.nd, D.NN, D.len, D.pedlen, E.rlen, D.hex_inv, D.overl_a, E.Ie, E.diag, E.nsrc, E.esrc,
                   E.Kf, E.hinvf, E.diagf, E.oaf, E.bt, cf, magic(D.n + 1), magic(D.n)};
   }
   int m(int l) const { return L[l - ls].n + 1; }
@@ -243,6 +244,8 @@ extern "C" int wt_elliptic_setup(wt_handle* h, double dt, double theta1, double 
     cudaMemcpy(X.diagf, diagf.data(), 4 * NN, cudaMemcpyHostToDevice);
     if ((rc = dalloc(*E, &X.oaf, 4 * NN))) break;
     k_d2f<<<nb(4 * NN), TPB>>>(4 * NN, D.overl_a, X.oaf);
+    if ((rc = dalloc(*E, &X.rlen, 3 * NN))) break;
+    k_recip<<<nb(3 * NN), TPB>>>(3 * NN, D.len, X.rlen);
     if ((rc = dalloc(*E, &X.bt, 18 * 10 * (int64_t)border_nodes(D.n)))) break;
     k_ell_border<<<nb(10 * (int64_t)(D.n + 1) * (D.n + 1)), TPB>>>(D.n, D.P, (int)NN, D.nsrc, D.esrc, X.bt);
     E->L.push_back(X);
@@ -256,6 +259,9 @@ extern "C" int wt_elliptic_setup(wt_handle* h, double dt, double theta1, double 
   for (MField* F : f32)
     if (rc == WT_OK) rc = alloc_field(*E, *F, true);
   if (rc == WT_OK) rc = dalloc(*E, &E->partial, E->nbmax);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&E->sms, cudaDevAttrMultiProcessorCount, dev);
   if (rc == WT_OK) rc = dalloc(*E, &E->ticket, 1);
   if (rc == WT_OK) rc = dalloc(*E, &E->clpart, CL_PARTIALS);
   if (rc == WT_OK) rc = dalloc(*E, &E->scal, 64);
@@ -280,9 +286,14 @@ void op(Ell& E, int OPK, int l, const double* q, const double* f, double* out, d
   if (OPK == OP_JACOBI) k_ell_op<OP_JACOBI, double><<<g, TPB, 0, E.s()>>>(V, q, f, out, w, nullptr);
 }
 
+// Blocks of a reduction over level l's nodes (ell_reduce).
+unsigned red_grid(const Ell& E, int l) {
+  return std::min<unsigned>(nb(10 * E.m(l) * E.m(l)), RED_PER_SM * E.sms);
+}
+
 // weighted dot / l2 into a device scalar; returns nothing (async)
 void dot_to(Ell& E, int l, const double* a, const double* b, double* out, int mode, const double* den = nullptr) {
-  k_ell_dot<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), a, b, E.partial, E.ticket, out, mode, den);
+  k_ell_dot<<<red_grid(E, l), TPB, 0, E.s()>>>(E.view(l), a, b, E.partial, E.ticket, out, mode, den);
 }
 void dot_dev(Ell& E, int l, const double* a, const double* b, int slot, int mode, const double* den = nullptr) {
   dot_to(E, l, a, b, E.scal + slot, mode, den);
@@ -357,7 +368,7 @@ void interp_level(Ell& E, int fl, const double* src, double* dst, bool add) {
 // |f - L u| / nrm on the device (residual and norm in one pass), to the host
 double res_err(Ell& E, MField& f, MField& u, double nrm_f, int l) {
   const int q = l - E.ls;
-  k_ell_resid_norm<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(E.view(l), u.lv[q], f.lv[q], nullptr, nullptr, nullptr,
+  k_ell_resid_norm<<<red_grid(E, l), TPB, 0, E.s()>>>(E.view(l), u.lv[q], f.lv[q], nullptr, nullptr, nullptr,
                                                                 0.0, E.partial, E.ticket, E.scal, 1, nullptr);
   return fetch(E, 0) / nrm_f;
 }
@@ -543,10 +554,10 @@ void srj(Ell& E, const wt_solver_opts& o, wt_solver_report& rep) {
       const int nb_ = std::min(m, max_iter - iter);
       for (int k = 0; k < nb_; ++k) {
         // norm of ring[k] (the state after sweep iter + k) and sweep iter + k + 1 into ring[k + 1]
-        k_ell_resid_norm<<<g, TPB, 0, E.s()>>>(V, ring[k], f.lv[q], nullptr, nullptr, ring[k + 1], w[(iter + k) % m],
+        k_ell_resid_norm<<<red_grid(E, l), TPB, 0, E.s()>>>(V, ring[k], f.lv[q], nullptr, nullptr, ring[k + 1], w[(iter + k) % m],
                                                E.partial, E.ticket, E.scal + 8 + k, 1, nullptr);
       }
-      k_ell_resid_norm<<<g, TPB, 0, E.s()>>>(V, ring[nb_], f.lv[q], nullptr, nullptr, nullptr, 0.0, E.partial, E.ticket,
+      k_ell_resid_norm<<<red_grid(E, l), TPB, 0, E.s()>>>(V, ring[nb_], f.lv[q], nullptr, nullptr, nullptr, 0.0, E.partial, E.ticket,
                                              E.scal + 8 + nb_, 1, nullptr);
       double nrm[m + 1];
       cudaMemcpyAsync(nrm, E.scal + 8, 8 * (nb_ + 1), cudaMemcpyDeviceToHost, E.s());

@@ -105,7 +105,7 @@ int mixed_ir(Ell& E, const wt_solver_opts& o, wt_solver_report& rep, bool fp64 =
   double err = 0.0;
   for (it = 0; it <= o.ir_max; ++it) {
     // the residual, its norm and (mixed) its FP32 copy in one pass
-    k_ell_resid_norm<<<nb(10 * E.m(l) * E.m(l)), TPB, 0, E.s()>>>(
+    k_ell_resid_norm<<<red_grid(E, l), TPB, 0, E.s()>>>(
         E.view(l), E.u.lv[q], E.f.lv[q], fp64 ? E.res.lv[q] : nullptr, fp64 ? nullptr : E.r32.lvf[q], nullptr, 0.0,
         E.partial, E.ticket, E.scal, 1, nullptr);
     err = fetch(E, 0) / nf;
