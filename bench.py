@@ -442,29 +442,28 @@ def adaptive_launches(L, need_r=4):
     (AdaptiveOcean.step with fixed thresholds once the tree's level_end is the
     top: one graph replay); C = L - 1 parent levels, the same number of levels
     above level_start.
-    * RK4, per stage: column, step1 and trend of every level (the levels above
-      level_start over their work lists), two scalar and one flux restriction
-      and three forward-wavelet kernels per parent level; four inverse kernels
-      per parent level after each of the first three stages and after adapt.
+    * RK4, per stage: column, step1 and the trend's scalars and velocity of every
+      level (the levels above level_start over their work lists), a scalar and a
+      flux restriction and three forward-wavelet kernels per parent level; four
+      inverse kernels per parent level after each of the first three stages and
+      after adapt.
     * adapt's mask sequence (init_masks_zero, mask_active, the sweeps with
-      refine() of the tree, complete_masks, mask_trsk and 3C + 6 comm_masks).
+      refine() of the tree, complete_masks, mask_trsk and 3C + 5 comm_masks).
     * The maps: one seed, need_r dilations and the cut to the tree; per parent
-      level seven reconstruct-map launches; three launches per work list (one
-      per level above level_start and one per parent level).
+      level four reconstruct-map launches; three launches for the work lists.
     * compress_wavelets of the dropped slots.
-    The ncu launch list of one step (profiles/adaptive_J5-J9x32_step_launch_list.md)
-    counts 360 for L = 5."""
+    The kernel timeline of one step at J4..J7 counts 243 for L = 4."""
     C = L - 1
-    stage = 12 * L + 12 * C + 12 * C + 16 * C
-    masks = C + 3 * L + 13 * C + 4
-    maps = 1 + need_r + C + 7 * C + 3 * C + 3 * C
+    stage = 16 * L + 8 * C + 12 * C + 16 * C
+    masks = 13 * C + 8
+    maps = 1 + need_r + 1 + 4 * C + 3
     return stage + masks + maps + C
 
 
 def algorithmic_bytes_trend_ml(level, nz, n_on=None, n_own=None, n_listed=None):
     """Compulsory bytes of one multi-level trend launch on a level with the
-    fused RK sub-step (k_trend_ml, k_trend_ml_list over the level's work list,
-    or k_trend_tma<MODE_ML> on the finest level, which stages every input plane
+    fused RK sub-step (k_trend_ml_scal and k_trend_ml_velo, their list forms over the
+    level's work list, or k_trend_tma on the finest level, which stages every input plane
     of a tile, so its traffic is higher).  Every node of [0, n]^2 reads its mask
     and writes dmass and dTheta (2 words a layer); every owned node writes the
     velocity source (3); the n_on nodes with mask_n >= TRSK also read theta,
@@ -748,7 +747,7 @@ def bench_ours(args):
         share = {k: pm[k] * pc[k] for k in pm}
         tot = sum(share.values())
         dom = max(share, key=lambda k: share[k])
-        # the roofline kernel: the finest level's k_trend_ml_list (its work list
+        # the roofline kernels: the finest level's trend, scalars and velocity (its work list
         # = the needed slots), timed in the profiled step that takes the same maps
         listed = r["tree"]["levels"][-1]["needed_owned_nodes"]
         ab = algorithmic_bytes_trend_ml(args.level, args.nz, n_on=r["masks"][-1]["trsk_nodes_0n"], n_listed=listed)
@@ -756,15 +755,6 @@ def bench_ours(args):
         ach = ab / (t_list / 1e3) / 1e9
         ab_dense = algorithmic_bytes_trend_ml(args.level, args.nz)
         t_dense = r["phase_ms_dense"]["trend_ml_top"]
-        traffic = None
-        tf = os.path.join(ROOT, "profiles", "trend_ml_list_traffic.json")
-        if os.path.exists(tf):
-            try:
-                tj = json.load(open(tf))
-                if tj.get("traffic_per_algorithmic_byte"):   # measured on a smaller case, scaled by the bytes
-                    traffic = int(tj["traffic_per_algorithmic_byte"] * ab)
-            except Exception:
-                traffic = None
         cpu = cpu_baseline(args, quick=True, tree_fraction=r["tree_init"]["tree_fraction"])
         L = args.level - args.lmin + 1
         line = {
@@ -789,16 +779,13 @@ def bench_ours(args):
                             "finest level's patch bytes out, every step (bytes: averages over the steps)",
                     "parts_ms_per_step": r["e2e_parts_ms"]},
             "gpu_launches": adaptive_launches(L) * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "k_trend_ml_list (level_end, over its work list)", "achieved": ach,
-                         "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_src, "traffic": traffic,
+            "roofline": {"bound": "hbm", "kernel": "k_trend_ml_scal_list + k_trend_ml_velo_list (level_end, over its work list)", "achieved": ach,
+                         "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_src, "traffic": None,
                          "algorithmic_bytes_per_launch": ab, "listed_owned_nodes": listed,
                          "kernel_ms": t_list,
                          "timing": "CUDA events around the kernel's launches in one profiled RK4 step (phase by phase, "
                                    "the same needed-node maps and work lists as the timed steps)",
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the same kernel on the "
-                                           "J5..J7 x 32 workload, per algorithmic byte, scaled to this launch "
-                                           "(profiles/trend_ml_list_traffic.json)" if traffic else None,
-                         "dense_tma_kernel": {"kernel": "k_trend_tma<MODE_ML> with every node computed (maps off)",
+                         "dense_tma_kernel": {"kernel": "k_trend_tma with every node computed (maps off)",
                                               "ms": t_dense, "algorithmic_bytes": ab_dense,
                                               "achieved_GBps": ab_dense / (t_dense / 1e3) / 1e9,
                                               "frac": ab_dense / (t_dense / 1e3) / 1e9 / hbm},
@@ -896,7 +883,7 @@ def bench_ours_uniform(args):
             "e2e": {"value": e2e_value, "unit": "simulated days per wall-clock hour",
                     "h2d_bytes_per_step": r["h2d_bytes_per_step"], "d2h_bytes_per_step": r["d2h_bytes_per_step"],
                     "path": "wt_rk4_step_host (C-ABI), pinned host buffers, state copied in and out every step"},
-            "gpu_launches": 12 * args.steps,
+            "gpu_launches": (16 if args.level >= 6 else 12) * args.steps,
             "roofline": {"bound": "hbm", "kernel": "trend_rk", "achieved": ach, "peak": hbm, "unit": "GB/s",
                          "frac": ach / hbm, "peak_source": peak_src, "traffic": traffic,
                          "dominant_kernel_by_time": dom, "kernel_ms_per_launch": kt},

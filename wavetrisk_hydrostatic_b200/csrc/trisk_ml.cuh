@@ -1,8 +1,7 @@
 // Trend of one level of the multi-level trend_ml (src/multi_level.f90:5-188):
 // scalar_trend with its mask, the velocity source computed (du_source) or
 // restricted from the child level (u_source_cpt_restr, src/multi_level.f90:
-// 365-392), and du_grad with its mask (src/ops.f90:739-832), in one pass per
-// (layer, node).  The Bernoulli function, Phi_k and the mass and Theta fluxes
+// 365-392), and du_grad with its mask (src/ops.f90:739-832).  The Bernoulli function, Phi_k and the mass and Theta fluxes
 // it reads are those of the level after their compute-or-restrict step.
 #pragma once
 #include "trisk_read.cuh"
