@@ -129,7 +129,8 @@ int wt_level_after_step(wt_handle* h, double* const* m, double* const* t, double
 // WT_after_step in pieces, for callers that launch each level pair's forward
 // wavelets as soon as both levels' fields are written: bind the stage's scaling
 // fields, wt_level_clean_wavelets, wt_level_wav_forward_pair for every l in
-// [level_start, level_end), wt_level_wav_finish, unbind.
+// [level_start, level_end), wt_level_wav_finish, unbind.  velo: the stream that writes
+// the velocity (null: the handle's, which writes the scalars).
 void wt_level_wav_bind(wt_handle* h, double* const* m, double* const* t, double* const* v);
 void wt_level_wav_unbind(wt_handle* h);
 int wt_level_wav_forward_pair(wt_handle* h, int level, cudaStream_t velo = nullptr);

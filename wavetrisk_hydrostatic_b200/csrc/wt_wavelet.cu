@@ -262,8 +262,8 @@ void wt_level_wav_unbind(wt_handle* h) {
 
 // The wavelets of level l+1 from the scaling fields of levels l and l+1, with
 // zero_float and compress_wavelets folded in (CMP), once both levels' fields
-// are written on the handle's stream: the scalar, inner and outer velocity
-// wavelets run on three side streams forked here.  The arrays must be clean
+// are written (the scalars on the handle's stream, the velocity on vs): the scalar,
+// inner and outer velocity wavelets run on three side streams forked here.  The arrays must be clean
 // (wt_level_clean_wavelets) before the first pair of a WT_after_step.
 int wt_level_wav_forward_pair(wt_handle* h, int l, cudaStream_t vs) {
   WavCtx* W = ctx(h);
