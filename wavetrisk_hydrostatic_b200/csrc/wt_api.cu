@@ -180,14 +180,16 @@ static int make_ghost_lists(wt_handle* h, const DevLevel& D, const std::vector<i
   return WT_OK;
 }
 
-// Trend input maps of the FP32 flux arrays.
-static int make_f32_maps(wt_handle* h) {
+// The pipelined kernels copy FP32 planes only where a row of the padded level is a
+// multiple of 16 bytes (from level 2 up); the L1 kernels take any level.
+static bool f32_staged(wt_handle* h) { return h->trend_variant == 0 && h->top().P % 4 == 0; }
+
+// Trend input maps of the FP32 flux arrays a (qe, hfm, hft, ke, theta).
+static int make_f32_maps(wt_handle* h, float* const* a, TrendMapsF& M) {
   const int nz = h->nz;
-  TrendMapsF& M = h->fmaps;
   auto mk = [&](CUtensorMap* m, const float* base, int planes) { return top_map(h, m, base, planes, FBX, PipeTile::BY); };
-  const bool ok = mk(&M.hfm, h->hfm32, 3 * nz) && mk(&M.hft, h->hft32, 3 * nz) && mk(&M.qe, h->qe32, 3 * nz) &&
-                  mk(&M.theta, h->theta32, nz) && mk(&M.ke, h->ke32, nz) &&
-                  top_map(h, &M.phik, h->phik, nz, PBX, PipeTile::BY) &&
+  const bool ok = mk(&M.qe, a[0], 3 * nz) && mk(&M.hfm, a[1], 3 * nz) && mk(&M.hft, a[2], 3 * nz) && mk(&M.ke, a[3], nz) &&
+                  mk(&M.theta, a[4], nz) && top_map(h, &M.phik, h->phik, nz, PBX, PipeTile::BY) &&
                   top_map(h, &M.pterm, h->pterm, nz, PBX, PipeTile::BY);
   if (!ok) {
     std::fprintf(stderr, "wavetrisk_gpu: tensor map encoding failed\n");
@@ -349,7 +351,9 @@ int wt_set_flux_precision(wt_handle* h, int bits) {
       if (e == cudaSuccess) e = cudaMemset(*arrays[q], 0, sizeof(float) * sizes[q]);
       if (e != cudaSuccess) return wt_handle_fail("flux fp32 arrays", e);
     }
-    if (int rc = make_f32_maps(h)) return rc;
+    float* a[] = {h->qe32, h->hfm32, h->hft32, h->ke32, h->theta32};
+    if (f32_staged(h))
+      if (int rc = make_f32_maps(h, a, h->fmaps)) return rc;
   }
   if (h->graph_exec) {
     cudaGraphExecDestroy(h->graph_exec);
@@ -473,7 +477,8 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   (void)halo_first;
   // block b: layer b % nz of node chunk b / nz (layer_node in trisk_kernels.cuh)
   const unsigned chunks = blocks_for(D.NN, NODE_TILE);
-  const bool pipe = h->trend_variant == 0;  // pipelined tiles (trisk_pipe.cuh)
+  const bool f32 = h->flux_bits == 32;
+  const bool pipe = f32 ? f32_staged(h) : h->trend_variant == 0;  // pipelined tiles (trisk_pipe.cuh)
   const unsigned cb = blocks_for(D.NN, COL_TILE);
   const unsigned gb = pipe ? ghost_blocks(h->ghosts.n_nodes + h->ghosts.n_edges, nz, COL_TILE) : 0;
   TB(1);
@@ -486,7 +491,6 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   double* dm = mode == MODE_RK ? om : h->dm;
   double* dt = mode == MODE_RK ? ot : h->dt;
   double* dv = mode == MODE_RK ? ov : h->dv;
-  const bool f32 = h->flux_bits == 32;
   if (pipe) {
     const int sb = (m == h->m1) ? 1 : (m == h->m2) ? 2 : 0;  // which state buffer the stage reads
     auto grid = [&](int nodes) {
