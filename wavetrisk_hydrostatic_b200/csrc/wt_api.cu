@@ -343,17 +343,27 @@ int wt_set_flux_precision(wt_handle* h, int bits) {
   if (!h || (bits != 64 && bits != 32)) return WT_ERR_ARG;
   if (bits == h->flux_bits) return WT_OK;
   if (bits == 32 && !h->qe32) {
+    // all or nothing: qe32 says that the five arrays and the maps are there
     const int64_t nn = (int64_t)h->nz * h->top().NN;
-    float** arrays[] = {&h->qe32, &h->hfm32, &h->hft32, &h->ke32, &h->theta32};
-    const int64_t sizes[] = {3 * nn, 3 * nn, 3 * nn, nn, nn};
-    for (int q = 0; q < 5; ++q) {
-      cudaError_t e = cudaMalloc(arrays[q], sizeof(float) * sizes[q]);
-      if (e == cudaSuccess) e = cudaMemset(*arrays[q], 0, sizeof(float) * sizes[q]);
-      if (e != cudaSuccess) return wt_handle_fail("flux fp32 arrays", e);
+    const int64_t sizes[5] = {3 * nn, 3 * nn, 3 * nn, nn, nn};
+    float* a[5] = {};
+    int rc = WT_OK;
+    for (int q = 0; q < 5 && rc == WT_OK; ++q) {
+      cudaError_t e = cudaMalloc(&a[q], sizeof(float) * sizes[q]);
+      if (e == cudaSuccess) e = cudaMemset(a[q], 0, sizeof(float) * sizes[q]);
+      if (e != cudaSuccess) rc = wt_handle_fail("flux fp32 arrays", e);
     }
-    float* a[] = {h->qe32, h->hfm32, h->hft32, h->ke32, h->theta32};
-    if (f32_staged(h))
-      if (int rc = make_f32_maps(h, a, h->fmaps)) return rc;
+    if (rc == WT_OK && f32_staged(h)) rc = make_f32_maps(h, a, h->fmaps);
+    if (rc != WT_OK) {
+      for (float* p : a) cudaFree(p);
+      cudaGetLastError();  // reported: a later call must not find the failed allocation
+      return rc;
+    }
+    h->qe32 = a[0];
+    h->hfm32 = a[1];
+    h->hft32 = a[2];
+    h->ke32 = a[3];
+    h->theta32 = a[4];
   }
   if (h->graph_exec) {
     cudaGraphExecDestroy(h->graph_exec);
