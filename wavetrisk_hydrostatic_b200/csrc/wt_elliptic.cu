@@ -123,11 +123,12 @@ int capture_graph(Ell& E, cudaGraphExec_t& ex, std::vector<const void*>& ptrs, c
   return WT_OK;
 }
 
+// A zeroed device array (zeroed on the solver's stream).
 template <class T>
 int dalloc(Ell& E, T** p, int64_t n) {
   cudaError_t e = cudaMalloc(p, sizeof(T) * std::max<int64_t>(1, n));
   if (e != cudaSuccess) return wt_handle_fail("elliptic alloc", e);
-  cudaMemset(*p, 0, sizeof(T) * std::max<int64_t>(1, n));
+  cudaMemsetAsync(*p, 0, sizeof(T) * std::max<int64_t>(1, n), E.s());
   E.allocs.push_back(*p);
   return WT_OK;
 }
@@ -237,17 +238,17 @@ extern "C" int wt_elliptic_setup(wt_handle* h, double dt, double theta1, double 
     if ((rc = dalloc(*E, &X.Kf, 3 * NN))) break;
     if ((rc = dalloc(*E, &X.hinvf, NN))) break;
     if ((rc = dalloc(*E, &X.diagf, NN))) break;
-    cudaMemcpy(X.Ie, Ie.data(), 8 * 3 * NN, cudaMemcpyHostToDevice);
-    cudaMemcpy(X.diag, diag.data(), 8 * NN, cudaMemcpyHostToDevice);
-    cudaMemcpy(X.Kf, Kf.data(), 4 * 3 * NN, cudaMemcpyHostToDevice);
-    cudaMemcpy(X.hinvf, hinvf.data(), 4 * NN, cudaMemcpyHostToDevice);
-    cudaMemcpy(X.diagf, diagf.data(), 4 * NN, cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(X.Ie, Ie.data(), 8 * 3 * NN, cudaMemcpyHostToDevice, E->s());
+    cudaMemcpyAsync(X.diag, diag.data(), 8 * NN, cudaMemcpyHostToDevice, E->s());
+    cudaMemcpyAsync(X.Kf, Kf.data(), 4 * 3 * NN, cudaMemcpyHostToDevice, E->s());
+    cudaMemcpyAsync(X.hinvf, hinvf.data(), 4 * NN, cudaMemcpyHostToDevice, E->s());
+    cudaMemcpyAsync(X.diagf, diagf.data(), 4 * NN, cudaMemcpyHostToDevice, E->s());
     if ((rc = dalloc(*E, &X.oaf, 4 * NN))) break;
-    k_d2f<<<nb(4 * NN), TPB>>>(4 * NN, D.overl_a, X.oaf);
+    k_d2f<<<nb(4 * NN), TPB, 0, E->s()>>>(4 * NN, D.overl_a, X.oaf);
     if ((rc = dalloc(*E, &X.rlen, 3 * NN))) break;
-    k_recip<<<nb(3 * NN), TPB>>>(3 * NN, D.len, X.rlen);
+    k_recip<<<nb(3 * NN), TPB, 0, E->s()>>>(3 * NN, D.len, X.rlen);
     if ((rc = dalloc(*E, &X.bt, 18 * 10 * (int64_t)border_nodes(D.n)))) break;
-    k_ell_border<<<nb(10 * (int64_t)(D.n + 1) * (D.n + 1)), TPB>>>(D.n, D.P, (int)NN, D.nsrc, D.esrc, X.bt);
+    k_ell_border<<<nb(10 * (int64_t)(D.n + 1) * (D.n + 1)), TPB, 0, E->s()>>>(D.n, D.P, (int)NN, D.nsrc, D.esrc, X.bt);
     E->L.push_back(X);
     E->nbmax = std::max<int>(E->nbmax, (int)nb(10 * (int64_t)(D.n + 1) * (D.n + 1)));
   }
@@ -265,8 +266,8 @@ extern "C" int wt_elliptic_setup(wt_handle* h, double dt, double theta1, double 
   if (rc == WT_OK) rc = dalloc(*E, &E->ticket, 1);
   if (rc == WT_OK) rc = dalloc(*E, &E->clpart, CL_PARTIALS);
   if (rc == WT_OK) rc = dalloc(*E, &E->scal, 64);
-  // the set-up ran on the default stream, which the handle's stream does not wait for
-  if (rc == WT_OK && cudaDeviceSynchronize() != cudaSuccess) rc = wt_handle_fail("elliptic setup", cudaGetLastError());
+  // all of it ran on the handle's stream: the process's other streams are not waited for
+  if (cudaError_t e = cudaStreamSynchronize(E->s()); rc == WT_OK && e != cudaSuccess) rc = wt_handle_fail("elliptic setup", e);
   if (rc != WT_OK) {
     ell_free(E);
     return rc;
