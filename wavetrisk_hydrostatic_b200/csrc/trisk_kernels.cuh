@@ -393,7 +393,9 @@ __device__ __forceinline__ void step1_node(const LevelDev& L, int nz, const doub
 // reference's update_bdry(horiz_flux)).  For MODE_RK every node of the padded
 // level (all layers) is written as dest = base + h * trend (trend = 0 where
 // the reference leaves it zero); MODE_TREND writes the trends themselves.
-enum { MODE_TREND = 0, MODE_RK = 1 };
+// MODE_ML: one level of the multi-level trend_ml at the finest level (no
+// restricted source), with the RK sub-step (trisk_tma.cuh only).
+enum { MODE_TREND = 0, MODE_RK = 1, MODE_ML = 2 };
 
 
 template <int MODE>

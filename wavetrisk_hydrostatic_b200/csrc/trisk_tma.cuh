@@ -1,6 +1,7 @@
-// Trend + RK sub-step kernel of a hierarchy's finest level with its stencil inputs
-// staged in shared memory by the tensor memory accelerator (TMA), and the step1 that
-// goes with it.  (The single-level stepper has pipelined kernels, trisk_pipe.cuh.)
+// Trend + RK sub-step kernel with its stencil inputs staged in shared memory by
+// the tensor memory accelerator (TMA), and the step1 that goes with it: a
+// hierarchy's finest level, and the single-level stepper with too few layers for its
+// pipelined kernels (trisk_pipe.cuh; the rule is flux_kernels in wt_api.cu).
 //
 // A block owns a TT_X x TT_Y tile of padded nodes of one lozenge and one layer.
 // One thread issues S_NPLANE tiled bulk-tensor copies (cp.async.bulk.tensor,
@@ -107,15 +108,17 @@ __device__ __forceinline__ void weights5_s(const double* __restrict__ S, int q, 
   w[0] = wgt[0]; w[1] = -wgt[1]; w[2] = wgt[2]; w[3] = -wgt[3]; w[4] = wgt[4];
 }
 
-// Same trends and sub-step as k_trend_ml (scalar_trend, du_source/Qperp, du_grad,
-// RK_sub_step; src/ops.f90:739-901, src/time_integr.f90:206-225) at the finest level
-// of a hierarchy (src/multi_level.f90:5-188): trends only where mask_n >= TRSK, dmass and dTheta written on
+// Same trends and sub-step as k_trend (scalar_trend, du_source/Qperp, du_grad,
+// RK_sub_step; src/ops.f90:739-901, src/time_integr.f90:206-225).
+// MODE_ML is the trend of the finest level of a hierarchy (trisk_ml.cuh,
+// src/multi_level.f90:5-188): trends only where mask_n >= TRSK, dmass and dTheta written on
 // [0, n]^2, the velocity source on [0, n)^2, the sub-step on every padded node;
 // with a needed-node map, tiles with no needed node are left out before any
 // copy is issued and nodes that are not needed write nothing.
 // Block b: layer b % nz, then tile x, tile y, lozenge.  err receives 1 when a
 // block's copies did not complete within the wait limit; inject != 0 forces
 // that path (test only, see TMA_INJECT_TX).
+template <int MODE>
 __global__ void __launch_bounds__(TT_X * TT_Y, 3)
     k_trend_tma(LevelDev L, int nz, int nbx, int nby, TrendIO io, int* __restrict__ err, int inject,
                 const __grid_constant__ TrendMaps M) {
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(TT_X * TT_Y, 3)
   const int d = b / nby;
   const int x0 = bx * TT_X, y0 = by * TT_Y;
   const int tid = threadIdx.x;
-  if (io.need) {
+  if (MODE == MODE_ML && io.need) {
     const int pi = x0 + tid % TT_X, pj = y0 + tid / TT_X;
     int v = 0;
     if (pi < L.P && pj < L.P) v = io.need[__ldg(L.nsrc + (d * L.P + pj) * L.P + pi)];
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(TT_X * TT_Y, 3)
   const bool own = inside && i >= 0 && j >= 0 && i < n && j < n;
   const int64_t vo = 3 * ko + id;
   double bm = 0.0, bt = 0.0, bv0 = 0.0, bv1 = 0.0, bv2 = 0.0;
-  if (inside) {
+  if ((MODE == MODE_RK || MODE == MODE_ML) && inside) {
     bm = io.base_m[ko + id];
     bt = io.base_t[ko + id];
     bv0 = io.base_v[vo];
@@ -223,8 +226,11 @@ __global__ void __launch_bounds__(TT_X * TT_Y, 3)
   __syncthreads();
 
   if (!inside) return;
-  if (io.need && !io.need[__ldg(L.nsrc + id)]) return;
-  const bool on = io.mask_n[id] >= 2;  // TRSK
+  bool on = true;
+  if (MODE == MODE_ML) {
+    if (io.need && !io.need[__ldg(L.nsrc + id)]) return;
+    on = io.mask_n[id] >= 2;  // TRSK
+  }
   const int q0 = (ty + 1) * TB_X + (tx + 2);
   constexpr int oE = 1, oW = -1, oN = TB_X, oS = -TB_X, oNE = TB_X + 1, oSW = -TB_X - 1, oSE = 1 - TB_X,
                 oNW = TB_X - 1;
@@ -275,29 +281,37 @@ __global__ void __launch_bounds__(TT_X * TT_Y, 3)
     dv2 = s2 / lUP - gB2 - interp(th0, thN) * gE2;
   }
 #undef SM
-  if (scal) {
-    io.dm[ko + id] = dms;
-    io.dtt[ko + id] = dts;
+  if (MODE == MODE_ML) {
+    if (scal) {
+      io.dm[ko + id] = dms;
+      io.dtt[ko + id] = dts;
+    }
+    if (own) {
+      io.src[vo] = s0;
+      io.src[vo + NN] = s1;
+      io.src[vo + 2 * NN] = s2;
+    }
   }
-  if (own) {
-    io.src[vo] = s0;
-    io.src[vo + NN] = s1;
-    io.src[vo + 2 * NN] = s2;
-  }
-  if (io.grad) {  // u_star
+  if (MODE == MODE_ML && io.grad) {  // u_star
     const double h = io.h, t1 = io.th1;
     io.dst_m[ko + id] = bm + h * dms;
     io.dst_t[ko + id] = bt + h * dts;
     io.dst_v[vo] = bv0 + h * (dv0 + t1 * io.grad[id]);
     io.dst_v[vo + NN] = bv1 + h * (dv1 + t1 * io.grad[NN + id]);
     io.dst_v[vo + 2 * NN] = bv2 + h * (dv2 + t1 * io.grad[2 * NN + id]);
-  } else {
+  } else if (MODE == MODE_RK || MODE == MODE_ML) {
     const double h = io.h;
     io.dst_m[ko + id] = bm + h * dms;
     io.dst_t[ko + id] = bt + h * dts;
     io.dst_v[vo] = bv0 + h * dv0;
     io.dst_v[vo + NN] = bv1 + h * dv1;
     io.dst_v[vo + 2 * NN] = bv2 + h * dv2;
+  } else {
+    io.dm[ko + id] = dms;
+    io.dtt[ko + id] = dts;
+    io.dv[vo] = dv0;
+    io.dv[vo + NN] = dv1;
+    io.dv[vo + 2 * NN] = dv2;
   }
 }
 

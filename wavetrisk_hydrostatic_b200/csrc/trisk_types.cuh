@@ -75,12 +75,12 @@ struct TrendIO {
   const double* base_m; const double* base_t; const double* base_v;
   double* dst_m; double* dst_t; double* dst_v;
   double h;
-  // MODE_TREND (and dm, dtt in k_trend_tma)
+  // MODE_TREND (and dm, dtt in MODE_ML)
   double* dm; double* dtt; double* dv;
-  // k_trend_tma: the level's node masks, the velocity source it writes on
+  // MODE_ML: the level's node masks, the velocity source it writes on
   // [0, n)^2, and the needed-node map (need_map.cuh) or null
   const int* mask_n; double* src; const unsigned char* need;
-  // k_trend_tma with u_star: velocity sub-step base + h * (trend + th1 * grad)
+  // MODE_ML with u_star: velocity sub-step base + h * (trend + th1 * grad)
   const double* grad; double th1;
 };
 

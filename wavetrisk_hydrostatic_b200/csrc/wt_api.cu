@@ -100,36 +100,39 @@ int wt_make_step1_maps(wt_handle* h, const double* m, const double* t, const dou
   return step1_maps(h, m, t, v, out) ? WT_OK : WT_ERR_CUDA;
 }
 
+static bool trend_maps(wt_handle* h, const double* hfm, const double* hft, const double* qe,
+                       const double* theta, const double* bern, const double* phik, TrendMaps* M) {
+  const DevLevel& D = h->top();
+  const int nz = h->nz;
+  return top_map(h, &M->hfm, hfm, 3 * nz) && top_map(h, &M->hft, hft, 3 * nz) && top_map(h, &M->qe, qe, 3 * nz) &&
+         top_map(h, &M->theta, theta, nz) && top_map(h, &M->bern, bern, nz) && top_map(h, &M->phik, phik, nz) &&
+         top_map(h, &M->part, D.part, 6) && top_map(h, &M->hinv, D.hex_inv, 1);
+}
+
 int wt_make_trend_maps(wt_handle* h, const double* hfm, const double* hft, const double* qe, const double* theta,
                        const double* bern, const double* phik, wtk::TrendMaps* M) {
   if (h->trend_variant != 0) return WT_ERR_STATE;
-  const DevLevel& D = h->top();
-  const int nz = h->nz;
-  const bool ok = top_map(h, &M->hfm, hfm, 3 * nz) && top_map(h, &M->hft, hft, 3 * nz) &&
-                  top_map(h, &M->qe, qe, 3 * nz) && top_map(h, &M->theta, theta, nz) &&
-                  top_map(h, &M->bern, bern, nz) && top_map(h, &M->phik, phik, nz) &&
-                  top_map(h, &M->part, D.part, 6) && top_map(h, &M->hinv, D.hex_inv, 1);
-  return ok ? WT_OK : WT_ERR_CUDA;
+  return trend_maps(h, hfm, hft, qe, theta, bern, phik, M) ? WT_OK : WT_ERR_CUDA;
 }
 
 // Tensor maps and launch limits of the TMA-staged kernels on the top level.
 static int make_trend_maps(wt_handle* h) {
-  const DevLevel& D = h->top();
   const int nz = h->nz;
+  bool ok = trend_maps(h, h->hfm, h->hft, h->qe, h->theta, h->bern, h->phik, &h->maps);
   auto mk = [&](CUtensorMap* m, const double* base, int planes) {
     return top_map(h, m, base, planes, PBX, PipeTile::BY);
   };
   TrendMapsD& M = h->pmaps;
-  bool ok = step1_maps(h, h->mass, h->temp, h->velo, &h->s1maps) && mk(&M.hfm, h->hfm, 3 * nz) &&
-            mk(&M.hft, h->hft, 3 * nz) && mk(&M.qe, h->qe, 3 * nz) && mk(&M.theta, h->theta, nz) &&
-            mk(&M.bern, h->bern, nz) && mk(&M.phik, h->phik, nz);
+  ok = ok && mk(&M.hfm, h->hfm, 3 * nz) && mk(&M.hft, h->hft, 3 * nz) && mk(&M.qe, h->qe, 3 * nz) &&
+       mk(&M.theta, h->theta, nz) && mk(&M.bern, h->bern, nz) && mk(&M.phik, h->phik, nz);
   double* SM[3] = {h->mass, h->m1, h->m2};
   double* ST[3] = {h->temp, h->t1, h->t2};
   double* SV[3] = {h->velo, h->v1, h->v2};
   for (int b = 0; b < 3 && ok; ++b) {
     PipeStateMaps& S = h->p1maps[b];
-    ok = mk(&S.mass, SM[b], nz) && mk(&S.temp, ST[b], nz) && mk(&S.velo, SV[b], 3 * nz) && mk(&S.mean_m, h->mean_m, nz) &&
-         mk(&S.mean_t, h->mean_t, nz) && mk(&S.phik, h->phik, nz) && mk(&S.pterm, h->pterm, nz);
+    ok = step1_maps(h, SM[b], ST[b], SV[b], &h->s1maps[b]) && mk(&S.mass, SM[b], nz) && mk(&S.temp, ST[b], nz) &&
+         mk(&S.velo, SV[b], 3 * nz) && mk(&S.mean_m, h->mean_m, nz) && mk(&S.mean_t, h->mean_t, nz) &&
+         mk(&S.phik, h->phik, nz) && mk(&S.pterm, h->pterm, nz);
   }
   if (!ok) {
     std::fprintf(stderr, "wavetrisk_gpu: tensor map encoding failed\n");
@@ -140,7 +143,9 @@ static int make_trend_maps(wt_handle* h) {
   CK(cudaDeviceGetAttribute(&h->pipe_slots, cudaDevAttrMultiProcessorCount, dev));  // one block a SM
   const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
   CK(cudaFuncSetAttribute(k_step1_tma, smem, STEP1_TMA_SMEM));
-  CK(cudaFuncSetAttribute(k_trend_tma, smem, TREND_TMA_SMEM));
+  CK(cudaFuncSetAttribute(k_trend_tma<MODE_RK>, smem, TREND_TMA_SMEM));
+  CK(cudaFuncSetAttribute(k_trend_tma<MODE_TREND>, smem, TREND_TMA_SMEM));
+  CK(cudaFuncSetAttribute(k_trend_tma<MODE_ML>, smem, TREND_TMA_SMEM));
   CK(cudaFuncSetAttribute(k_step1_pipe<double>, smem, Step1Pipe<double>::SMEM));
   CK(cudaFuncSetAttribute(k_step1_pipe<float>, smem, Step1Pipe<float>::SMEM));
   CK(cudaFuncSetAttribute(k_trend_pipe<double, MODE_RK>, smem, TrendPipe<double, MODE_RK>::SMEM));
@@ -475,6 +480,28 @@ struct KTimer {
 #define TE(id) \
   if (tm) tm->end(id)
 
+// The kernels of one trend evaluation.  The pipelined tiles keep a tile's geometry over
+// a group of layers, which one or two layers do not pay back; measured, us a step
+// (pipelined tiles / tiles of one layer / L1 kernels):
+//   FP64, 1 layer:  J6 107 / 70 / 86,   J7 179 / 129 / 158,  J8 522 / 402 / 678
+//   FP64, 2 layers: J6 117 / 108 / 95,  J7 247 / 229 / 324,  J8 707 / 685 / 1244
+//   FP64, 3 layers: J6 125 / 127 / 149, J7 292 / 339 / 486,  J8 889 / 982 / 1806
+//   FP32, 1 layer:  J6 109 / - / 84,    J7 182 / - / 154,    J8 539 / - / 597
+//   FP32, 2 layers: J6 116 / - / 94,    J7 232 / - / 268,    J8 689 / - / 1077
+//   FP32, 3 layers: J6 125 / - / 128,   J7 279 / - / 407
+// FP64 takes the pipelined tiles from three layers up; FP32 fluxes, whose L1 kernels are
+// further off, also below that where the blocks have eight rounds of tiles or more
+// (J7: 5.5 rounds with one layer, 10.9 with two).
+enum FluxKernels { FLUX_L1, FLUX_TILES, FLUX_PIPE };
+static FluxKernels flux_kernels(wt_handle* h) {
+  const int P = h->top().P;
+  const int64_t tiles = (int64_t)10 * ((P + PX - 1) / PX) * ((P + PY - 1) / PY);
+  if (h->trend_variant != 0) return FLUX_L1;
+  if (h->flux_bits == 32)
+    return f32_staged(h) && (h->nz >= 3 || tiles * h->nz >= 8 * (int64_t)h->pipe_slots) ? FLUX_PIPE : FLUX_L1;
+  return h->nz >= 3 ? FLUX_PIPE : FLUX_TILES;
+}
+
 // Launch sequence of one trend evaluation of state (m, t, v); MODE_RK writes
 // dst = base + hstep * trend, MODE_TREND writes the trends into h->dm/dt/dv.
 static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode, const double* bm, const double* bt,
@@ -488,7 +515,8 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   // block b: layer b % nz of node chunk b / nz (layer_node in trisk_kernels.cuh)
   const unsigned chunks = blocks_for(D.NN, NODE_TILE);
   const bool f32 = h->flux_bits == 32;
-  const bool pipe = f32 ? f32_staged(h) : h->trend_variant == 0;  // pipelined tiles (trisk_pipe.cuh)
+  const FluxKernels kernels = flux_kernels(h);
+  const bool pipe = kernels == FLUX_PIPE;
   const unsigned cb = blocks_for(D.NN, COL_TILE);
   const unsigned gb = pipe ? ghost_blocks(h->ghosts.n_nodes + h->ghosts.n_edges, nz, COL_TILE) : 0;
   TB(1);
@@ -501,8 +529,8 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   double* dm = mode == MODE_RK ? om : h->dm;
   double* dt = mode == MODE_RK ? ot : h->dt;
   double* dv = mode == MODE_RK ? ov : h->dv;
+  const int sb = (m == h->m1) ? 1 : (m == h->m2) ? 2 : 0;  // which state buffer the stage reads
   if (pipe) {
-    const int sb = (m == h->m1) ? 1 : (m == h->m2) ? 2 : 0;  // which state buffer the stage reads
     auto grid = [&](int nodes) {
       PipeGrid G{(nodes + PX - 1) / PX, (nodes + PY - 1) / PY, 0, 0, 0};
       const int tiles = G.nbx * G.nby * 10;
@@ -565,14 +593,25 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   }
   Step1Out so{h->qe, h->hfm, h->hft, h->bern, h->theta};
   TB(2);
-  k_step1<<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, m, t, v, h->mean_m, h->mean_t, h->phik, h->pterm, so, nullptr);
+  if (kernels == FLUX_TILES) {
+    const int nbx = (D.n + 1 + TT_X - 1) / TT_X, nby = (D.n + 1 + TT_Y - 1) / TT_Y;
+    k_step1_tma<<<(unsigned)(nz * nbx * nby * 10), TT_X * TT_Y, STEP1_TMA_SMEM, s>>>(
+        L, nz, nbx, nby, m, t, v, h->mean_m, h->phik, h->pterm, so, h->dflag, h->tma_inject, h->s1maps[sb], nullptr);
+  } else {
+    k_step1<<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, m, t, v, h->mean_m, h->mean_t, h->phik, h->pterm, so, nullptr);
+  }
   TE(2);
   TrendIO io{};
   io.theta = h->theta; io.qe = h->qe; io.hfm = h->hfm; io.hft = h->hft; io.bern = h->bern; io.phik = h->phik;
   io.base_m = bm; io.base_t = bt; io.base_v = bv; io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
   io.dm = h->dm; io.dtt = h->dt; io.dv = h->dv;
   TB(5);
-  if (mode == MODE_RK)
+  if (kernels == FLUX_TILES) {
+    const int nbx = (D.P + TT_X - 1) / TT_X, nby = (D.P + TT_Y - 1) / TT_Y;
+    const auto k = mode == MODE_RK ? k_trend_tma<MODE_RK> : k_trend_tma<MODE_TREND>;
+    k<<<(unsigned)(nz * nbx * nby * 10), TT_X * TT_Y, TREND_TMA_SMEM, s>>>(L, nz, nbx, nby, io, h->dflag, h->tma_inject,
+                                                                           h->maps);
+  } else if (mode == MODE_RK)
     k_trend<MODE_RK><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
   else
     k_trend<MODE_TREND><<<chunks * nz, NODE_TILE, 0, s>>>(L, nz, io);
@@ -581,14 +620,14 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   return WT_OK;
 }
 
-// k_trend_tma on the top level: the multi-level trend of the finest
+// k_trend_tma<MODE_ML> on the top level: the multi-level trend of the finest
 // level with the RK sub-step, its inputs read through the maps M.
 int wt_level_trend_ml_tma(wt_handle* h, const wtk::TrendIO& io, const wtk::TrendMaps& M, cudaStream_t stream) {
   const DevLevel& D = h->top();
   const int nz = h->nz;
   const int nbx = (D.P + TT_X - 1) / TT_X, nby = (D.P + TT_Y - 1) / TT_Y;
   const unsigned nblk = (unsigned)(nz * nbx * nby * 10);
-  k_trend_tma<<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, stream ? stream : h->stream>>>(D.view(), nz, nbx, nby, io,
+  k_trend_tma<MODE_ML><<<nblk, TT_X * TT_Y, TREND_TMA_SMEM, stream ? stream : h->stream>>>(D.view(), nz, nbx, nby, io,
                                                                                            h->dflag, h->tma_inject, M);
   CK(cudaGetLastError());
   return WT_OK;

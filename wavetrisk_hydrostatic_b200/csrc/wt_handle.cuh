@@ -51,7 +51,10 @@ struct wt_handle {
   double *dm = nullptr, *dt = nullptr, *dv = nullptr;
   double *qe = nullptr, *hfm = nullptr, *hft = nullptr, *bern = nullptr, *phik = nullptr, *pterm = nullptr;
   double* theta = nullptr;  // Theta/rho of the stage state, written by k_step1
-  wtk::Step1Maps s1maps{};  // k_step1_tma's input maps of the state (mass, temp, velo) (hierarchy)
+  // the TMA-staged kernels of trisk_tma.cuh: trend inputs, step1 inputs of the state buffers (mass, temp, velo),
+  // (m1, t1, v1), (m2, t2, v2)
+  wtk::TrendMaps maps{};
+  wtk::Step1Maps s1maps[3]{};
   // the single-level stepper's pipelined kernels (trisk_pipe.cuh): step1 inputs of the state buffers (mass, temp,
   // velo), (m1, t1, v1), (m2, t2, v2), trend inputs, geometry, and the blocks the device keeps resident
   wtk::GhostLists ghosts{};
@@ -102,7 +105,7 @@ void wt_trend_ml_release(wt_handle* h);
 // level's geometry), for k_trend_tma; WT_ERR_STATE unless the TMA variant is on.
 int wt_make_trend_maps(wt_handle* h, const double* hfm, const double* hft, const double* qe, const double* theta,
                        const double* bern, const double* phik, wtk::TrendMaps* M);
-// k_trend_tma on the top level (stream: the handle's when null).
+// k_trend_tma<MODE_ML> on the top level (stream: the handle's when null).
 int wt_level_trend_ml_tma(wt_handle* h, const wtk::TrendIO& io, const wtk::TrendMaps& M, cudaStream_t stream);
 int wt_level_step1(wt_handle* h, int level, const double* m, const double* t, const double* v, const double* mean_m,
                    const double* mean_t, double* phik, double* pterm, double* qe, double* hfm, double* hft,

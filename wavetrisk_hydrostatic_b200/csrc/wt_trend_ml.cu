@@ -217,7 +217,7 @@ int trend_multi(wt_handle* h, const States& S, PhaseTimer* tm = nullptr, const S
     const wtk::Step1Maps* maps = nullptr;
     if (l == h->level_end && h->trend_variant == 0) {
       if (S.m[q] == h->mass && S.t[q] == h->temp && S.v[q] == h->velo) {
-        maps = &h->s1maps;
+        maps = &h->s1maps[0];
       } else if (S.m[q] == V.m1 && S.t[q] == V.t1 && S.v[q] == V.v1) {
         if (!M->q1maps_ok) {
           if (int rc = wt_make_step1_maps(h, V.m1, V.t1, V.v1, &M->q1maps)) return rc;
