@@ -16,6 +16,7 @@
 // to the CPU restatement.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "trisk_read.cuh"
 #include "trisk_types.cuh"
@@ -51,16 +52,20 @@ __global__ void k_halo_state(int nz, int64_t NN, const int2* __restrict__ hn, in
 // node (i, j) in [0, n]^2 of every lozenge.  Writes the layer geopotential
 // Phi_k = interp(geopot, geopot_lower) and press/(rho0*phi).
 constexpr int COL_TILE = 64;  // threads of a column block
+template <int COL_B>
+constexpr int COL_MINB = COL_B == 8 ? 12 : 20;  // resident blocks: registers for the layers read at once
+template <int COL_B>
 __device__ __forceinline__ void column_node(const LevelDev& L, const Phys& ph, int nz, const double* __restrict__ mass,
                                             const double* __restrict__ temp, const double* __restrict__ mean_m,
                                             const double* __restrict__ mean_t, double* __restrict__ phik,
                                             double* __restrict__ pterm, int id, int i, int j) {
   // The two recursions are serial in the layer but their loads are not: COL_B
-  // layers' values are read before they are summed.  Both quotients share the
+  // layers' values are read before they are summed (column_batch chooses COL_B; past
+  // the last layer its values are read again, since a load under a condition waits
+  // for the one before: J5 x 8 100 -> 113 us a step).  Both quotients share the
   // divisor rho0.  The second pass reads the layers again, from L2: kept in shared
   // memory (16 KB a block at 16 layers) they cost more in resident blocks than they
   // save (J7 x 16 with the ghost copies: 44 us against 36, and 34 with COL_B = 8 for 4).
-  constexpr int COL_B = 8;
   const int src = (i < L.n && j < L.n) ? id : L.nsrc[id];
   const double rho0 = ph.ref_density * 1.0, y0 = 1.0 / rho0;
   double rho_dz[COL_B], rho_dz_theta[COL_B];
@@ -98,9 +103,19 @@ __device__ __forceinline__ void column_node(const LevelDev& L, const Phys& ph, i
   }
 }
 
+// Calls f with the layers a column reads at once: 8, and no more than there are of one
+// or two.  Host code.
+template <class F>
+inline void column_batch(int nz, F f) {
+  if (nz == 1) f(std::integral_constant<int, 1>{});
+  else if (nz == 2) f(std::integral_constant<int, 2>{});
+  else f(std::integral_constant<int, 8>{});
+}
+
 // A column is one thread's serial work: small blocks spread a level's few columns
 // over the SMs.
-__global__ void __launch_bounds__(COL_TILE, 12) k_column(LevelDev L, Phys ph, int nz, const double* __restrict__ mass,
+template <int COL_B>
+__global__ void __launch_bounds__(COL_TILE, COL_MINB<COL_B>) k_column(LevelDev L, Phys ph, int nz, const double* __restrict__ mass,
                                                      const double* __restrict__ temp, const double* __restrict__ mean_m,
                                                      const double* __restrict__ mean_t, double* __restrict__ phik,
                                                      double* __restrict__ pterm,
@@ -113,11 +128,12 @@ __global__ void __launch_bounds__(COL_TILE, 12) k_column(LevelDev L, Phys ph, in
   node_ij(L, id, i, j);
   if (i < 0 || j < 0 || i > L.n || j > L.n) return;
   if (need && !need[__ldg(L.nsrc + id)]) return;
-  column_node(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
+  column_node<COL_B>(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
 }
 
 // The same over a work list (persistent blocks).
-__global__ void __launch_bounds__(COL_TILE, 12) k_column_list(LevelDev L, Phys ph, int nz, const double* __restrict__ mass,
+template <int COL_B>
+__global__ void __launch_bounds__(COL_TILE, COL_MINB<COL_B>) k_column_list(LevelDev L, Phys ph, int nz, const double* __restrict__ mass,
                                                           const double* __restrict__ temp,
                                                           const double* __restrict__ mean_m,
                                                           const double* __restrict__ mean_t, double* __restrict__ phik,
@@ -126,7 +142,7 @@ __global__ void __launch_bounds__(COL_TILE, 12) k_column_list(LevelDev L, Phys p
   for (int64_t w = blockIdx.x; w < list_items<COL_TILE>(cnt, 1); w += gridDim.x) {
     int k, id, i, j;
     if (!list_entry<COL_TILE>(L, 1, W, cnt, w, k, id, i, j) || i < 0 || j < 0 || i > L.n || j > L.n) continue;
-    column_node(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
+    column_node<COL_B>(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
   }
 }
 

@@ -657,7 +657,8 @@ __device__ __forceinline__ void ghost_copy(int2 e, int k0, int nz, int64_t strid
 
 // The column pass, and in the blocks before `ghosts` the ghost copy of the state:
 // columns read owned slots only, so the two may run side by side.
-__global__ void __launch_bounds__(COL_TILE, 12) k_column_halo(LevelDev L, Phys ph, int nz, unsigned ghosts, GhostLists H,
+template <int COL_B>
+__global__ void __launch_bounds__(COL_TILE, COL_MINB<COL_B>) k_column_halo(LevelDev L, Phys ph, int nz, unsigned ghosts, GhostLists H,
                                                           double* mass, double* temp, double* velo,
                                                           const double* __restrict__ mean_m,
                                                           const double* __restrict__ mean_t, double* __restrict__ phik,
@@ -668,7 +669,7 @@ __global__ void __launch_bounds__(COL_TILE, 12) k_column_halo(LevelDev L, Phys p
     int i, j;
     node_ij(L, id, i, j);
     if (i < 0 || j < 0 || i > L.n || j > L.n) return;
-    column_node(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
+    column_node<COL_B>(L, ph, nz, mass, temp, mean_m, mean_t, phik, pterm, id, i, j);
     return;
   }
   const int t = blockIdx.x * COL_TILE + threadIdx.x, per = H.n_nodes + H.n_edges;

@@ -520,11 +520,13 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   const unsigned cb = blocks_for(D.NN, COL_TILE);
   const unsigned gb = pipe ? ghost_blocks(h->ghosts.n_nodes + h->ghosts.n_edges, nz, COL_TILE) : 0;
   TB(1);
-  if (pipe)
-    k_column_halo<<<cb + gb, COL_TILE, 0, s>>>(L, h->ph, nz, gb, h->ghosts, m, t, v, h->mean_m, h->mean_t,
-                                                              h->phik, h->pterm);
-  else
-    k_column<<<cb, COL_TILE, 0, s>>>(L, h->ph, nz, m, t, h->mean_m, h->mean_t, h->phik, h->pterm, nullptr);
+  column_batch(nz, [&](auto B) {
+    if (pipe)
+      k_column_halo<B.value><<<cb + gb, COL_TILE, 0, s>>>(L, h->ph, nz, gb, h->ghosts, m, t, v, h->mean_m, h->mean_t,
+                                                          h->phik, h->pterm);
+    else
+      k_column<B.value><<<cb, COL_TILE, 0, s>>>(L, h->ph, nz, m, t, h->mean_m, h->mean_t, h->phik, h->pterm, nullptr);
+  });
   TE(1);
   double* dm = mode == MODE_RK ? om : h->dm;
   double* dt = mode == MODE_RK ? ot : h->dt;
@@ -644,14 +646,19 @@ int wt_level_step1(wt_handle* h, int level, const double* m, const double* t, co
   Step1Out so{qe, hfm, hft, bern, theta};
   const unsigned chunks = blocks_for(D.NN, NODE_TILE);
   if (list && list->ids) {  // the needed slots only, persistent blocks over the level's work list
-    k_column_list<<<persistent_grid(k_column_list, blocks_for(D.NN, COL_TILE), COL_TILE), COL_TILE, 0, s>>>(
-        L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, *list);
+    column_batch(nz, [&](auto B) {
+      k_column_list<B.value><<<persistent_grid(k_column_list<B.value>, blocks_for(D.NN, COL_TILE), COL_TILE), COL_TILE,
+                               0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, *list);
+    });
     k_step1_list<<<persistent_grid(k_step1_list, chunks * nz), NODE_TILE, 0, s>>>(L, nz, m, t, v, mean_m, mean_t,
                                                                                   phik, pterm, so, *list);
     CK(cudaGetLastError());
     return WT_OK;
   }
-  k_column<<<blocks_for(D.NN, COL_TILE), COL_TILE, 0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm, need);
+  column_batch(nz, [&](auto B) {
+    k_column<B.value><<<blocks_for(D.NN, COL_TILE), COL_TILE, 0, s>>>(L, h->ph, nz, m, t, mean_m, mean_t, phik, pterm,
+                                                                      need);
+  });
   if (maps && level == h->level_end && h->trend_variant == 0) {
     const int nbx = (D.n + 1 + TT_X - 1) / TT_X, nby = (D.n + 1 + TT_Y - 1) / TT_Y;
     const unsigned nblk = (unsigned)(nz * nbx * nby * 10);
