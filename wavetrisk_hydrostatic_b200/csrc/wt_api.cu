@@ -483,12 +483,12 @@ struct KTimer {
 // The kernels of one trend evaluation.  The pipelined tiles keep a tile's geometry over
 // a group of layers, which one or two layers do not pay back; measured, us a step
 // (pipelined tiles / tiles of one layer / L1 kernels):
-//   FP64, 1 layer:  J6 107 / 70 / 86,   J7 179 / 129 / 158,  J8 522 / 402 / 678
-//   FP64, 2 layers: J6 117 / 108 / 95,  J7 247 / 229 / 324,  J8 707 / 685 / 1244
-//   FP64, 3 layers: J6 125 / 127 / 149, J7 292 / 339 / 486,  J8 889 / 982 / 1806
-//   FP32, 1 layer:  J6 109 / - / 84,    J7 182 / - / 154,    J8 539 / - / 597
-//   FP32, 2 layers: J6 116 / - / 94,    J7 232 / - / 268,    J8 689 / - / 1077
-//   FP32, 3 layers: J6 125 / - / 128,   J7 279 / - / 407
+//   FP64, 1 layer:  J6 102 / 70 / 84,   J7 164 / 124 / 152,  J8 476 / 391 / 662,  J9 1528 / 1249
+//   FP64, 2 layers: J6 113 / 107 / 92,  J7 231 / 222 / 308,  J8 664 / 670 / 1217, J9 2411 / 2241
+//   FP64, 3 layers: J6 125 / 126 / 145, J7 288 / 337 / 477,  J8 880 / 984 / 1777, J9 3171 / 3371
+//   FP32, 1 layer:  J6 105 / - / 83,    J7 166 / - / 150,    J8 491 / - / 587,    J9 1570 / - / 2063
+//   FP32, 2 layers: J6 113 / - / 92,    J7 220 / - / 263,    J8 650 / - / 1061,   J9 2262 / - / 3813
+//   FP32, 3 layers: J6 125 / - / 131,   J7 276 / - / 404,    J8 838 / - / 1573,   J9 2972 / - / 5649
 // FP64 takes the pipelined tiles from three layers up; FP32 fluxes, whose L1 kernels are
 // further off, also below that where the blocks have eight rounds of tiles or more
 // (J7: 5.5 rounds with one layer, 10.9 with two).
