@@ -1020,10 +1020,12 @@ int restrict_flux(wt_handle* h, int level, double* par0, double* par1, const dou
   if (!V.rf_pi) return WT_ERR_ARG;
   const int m = h->at(level).n;
   const int64_t ne = (int64_t)3 * 10 * m * m;
-  const dim3 blk(32, 2 * std::min(nz, 8));
+  // a lone layer has two warps stage its plan
+  const dim3 blk(32, (par1 ? 2 : 1) * std::min(nz, 8) + (!par1 && nz == 1));
   const ParentList PL = wt_level_plist(h, level);
   const unsigned dense = (unsigned)((ne + 31) / 32);
-  k_restr_flux3<<<PL.ids ? pgrid(k_restr_flux3, (int)(blk.x * blk.y), dense) : dense, blk, 0, h->stream>>>(
+  const auto k = par1 ? k_restr_flux3<2> : k_restr_flux3<1>;
+  k<<<PL.ids ? pgrid(k, (int)(blk.x * blk.y), dense) : dense, blk, 0, h->stream>>>(
       view(h, level), m, nz, V.rf_pi, V.rf_pd, par0, par1, chd0, chd1, dsc0, dsc1, (int)h->at(level + 1).NN, PL);
   CKW(cudaGetLastError());
   return WT_OK;
