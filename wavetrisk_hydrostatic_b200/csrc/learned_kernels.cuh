@@ -622,119 +622,70 @@ __global__ void __launch_bounds__(256) k_lp_wgrad_out(int ns, const int* __restr
 }
 
 // Weight gradient of the 2 -> 32 layer: dW[t][ci][co] = sum_s dz(s)[co]
-// x(tap_t(s))[ci].  A warp takes a node, a lane one output channel; the 14 taps'
-// inputs are warp-uniform reads beside the node's coalesced dz row.
-__global__ void __launch_bounds__(256) k_lp_wgrad_in(int ns, const int* __restrict__ tap, const float2* __restrict__ x,
+// x(tap_t(s))[ci].  A block stages kChunk nodes' 14 tap inputs and dz rows in shared
+// memory; a thread owns up to two of the 448 entries, sums them over the block's
+// chunks and adds them once to the global gradient.  J7 45 us, J8 160; a node a warp
+// with an output channel a lane, whose tap reads hang on one another, takes 82 and 308.
+__global__ void __launch_bounds__(256) k_lp_wgrad_in(int ns, const int* __restrict__ tap, const float* __restrict__ x,
                                                      const float* __restrict__ dz, float* __restrict__ dW) {
-  __shared__ float sh[kTaps * kIn * kC];
-  const int lane = threadIdx.x & 31;
-  float a0[kTaps], a1[kTaps];
+  constexpr int K = kTaps * kIn, NE = K * kC, PER = (NE + 255) / 256;
+  __shared__ float A[kChunk][K];
+  __shared__ float G[kChunk][kC];
+  float acc[PER];
 #pragma unroll
-  for (int t = 0; t < kTaps; ++t) a0[t] = a1[t] = 0.0f;
-  const int stride = gridDim.x * 8;
-#pragma unroll 2
-  for (int s = blockIdx.x * 8 + (threadIdx.x >> 5); s < ns; s += stride) {
-    const float g = dz[(int64_t)s * kC + lane];
-#pragma unroll
-    for (int t = 0; t < kTaps; ++t) {
-      const int u = tap[t * ns + s];
-      const float2 v = u >= 0 ? x[u] : make_float2(0.0f, 0.0f);
-      a0[t] = fmaf(v.x, g, a0[t]);
-      a1[t] = fmaf(v.y, g, a1[t]);
-    }
-  }
-  for (int q = threadIdx.x; q < kTaps * kIn * kC; q += 256) sh[q] = 0.0f;
-  __syncthreads();
-#pragma unroll
-  for (int t = 0; t < kTaps; ++t) {
-    atomicAdd(&sh[(t * kIn) * kC + lane], a0[t]);
-    atomicAdd(&sh[(t * kIn + 1) * kC + lane], a1[t]);
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < kTaps * kIn * kC; q += 256) atomicAdd(&dW[q], sh[q]);
-}
-
-// Input gradient of the 32 -> 32 layer for the nodes whose inverse taps hold at
-// most one entry a tap, itap[t][u] = s with tap_t(s) = u (or -1): 256 nodes x 32
-// channels a block, 8 x 8 a thread, tap by tap through shared memory (the tap's
-// gathered dz rows, transposed, and its weights).  The entries are added in the
-// order of the list form, which takes the few other nodes (irr).
-constexpr int kIgNodes = 256, kIgPitch = kIgNodes + 1;
-__global__ void __launch_bounds__(128) k_lp_igrad32(int ns, const int* __restrict__ itap, const float* __restrict__ W,
-                                                    const float* __restrict__ dz, const uint4* __restrict__ h,
-                                                    float slope, float* __restrict__ dzin) {
-  __shared__ float A[kC][kIgPitch];
-  __shared__ __align__(16) float Wt[kC][kC];  // [co][ci]
-  const int tid = threadIdx.x, cg = tid & 3, ng = tid >> 2, u0 = blockIdx.x * kIgNodes;
-  unsigned long long acc[8][4];
-#pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
-  for (int t = 0; t < kTaps; ++t) {
+  for (int r = 0; r < PER; ++r) acc[r] = 0.0f;
+  const int nchunk = (ns + kChunk - 1) / kChunk;
+  for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
+    const int s0 = c * kChunk;
     __syncthreads();
-#pragma unroll 4
-    for (int q = tid; q < kIgNodes * 8; q += 128) {
-      const int nl = q >> 3, c4 = q & 7, u = u0 + nl;
-      const int s = u < ns ? itap[t * ns + u] : -1;
-      const float4 g = s >= 0 ? reinterpret_cast<const float4*>(dz)[(int64_t)s * 8 + c4] : make_float4(0.f, 0.f, 0.f, 0.f);
-      A[4 * c4][nl] = g.x;
-      A[4 * c4 + 1][nl] = g.y;
-      A[4 * c4 + 2][nl] = g.z;
-      A[4 * c4 + 3][nl] = g.w;
+    for (int q = threadIdx.x; q < kChunk * K; q += 256) {
+      const int nl = q / K, k = q % K, s = s0 + nl;
+      const int u = s < ns ? tap[(k / kIn) * ns + s] : -1;
+      A[nl][k] = u >= 0 ? x[(int64_t)u * kIn + k % kIn] : 0.0f;
     }
-    for (int q = tid; q < kC * kC; q += 128) Wt[q & 31][q >> 5] = W[(t * kC + (q >> 5)) * kC + (q & 31)];
+    for (int q = threadIdx.x; q < kChunk * kC; q += 256) {
+      const int s = s0 + q / kC;
+      G[q / kC][q % kC] = s < ns ? dz[(int64_t)s * kC + q % kC] : 0.0f;
+    }
     __syncthreads();
-#pragma unroll 4
-    for (int co = 0; co < kC; ++co) {
-      const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&Wt[co][4 * cg]);
-      const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(&Wt[co][16 + 4 * cg]);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float g = A[co][ng + 32 * q];
-        const unsigned long long gg = pack2(g, g);
-        acc[q][0] = ffma2(w0.x, gg, acc[q][0]);
-        acc[q][1] = ffma2(w0.y, gg, acc[q][1]);
-        acc[q][2] = ffma2(w1.x, gg, acc[q][2]);
-        acc[q][3] = ffma2(w1.y, gg, acc[q][3]);
+    for (int r = 0; r < PER; ++r) {
+      const int e = threadIdx.x + 256 * r;
+      if (e < NE) {
+        const int k = e / kC, co = e % kC;
+        float a = acc[r];
+#pragma unroll 8
+        for (int nl = 0; nl < kChunk; ++nl) a = fmaf(A[nl][k], G[nl][co], a);
+        acc[r] = a;
       }
     }
   }
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int u = u0 + ng + 32 * q;
-    if (u >= ns) continue;
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {  // channels 16 b + 4 cg .. + 3
-      const uint2 hv = reinterpret_cast<const uint2*>(h + 4 * (int64_t)u)[4 * b + cg];
-      float x, y, z, w;
-      unpack2(acc[q][2 * b], x, y);
-      unpack2(acc[q][2 * b + 1], z, w);
-      reinterpret_cast<float4*>(dzin)[(int64_t)u * 8 + 4 * b + cg] =
-          make_float4(x * lp_dact(__uint_as_float(hv.x << 16), slope), y * lp_dact(__uint_as_float(hv.x & 0xffff0000u), slope),
-                      z * lp_dact(__uint_as_float(hv.y << 16), slope), w * lp_dact(__uint_as_float(hv.y & 0xffff0000u), slope));
-    }
+  for (int r = 0; r < PER; ++r) {
+    const int e = threadIdx.x + 256 * r;
+    if (e < NE) atomicAdd(&dW[e], acc[r]);
   }
 }
 
 // Gradient at the input of one layer, gathered: for node u,
 //   dh(u)[ci] = sum over (s, t) with tap_t(s) = u of sum_co W[t][ci][co] dz(s)[co],
 // the pairs listed in the inverse tap table (inv[inv_ptr[u] .. inv_ptr[u+1]),
-// entry 8 s + t), then through the activation whose stored output is h(u); u runs
-// over all ns nodes or over the ns listed ones:
-// dzin(u)[ci] = dh(u)[ci] * act'(h(u)[ci]).  Node-major FP32 output.
+// entry 8 s + t), then through the activation whose stored output is h(u):
+// dzin(u)[ci] = dh(u)[ci] * act'(h(u)[ci]).  Node-major FP32 output.  A thread a node:
+// 32 -> 32 at J5 40 us, J7 136, J8 465.  Tap by tap through shared memory, 256 nodes x
+// 32 channels a block in 8 x 8 register tiles, with the nodes that one tap reaches twice
+// (poles, pentagons) in a launch of their own, it took 117, 216 and 526 us: gathers and
+// sums take turns there, and the second launch is 39 us at any level.
 template <int COUT>
-__global__ void __launch_bounds__(128) k_lp_igrad(int ns, const int* __restrict__ nodes,
-                                                  const int* __restrict__ inv_ptr, const int* __restrict__ inv,
-                                                  const float* __restrict__ W,
+__global__ void __launch_bounds__(128) k_lp_igrad(int ns, const int* __restrict__ inv_ptr,
+                                                  const int* __restrict__ inv, const float* __restrict__ W,
                                                   const float* __restrict__ dz, const __nv_bfloat16* __restrict__ h,
                                                   float slope, float* __restrict__ dzin) {
   __shared__ __align__(16) float sw[kTaps * kC * COUT];
   for (int q = threadIdx.x; q < kTaps * kC * COUT; q += blockDim.x) sw[q] = W[q];
   __syncthreads();
-  int u = blockIdx.x * blockDim.x + threadIdx.x;
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= ns) return;
-  if (nodes) u = nodes[u];
   float acc[kC];
 #pragma unroll
   for (int ci = 0; ci < kC; ++ci) acc[ci] = 0.0f;

@@ -25,9 +25,6 @@ struct LPNet {
   int* slot = nullptr;  // ns node slots of the level
   int* tap = nullptr;   // 7*ns compact tap indices
   int *inv_ptr = nullptr, *inv = nullptr;  // inverse taps: (s, t) with tap_t(s) = u, entry 8 s + t
-  int* itap = nullptr;                     // 7*ns: the s of tap t, or -1 (one of them where irr lists the node)
-  int* irr = nullptr;                      // nodes with two entries of one tap (poles, pentagons)
-  int nirr = 0;
   float* own = nullptr; // ns: 1 on owned nodes, 0 at the pole slots
   float *w = nullptr, *wr = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
   __nv_bfloat16* wpk = nullptr;  // W2 packed for the tensor cores
@@ -164,17 +161,6 @@ int lp_build(Ell& E, uint64_t seed) {
         if (u >= 0) inv[fill[u]++] = 8 * s + t;
       }
   }
-  std::vector<int> itap((size_t)kTaps * ns, -1), irr;
-  for (int u = 0; u < ns; ++u) {
-    bool twice = false;
-    for (int e = inv_ptr[u]; e < inv_ptr[u + 1]; ++e) {
-      int& x = itap[(size_t)(inv[e] & 7) * ns + u];
-      twice = twice || x >= 0;
-      x = inv[e] >> 3;
-    }
-    if (twice) irr.push_back(u);
-  }
-  N->nirr = (int)irr.size();
   auto& A = N->allocs;
   int rc = WT_OK;
   auto al = [&](auto** p, int64_t cnt) {
@@ -184,8 +170,6 @@ int lp_build(Ell& E, uint64_t seed) {
   al(&N->tap, (int64_t)kTaps * ns);
   al(&N->inv_ptr, ns + 1);
   al(&N->inv, std::max<int64_t>(1, (int64_t)inv.size()));
-  al(&N->itap, (int64_t)kTaps * ns);
-  al(&N->irr, (int64_t)irr.size());
   al(&N->own, ns);
   for (float** p : {&N->w, &N->wr, &N->g, &N->m, &N->v}) al(p, kLpParams);
   al(&N->wpk, (int64_t)kTaps * kC * kC);
@@ -210,8 +194,6 @@ int lp_build(Ell& E, uint64_t seed) {
     cudaMemcpy(N->tap, tap.data(), 4 * tap.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(N->own, own.data(), 4 * (size_t)ns, cudaMemcpyHostToDevice);
     cudaMemcpy(N->inv_ptr, inv_ptr.data(), 4 * (size_t)(ns + 1), cudaMemcpyHostToDevice);
-    cudaMemcpy(N->itap, itap.data(), 4 * itap.size(), cudaMemcpyHostToDevice);
-    if (!irr.empty()) cudaMemcpy(N->irr, irr.data(), 4 * irr.size(), cudaMemcpyHostToDevice);
     if (!inv.empty()) cudaMemcpy(N->inv, inv.data(), 4 * inv.size(), cudaMemcpyHostToDevice);
     // persistent CTAs of the tensor-core layer: as many as fit on the device at once
     int dev = 0, nsm = 0, per_sm = 0;
@@ -287,15 +269,14 @@ void lp_backward(Ell& E, LPNet& N, const double* e, const double* rs, double* lo
   cudaMemsetAsync(N.g, 0, 4 * kLpParams, st);
   const auto* h1 = reinterpret_cast<const __nv_bfloat16*>(N.h1);
   const auto* h2 = reinterpret_cast<const __nv_bfloat16*>(N.h2);
-  // persistent blocks: two a SM for the register-tiled kernel, eight for the row-by-row ones
-  const unsigned g32 = std::min<unsigned>((ns + kChunk - 1) / kChunk, 148 * 2), grow = std::min<unsigned>((ns + 15) / 16, 148 * 8);
+  // persistent blocks: two a SM for the register-tiled kernel, eight for the row-by-row one, four for the chunked one
+  const unsigned chunks = (ns + kChunk - 1) / kChunk, sms = (unsigned)E.sms;
+  const unsigned g32 = std::min(chunks, 2 * sms), grow = std::min<unsigned>((ns + 15) / 16, 8 * sms), gin = std::min(chunks, 4 * sms);
   k_lp_wgrad_out<<<grow, 256, 0, st>>>(ns, N.tap, reinterpret_cast<const unsigned*>(N.h2), N.dy, N.g + kW3);
-  k_lp_igrad<1><<<lpg(ns), LP_TPB, 0, st>>>(ns, nullptr, N.inv_ptr, N.inv, N.wr + kW3, N.dy, h2, N.slope, N.dz2);
+  k_lp_igrad<1><<<lpg(ns), LP_TPB, 0, st>>>(ns, N.inv_ptr, N.inv, N.wr + kW3, N.dy, h2, N.slope, N.dz2);
   k_lp_wgrad32<<<g32, 256, 0, st>>>(ns, N.tap, N.h1, N.dz2, N.g + kW2);
-  k_lp_igrad32<<<lpg(ns, kIgNodes), 128, 0, st>>>(ns, N.itap, N.wr + kW2, N.dz2, N.h1, N.slope, N.dz1);
-  if (N.nirr)
-    k_lp_igrad<kC><<<lpg(N.nirr), LP_TPB, 0, st>>>(N.nirr, N.irr, N.inv_ptr, N.inv, N.wr + kW2, N.dz2, h1, N.slope, N.dz1);
-  k_lp_wgrad_in<<<grow, 256, 0, st>>>(ns, N.tap, reinterpret_cast<const float2*>(N.x), N.dz1, N.g + kW1);
+  k_lp_igrad<kC><<<lpg(ns), LP_TPB, 0, st>>>(ns, N.inv_ptr, N.inv, N.wr + kW2, N.dz2, h1, N.slope, N.dz1);
+  k_lp_wgrad_in<<<gin, 256, 0, st>>>(ns, N.tap, N.x, N.dz1, N.g + kW1);
 }
 
 void lp_adam(Ell& E, LPNet& N, float lr) {
