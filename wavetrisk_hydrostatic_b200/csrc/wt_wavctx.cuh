@@ -105,6 +105,9 @@ struct WavCtx {
   int* plist = nullptr;
   int* pcount = nullptr;
   double* pack = nullptr;
+  // cal_lnorm's block partials and counts, blocks a level and result (wt_lnorm), allocated on first use
+  double *ln_part = nullptr, *ln_out = nullptr;
+  int *ln_cnt = nullptr, *ln_blocks = nullptr;
   template <class T>
   cudaError_t alloc(T** p, size_t count) {
     cudaError_t e = cudaMalloc(p, count * sizeof(T));
