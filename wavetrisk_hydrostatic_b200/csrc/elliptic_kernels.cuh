@@ -300,6 +300,9 @@ __device__ __forceinline__ double ell_finish(double v, int mode, const double* d
 // a reduction instead of two, and one fence and one ticket a resident block, not a
 // chunk (2580 at J8: k_ell_resid_norm 39 -> 35 us).
 constexpr int RED_PER_SM = 4;  // resident blocks of 256 threads
+// of a plain sum, whose 40 registers let J7's 651 chunks run in one round: wt_elliptic_l2
+// at J7 28 us a call with 4, 26 with 6; at J9 41 and 34
+constexpr int DOT_PER_SM = 6;
 template <class F>
 __device__ __forceinline__ void ell_reduce(int nodes, F value, double* partial, unsigned* ticket, double* out, int mode,
                                            const double* den) {
@@ -329,7 +332,7 @@ __device__ __forceinline__ void ell_reduce(int nodes, F value, double* partial, 
   }
 }
 
-__global__ void __launch_bounds__(256, RED_PER_SM)
+__global__ void __launch_bounds__(256, DOT_PER_SM)
     k_ell_dot(EllLev L, const double* __restrict__ a, const double* __restrict__ b, double* partial, unsigned* ticket,
               double* out, int mode, const double* den) {
   const int m = L.n + 1;

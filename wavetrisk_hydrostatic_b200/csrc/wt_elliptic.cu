@@ -288,13 +288,13 @@ void op(Ell& E, int OPK, int l, const double* q, const double* f, double* out, d
 }
 
 // Blocks of a reduction over level l's nodes (ell_reduce).
-unsigned red_grid(const Ell& E, int l) {
-  return std::min<unsigned>(nb(10 * E.m(l) * E.m(l)), RED_PER_SM * E.sms);
+unsigned red_grid(const Ell& E, int l, int per_sm = RED_PER_SM) {
+  return std::min<unsigned>(nb(10 * E.m(l) * E.m(l)), per_sm * E.sms);
 }
 
 // weighted dot / l2 into a device scalar; returns nothing (async)
 void dot_to(Ell& E, int l, const double* a, const double* b, double* out, int mode, const double* den = nullptr) {
-  k_ell_dot<<<red_grid(E, l), TPB, 0, E.s()>>>(E.view(l), a, b, E.partial, E.ticket, out, mode, den);
+  k_ell_dot<<<red_grid(E, l, DOT_PER_SM), TPB, 0, E.s()>>>(E.view(l), a, b, E.partial, E.ticket, out, mode, den);
 }
 void dot_dev(Ell& E, int l, const double* a, const double* b, int slot, int mode, const double* den = nullptr) {
   dot_to(E, l, a, b, E.scal + slot, mode, den);
