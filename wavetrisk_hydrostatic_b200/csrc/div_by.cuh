@@ -7,10 +7,12 @@ namespace wtk {
 // a / b from y = RN(1 / b) (__drcp_rn or 1.0 / b), correctly rounded: the quotient
 // estimate a y is within two units in the last place, one residual correction
 // makes it faithful and, by Markstein's theorem (P. Markstein, IBM J. Res. Dev.
-// 34(1), 1990), the second rounds it as the division does, short of underflow in
-// the residual (|a| below 2^-960 or so).  A zero, infinite or NaN estimate is returned
-// as it is, with its sign.  Five dependent operations replace a division's some
-// fifteen instructions wherever quotients share a divisor.
+// 34(1), 1990), the second rounds it as the division does.  That holds for a normal
+// quotient, b and y normal (|b| in 2^-1022 .. 2^1022: the divisors are edge lengths and
+// densities) and no underflow in the residual (|a| above 2^-960 or so).  A zero,
+// subnormal, infinite or NaN estimate is returned as it is, with its sign: the
+// division's value, but for a last unit of a subnormal one.  Five dependent operations
+// replace a division's some fifteen instructions wherever quotients share a divisor.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q0 = a * y;
   const double q1 = fma(fma(-b, q0, a), y, q0);
