@@ -28,13 +28,17 @@ def test_setup_does_not_wait_for_other_streams():
     S = EllipticSolver(levels, topos)       # loads the set-up's kernels
     want = solve(S)
     side = torch.cuda.Stream()
-    done = torch.cuda.Event()
-    with torch.cuda.stream(side):
-        torch.cuda._sleep(2_000_000_000)    # clock cycles: 1.0 s at 1965 MHz
-        done.record(side)
-    T = EllipticSolver(levels, topos)
-    running = not done.query()
-    side.synchronize()
+    for attempt in range(3):                # an allocation can take longer than the spin on a busy host
+        done = torch.cuda.Event()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(2_000_000_000)  # clock cycles: 1.0 s at 1965 MHz
+            done.record(side)
+        T = EllipticSolver(levels, topos)
+        running = not done.query()
+        side.synchronize()
+        if running:
+            break
+        T.close()
     assert running
     assert np.array_equal(solve(T), want)
     S.close()
