@@ -503,15 +503,14 @@ static FluxKernels flux_kernels(wt_handle* h) {
 }
 
 // Launch sequence of one trend evaluation of state (m, t, v); MODE_RK writes
-// dst = base + hstep * trend, MODE_TREND writes the trends into h->dm/dt/dv.
-static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode, const double* bm, const double* bt,
-                        const double* bv, double* om, double* ot, double* ov, double hstep, bool halo_first,
-                        KTimer* tm = nullptr) {
+// dst = base + hstep * trend, base the resident state, MODE_TREND writes the trends into
+// h->dm/dt/dv.
+static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode, double* om, double* ot, double* ov,
+                        double hstep, KTimer* tm = nullptr) {
   DevLevel& D = h->top();
   LevelDev L = D.view();
   const int nz = h->nz;
   cudaStream_t s = h->stream;
-  (void)halo_first;
   // block b: layer b % nz of node chunk b / nz (layer_node in trisk_kernels.cuh)
   const unsigned chunks = blocks_for(D.NN, NODE_TILE);
   const bool f32 = h->flux_bits == 32;
@@ -582,7 +581,8 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
     TrendIOF io{};
     io.theta = h->theta32; io.qe = h->qe32; io.hfm = h->hfm32; io.hft = h->hft32; io.ke = h->ke32;
     io.phik = h->phik; io.pterm = h->pterm;
-    io.base_m = bm; io.base_t = bt; io.base_v = bv; io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
+    io.base_m = h->mass; io.base_t = h->temp; io.base_v = h->velo;
+    io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
     io.dm = h->dm; io.dtt = h->dt; io.dv = h->dv;
     TB(5);
     if (mode == MODE_RK)
@@ -605,7 +605,8 @@ static int launch_trend(wt_handle* h, double* m, double* t, double* v, int mode,
   TE(2);
   TrendIO io{};
   io.theta = h->theta; io.qe = h->qe; io.hfm = h->hfm; io.hft = h->hft; io.bern = h->bern; io.phik = h->phik;
-  io.base_m = bm; io.base_t = bt; io.base_v = bv; io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
+  io.base_m = h->mass; io.base_t = h->temp; io.base_v = h->velo;
+  io.dst_m = om; io.dst_t = ot; io.dst_v = ov; io.h = hstep;
   io.dm = h->dm; io.dtt = h->dt; io.dv = h->dv;
   TB(5);
   if (kernels == FLUX_TILES) {
@@ -675,8 +676,7 @@ extern "C" {
 
 int wt_trend(wt_handle* h) {
   if (!h) return WT_ERR_ARG;
-  int rc = launch_trend(h, h->mass, h->temp, h->velo, MODE_TREND, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                        0.0, true);
+  int rc = launch_trend(h, h->mass, h->temp, h->velo, MODE_TREND, nullptr, nullptr, nullptr, 0.0);
   if (rc) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return WT_OK;
@@ -712,7 +712,7 @@ static int record_rk4(wt_handle* h, double dt, KTimer* tm = nullptr) {
     double* om = SM[oi[stage]];
     double* ot = ST[oi[stage]];
     double* ov = SV[oi[stage]];
-    int rc = launch_trend(h, qm, qt, qv, MODE_RK, h->mass, h->temp, h->velo, om, ot, ov, hs[stage], false, tm);
+    int rc = launch_trend(h, qm, qt, qv, MODE_RK, om, ot, ov, hs[stage], tm);
     if (rc) return rc;
   }
   CK(cudaGetLastError());

@@ -94,7 +94,7 @@ int ensure(wt_handle* h) {
   CKM(cudaStreamCreateWithPriority(&M->vs, cudaStreamNonBlocking, medium));
   M->flx.resize(M->L.size());
   for (cudaEvent_t& e : M->flx) CKM(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  M->edge_slots = (int)wtk::persistent_grid(wtk::k_trend_ml_velo, ~0u, wtk::EDGE_BLOCK);
+  M->edge_slots = (int)wtk::persistent_grid(wtk::k_trend_ml_velo, 1u << 16, wtk::EDGE_BLOCK);
   for (int l = h->level_start; l < h->level_end; ++l) {
     cudaStream_t s;
     cudaEvent_t e, r;

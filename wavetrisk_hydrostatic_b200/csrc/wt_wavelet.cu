@@ -627,9 +627,10 @@ MaskSet mask_set(wt_handle* h, int a, int b, int add) {
 }
 template <class K>
 void mask_sweep(wt_handle* h, K kernel, int a, int b, int add) {
-  if (a > b) return;
-  const MaskSet S = mask_set(h, a, b, add);
-  kernel<<<nb(S.start[S.nl]), TPB, 0, h->stream>>>(S);
+  for (; a <= b; a += MS_MAXL) {
+    const MaskSet S = mask_set(h, a, std::min(b, a + MS_MAXL - 1), add);
+    kernel<<<nb(S.start[S.nl]), TPB, 0, h->stream>>>(S);
+  }
 }
 }  // namespace
 
