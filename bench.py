@@ -452,7 +452,8 @@ def adaptive_launches(L, need_r=4):
     * The maps: one seed, need_r dilations and the cut to the tree; per parent
       level four reconstruct-map launches; three launches for the work lists.
     * compress_wavelets of the dropped slots.
-    The kernel timeline of one step at J4..J7 counts 243 for L = 4."""
+    The ncu launch list of one step (profiles/adaptive_J5-J9x32_step_launch_list.md)
+    counts 313 for L = 5."""
     C = L - 1
     stage = 16 * L + 8 * C + 12 * C + 16 * C
     masks = 13 * C + 8
@@ -463,7 +464,7 @@ def adaptive_launches(L, need_r=4):
 def algorithmic_bytes_trend_ml(level, nz, n_on=None, n_own=None, n_listed=None):
     """Compulsory bytes of one multi-level trend launch on a level with the
     fused RK sub-step (k_trend_ml_scal and k_trend_ml_velo, their list forms over the
-    level's work list, or k_trend_tma on the finest level, which stages every input plane
+    level's work list, or k_trend_tma<MODE_ML> on the finest level, which stages every input plane
     of a tile, so its traffic is higher).  Every node of [0, n]^2 reads its mask
     and writes dmass and dTheta (2 words a layer); every owned node writes the
     velocity source (3); the n_on nodes with mask_n >= TRSK also read theta,
@@ -755,6 +756,15 @@ def bench_ours(args):
         ach = ab / (t_list / 1e3) / 1e9
         ab_dense = algorithmic_bytes_trend_ml(args.level, args.nz)
         t_dense = r["phase_ms_dense"]["trend_ml_top"]
+        traffic = None
+        tf = os.path.join(ROOT, "profiles", "trend_ml_list_traffic.json")
+        if os.path.exists(tf):
+            try:
+                ratio = json.load(open(tf)).get("traffic_per_algorithmic_byte")
+                if ratio:   # measured on a smaller case, scaled by the bytes
+                    traffic = int(ratio * ab)
+            except Exception:
+                traffic = None
         cpu = cpu_baseline(args, quick=True, tree_fraction=r["tree_init"]["tree_fraction"])
         L = args.level - args.lmin + 1
         line = {
@@ -780,12 +790,15 @@ def bench_ours(args):
                     "parts_ms_per_step": r["e2e_parts_ms"]},
             "gpu_launches": adaptive_launches(L) * args.steps,
             "roofline": {"bound": "hbm", "kernel": "k_trend_ml_scal_list + k_trend_ml_velo_list (level_end, over its work list)", "achieved": ach,
-                         "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_src, "traffic": None,
+                         "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_src, "traffic": traffic,
                          "algorithmic_bytes_per_launch": ab, "listed_owned_nodes": listed,
                          "kernel_ms": t_list,
                          "timing": "CUDA events around the kernel's launches in one profiled RK4 step (phase by phase, "
                                    "the same needed-node maps and work lists as the timed steps)",
-                         "dense_tma_kernel": {"kernel": "k_trend_tma with every node computed (maps off)",
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the same kernels on the "
+                                           "J5..J7 x 32 workload, per algorithmic byte, scaled to this launch "
+                                           "(profiles/trend_ml_list_traffic.json)" if traffic else None,
+                         "dense_tma_kernel": {"kernel": "k_trend_tma<MODE_ML> with every node computed (maps off)",
                                               "ms": t_dense, "algorithmic_bytes": ab_dense,
                                               "achieved_GBps": ab_dense / (t_dense / 1e3) / 1e9,
                                               "frac": ab_dense / (t_dense / 1e3) / 1e9 / hbm},
@@ -883,7 +896,7 @@ def bench_ours_uniform(args):
             "e2e": {"value": e2e_value, "unit": "simulated days per wall-clock hour",
                     "h2d_bytes_per_step": r["h2d_bytes_per_step"], "d2h_bytes_per_step": r["d2h_bytes_per_step"],
                     "path": "wt_rk4_step_host (C-ABI), pinned host buffers, state copied in and out every step"},
-            "gpu_launches": (16 if args.level >= 6 else 12) * args.steps,
+            "gpu_launches": (16 if args.level >= 6 and args.nz >= 3 else 12) * args.steps,  # pipelined tiles: four a stage
             "roofline": {"bound": "hbm", "kernel": "trend_rk", "achieved": ach, "peak": hbm, "unit": "GB/s",
                          "frac": ach / hbm, "peak_source": peak_src, "traffic": traffic,
                          "dominant_kernel_by_time": dom, "kernel_ms_per_launch": kt},

@@ -47,7 +47,7 @@ constexpr int ML_TRSK = 2, ML_ADJZONE = 8;
 // 480 us of a stage (J4..J7 x 16).
 //
 // The velocity takes a thread an edge, the edge (`part`) the same for a whole warp.
-// A thread does up to four layers of its entry: remapped slots, Coriolis weights (the
+// A thread does up to four layers of its entry (up to eight without a list): remapped slots, Coriolis weights (the
 // remap's signs and the factor 1/2 of interp folded in, both exact) and the reciprocal
 // length are made once (14 + 12 loads and 28 operations a layer less).  Measured a
 // step, lists of J4..J7: one thread a node 832 us, an edge and a layer a thread 892,

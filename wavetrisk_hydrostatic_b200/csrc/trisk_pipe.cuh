@@ -15,11 +15,11 @@
 // k_step1 / k_trend (trisk_kernels.cuh) and their FP32-flux twins (trisk_mixed.cuh),
 // expression for expression.
 //
-// Tiles are 44 nodes wide: 44 divides the padded width at J7 exactly and wastes under
-// 2 % from there up, and the 48-wide box keeps every copy on a 16-byte boundary.
-// 44 x 5 nodes fill seven warps a part to 98 % (22 warps, 80 registers);
-// step1's spill 28 bytes at that, and 20 warps of 96 registers with 44 x 4 nodes are
-// slower (36.2 against 35.4 ms in 25 steps).
+// Tiles are 44 nodes wide: 44 divides the padded width at J7 exactly (the trend tiles the
+// padded level; 2.3 % of the width is wasted at J9), leaves 2.3 % of step1's n + 1 nodes
+// at J7 and 2.7 % at J8 empty, and the 48-wide box keeps every copy on a 16-byte boundary.
+// 44 x 5 nodes fill seven warps a part to 98 % (22 warps, 80 registers); step1's spill 28
+// bytes at that, and 20 warps of 96 registers with 44 x 4 nodes were 2 % slower.
 //
 // One layer of one tile a block, with its geometry, its copies waited for on the spot
 // and its ghosts patched in place (the kernels before: 24 warps a SM, 66 to 75 % of

@@ -1,7 +1,7 @@
 // C-ABI of trend_ml over the handle's whole hierarchy (src/multi_level.f90:5-188):
 // per level, fine to coarse, the level's operator arrays are computed by the
 // single-level column and step1 kernels, the coarse ones are then restricted
-// from the level above, and k_trend_ml finishes the level (scalar trends,
+// from the level above, and k_trend_ml_scal and _velo finish the level (scalar trends,
 // velocity source computed or restricted, gradient terms).  All layers of a
 // level are processed per launch: the layers interact only through the
 // pressure column, which k_column integrates bottom-up.
@@ -176,7 +176,7 @@ States hierarchy_state(wt_handle* h) {
 }
 
 // trend_ml of the state S into each level's dm, dt, dv (stream-ordered).  With
-// base and dest, each level's k_trend_ml also takes the RK sub-step
+// base and dest, each level's trend kernels also take the RK sub-step
 // dest = base + hs * trend (RK_sub_step, src/time_integr.f90:206-225) instead of
 // writing dv: a level's state is not read after its step1, so dest may be S.
 // With wav (and dest), the forward wavelets of WT_after_step for the level
@@ -533,7 +533,7 @@ int wt_adaptive_step(wt_handle* h, double dt, const double* threshold, int level
 
 // wt_rk4_multi with CUDA events around its phases: ms[p] = mean time of one
 // occurrence of phase p (0 column+step1 of level_end, 1 column+step1 of one
-// coarser level, 2 restrictions into one level, 3 k_trend_ml of level_end with
+// coarser level, 2 restrictions into one level, 3 the trend of level_end with
 // the fused RK sub-step, 4 the same on one coarser level, 5 unused (the RK
 // sub-step is fused), 6 WT_after_step); count[p] = occurrences per step.
 int wt_profile_rk4_multi(wt_handle* h, double dt, int nsteps, double* ms, int* count) {
