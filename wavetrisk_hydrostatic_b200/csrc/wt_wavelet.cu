@@ -212,13 +212,18 @@ void inverse(wt_handle* h, int partial = 0) {
     const ParentList PL = rec ? wt_level_plist(h, l) : kNoList;
     const dim3 pb = plan_block(nz);
     const int pt = (int)(pb.x * pb.y);
+    // Seven or eight layers: two a thread.  With one, the outer kernel's blocks of one edge have
+    // nothing to run beside their staging (inverse J5..J8 x 8: 514 us with eight rows, 452 with
+    // four, 508 with blocks of three edges); at five and six three rows cost the RK step 1-2 %.
+    const dim3 po(32, nz == 7 || nz == 8 ? 4 : pb.y);
+    const int ot = (int)(po.x * po.y);
     k_prolong_l<<<PL.ids ? pgrid(k_prolong_l, TPBL, nbl(par1, nz)) : nbl(par1, nz), TPBL, 0, sa>>>(P, C, nz, lpt_for(nz),
                                                                                                   rec, PL);
     k_recon_scalar_l<<<PL.ids ? pgrid(k_recon_scalar_l, TPBL, nbl(par0, nz)) : nbl(par0, nz), TPBL, 0, sa>>>(
         P, C, np, nz, lpt_for(nz), rec, PL);
     cudaEventRecord(W->ready_s[q], sa);
     const WavLevel& V = W->L[l - h->level_start];
-    k_recon_outer_p<<<PL.ids ? pgrid(k_recon_outer_p, pt, 3 * plan_grid(par1)) : 3 * plan_grid(par1), pb, 0, s>>>(
+    k_recon_outer_p<<<PL.ids ? pgrid(k_recon_outer_p, ot, 3 * plan_grid(par1)) : 3 * plan_grid(par1), po, 0, s>>>(
         P, C, nz, V.op_i, V.op_d, rec, PL);
     k_recon_inner_p<<<PL.ids ? pgrid(k_recon_inner_p, pt, plan_grid(par0)) : plan_grid(par0), pb, 0, s>>>(
         P, C, nz, V.ip_i, V.ip_d, rec, PL);
