@@ -188,18 +188,18 @@ __device__ __forceinline__ int ncode(const WLev& C, int d, int i, int j) {
   if (!inr(C, i, j)) return -1;
   return __ldg(C.nsrc + nid(C, d, i, j));
 }
-// With two fluxes (NF), as we / wn of wavelet_layers.cuh: no branch, read-only loads (the
-// child's fields).  One flux's blocks have half the threads, and skipping the absent
-// values' loads is the faster form there (J6 of J5..J7 x 8: 30.8 us a call, 33.3 without).
-template <int NF>
+// SPLIT (a thread takes one of two fluxes): as we / wn of wavelet_layers.cuh, no branch,
+// read-only loads (the child's fields).  Else the absent values' loads are skipped, the
+// faster form in blocks of 256 (J6 of J5..J7 x 8, one flux: 30.8 us a call, 33.3 without).
+template <bool SPLIT>
 __device__ __forceinline__ double fe(const double* __restrict__ f, int c) {
-  if (NF == 1 && c < 0) return 0.0;
+  if (!SPLIT && c < 0) return 0.0;
   const double v = __ldg(f + (max(c, 0) >> 1));
   return c < 0 ? 0.0 : (c & 1) ? -v : v;
 }
-template <int NF>
+template <bool SPLIT>
 __device__ __forceinline__ double fn(const double* __restrict__ f, int c) {
-  if (NF == 1 && c < 0) return 0.0;
+  if (!SPLIT && c < 0) return 0.0;
   const double v = __ldg(f + max(c, 0));
   return c < 0 ? 0.0 : v;
 }
@@ -322,60 +322,71 @@ __global__ void k_rf_plan(WLev P, WLev C, int* __restrict__ pi, double* __restri
 
 // One small flux of interp_flux from the staged plan: slots a at ia (9 codes)
 // and wd (6 weights) of edge x, sign pos.
-template <int NF>
+template <bool SPLIT>
 __device__ __forceinline__ double sm_eval_s(const int (*si)[32], const double (*sd)[32], int ia, int wd, int x,
                                             bool pos, const double* __restrict__ h) {
-  double s1 = fe<NF>(h, si[ia + 0][x]) * sd[wd + 0][x];
-  s1 = s1 + fe<NF>(h, si[ia + 1][x]) * sd[wd + 1][x];
-  s1 = s1 + fe<NF>(h, si[ia + 2][x]) * sd[wd + 2][x];
-  double s2 = (fe<NF>(h, si[ia + 3][x]) - fe<NF>(h, si[ia + 6][x])) * sd[wd + 3][x];
-  s2 = s2 + (fe<NF>(h, si[ia + 4][x]) - fe<NF>(h, si[ia + 7][x])) * sd[wd + 4][x];
-  s2 = s2 + (fe<NF>(h, si[ia + 5][x]) - fe<NF>(h, si[ia + 8][x])) * sd[wd + 5][x];
+  double s1 = fe<SPLIT>(h, si[ia + 0][x]) * sd[wd + 0][x];
+  s1 = s1 + fe<SPLIT>(h, si[ia + 1][x]) * sd[wd + 1][x];
+  s1 = s1 + fe<SPLIT>(h, si[ia + 2][x]) * sd[wd + 2][x];
+  double s2 = (fe<SPLIT>(h, si[ia + 3][x]) - fe<SPLIT>(h, si[ia + 6][x])) * sd[wd + 3][x];
+  s2 = s2 + (fe<SPLIT>(h, si[ia + 4][x]) - fe<SPLIT>(h, si[ia + 7][x])) * sd[wd + 4][x];
+  s2 = s2 + (fe<SPLIT>(h, si[ia + 5][x]) - fe<SPLIT>(h, si[ia + 8][x])) * sd[wd + 5][x];
   return pos ? s1 + s2 : -s1 - s2;
 }
 
 // flux_cpt_restr of up to two fluxes (mass, Theta: fp0/fp1 from the child's
 // fc0/fc1 and dscalar dc0/dc1) on the restricted parent edges (mask_e >=
-// RESTRCT).  Block (32, fluxes x ny): 32 consecutive parent edges of the plan, ny
-// threads per edge and flux taking layers y, y + ny, ...; blocks without a restricted
-// edge return before staging.  With a work list (PL), persistent blocks take
+// RESTRCT).  Block (32, ny): 32 consecutive parent edges of the plan, ny threads per edge
+// taking layers y, y + ny, ..., the fluxes in turn; SPLIT: (32, 2 ny), ny threads per edge
+// and flux.  Blocks without a restricted edge return before staging.  With a work list (PL), persistent blocks take
 // 32 of the listed parents' edges at a time.  Same expression trees and operand order as
 // part_coarse_flux + coarse_flux + interp_flux of the reference.
-template <int NF>
+template <int NF, bool SPLIT>
 __device__ __forceinline__ void restr_flux_one(const WLev& P, int nz, const int (*si)[32], const double (*sd)[32],
                                                int x, int d, int ip, int jp, int e, double* __restrict__ fp0,
                                                double* __restrict__ fp1, const double* __restrict__ fc0,
                                                const double* __restrict__ fc1, const double* __restrict__ dc0,
                                                const double* __restrict__ dc1, int NNc) {
-  const int y = threadIdx.y / NF, ny = blockDim.y / NF, f = threadIdx.y % NF;
+  constexpr int TF = SPLIT ? NF : 1;  // threads an edge and layer
+  const int y = threadIdx.y / TF, ny = blockDim.y / TF;
   const bool pa = (e & 1) != 0, pb = ((e + 1) & 1) != 0;
   const int64_t so = (int64_t)e * P.NN + nid(P, d, ip, jp);
   const double ar0 = sd[12][x], ar1 = sd[13][x], o0 = sd[14][x], o1 = sd[15][x], o2 = sd[16][x], o3 = sd[17][x];
-  double* __restrict__ fp = f == 0 ? fp0 : fp1;
-  for (int k = y; k < nz; k += ny) {
-    const double* __restrict__ h = (f == 0 ? fc0 : fc1) + (int64_t)3 * k * NNc;
-    const double* __restrict__ ds = (f == 0 ? dc0 : dc1) + (int64_t)k * NNc;
-    const double sma = sm_eval_s<NF>(si, sd, 0, 0, x, pa, h), smb = sm_eval_s<NF>(si, sd, 9, 6, x, pb, h);
-    double tp = fe<NF>(h, si[18][x]) * ar0;
-    tp = tp + fe<NF>(h, si[19][x]) * ar1;
-    tp = tp - (fe<NF>(h, si[20][x]) + fe<NF>(h, si[21][x])) * ar1;
-    tp = tp - (fe<NF>(h, si[22][x]) + fe<NF>(h, si[23][x])) * ar0;
-    tp = tp + o2 * fn<NF>(ds, si[24][x]);
-    tp = tp - o3 * fn<NF>(ds, si[26][x]);
-    tp = tp - o0 * fn<NF>(ds, si[25][x]);
-    tp = tp + o1 * fn<NF>(ds, si[27][x]);
-    const double dmz = fn<NF>(ds, si[28][x]), dpz = fn<NF>(ds, si[29][x]);
-    double tc = sd[18][x] * (dpz - dmz);
-    tc = tc + sd[19][x] * (fn<NF>(ds, si[32][x]) - dmz);
-    tc = tc + sd[20][x] * (fn<NF>(ds, si[31][x]) - dmz);
-    tc = tc + sd[21][x] * (dpz - fn<NF>(ds, si[33][x]));
-    tc = tc + sd[22][x] * (dpz - fn<NF>(ds, si[30][x]));
-    fp[(int64_t)3 * k * P.NN + so] = tp + tc + sma + smb;
-  }
+  for (int k = y; k < nz; k += ny)
+#pragma unroll 1
+    for (int q = 0; q < NF / TF; ++q) {
+      const int f = SPLIT ? threadIdx.y % TF : q;
+      double* __restrict__ fp = f == 0 ? fp0 : fp1;
+      const double* __restrict__ h = (f == 0 ? fc0 : fc1) + (int64_t)3 * k * NNc;
+      const double* __restrict__ ds = (f == 0 ? dc0 : dc1) + (int64_t)k * NNc;
+      const double sma = sm_eval_s<SPLIT>(si, sd, 0, 0, x, pa, h), smb = sm_eval_s<SPLIT>(si, sd, 9, 6, x, pb, h);
+      double tp = fe<SPLIT>(h, si[18][x]) * ar0;
+      tp = tp + fe<SPLIT>(h, si[19][x]) * ar1;
+      tp = tp - (fe<SPLIT>(h, si[20][x]) + fe<SPLIT>(h, si[21][x])) * ar1;
+      tp = tp - (fe<SPLIT>(h, si[22][x]) + fe<SPLIT>(h, si[23][x])) * ar0;
+      tp = tp + o2 * fn<SPLIT>(ds, si[24][x]);
+      tp = tp - o3 * fn<SPLIT>(ds, si[26][x]);
+      tp = tp - o0 * fn<SPLIT>(ds, si[25][x]);
+      tp = tp + o1 * fn<SPLIT>(ds, si[27][x]);
+      const double dmz = fn<SPLIT>(ds, si[28][x]), dpz = fn<SPLIT>(ds, si[29][x]);
+      double tc = sd[18][x] * (dpz - dmz);
+      tc = tc + sd[19][x] * (fn<SPLIT>(ds, si[32][x]) - dmz);
+      tc = tc + sd[20][x] * (fn<SPLIT>(ds, si[31][x]) - dmz);
+      tc = tc + sd[21][x] * (dpz - fn<SPLIT>(ds, si[33][x]));
+      tc = tc + sd[22][x] * (dpz - fn<SPLIT>(ds, si[30][x]));
+      fp[(int64_t)3 * k * P.NN + so] = tp + tc + sma + smb;
+    }
 }
 
-template <int NF>
-__global__ void __launch_bounds__(256 * NF, NF == 2 ? 2 : 4)
+// Two fluxes are split with few layers, where a block's rows are few, over a work list's
+// few parents or in a dense launch of few blocks (J4 and J5 parents): adaptive step J4..J6 x
+// 2 734 us, 764 in turn; x 5 860, 884; all patches J4..J6 x 4 763, 783, x 6 888, 900.  More
+// layers, and a larger dense launch, whose blocks mostly return at once, take them in turn:
+// J5..J8 x 6 2372 us, 2440 split, x 16 4330, 4405; all patches J5..J9 x 8 8260, 9250 split.
+constexpr int RF_SPLIT_LIST = 5, RF_SPLIT = 6;
+constexpr unsigned RF_SPLIT_BLOCKS = 1000;
+template <int NF, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 512 : 256, SPLIT ? 2 : 4)  // 64 registers; at 80 the split form is 2 % of a step slower
     k_restr_flux3(WLev P, int m, int nz, const int* __restrict__ pi, const double* __restrict__ pd,
                   double* __restrict__ fp0, double* __restrict__ fp1, const double* __restrict__ fc0,
                   const double* __restrict__ fc1, const double* __restrict__ dc0, const double* __restrict__ dc1,
@@ -401,7 +412,7 @@ __global__ void __launch_bounds__(256 * NF, NF == 2 ? 2 : 4)
               sd[q - RF_NI][x] = pd[(q - RF_NI) * ne + u];
           }
         __syncthreads();
-        if (on) restr_flux_one<NF>(P, nz, si, sd, x, d, ip, jp, e, fp0, fp1, fc0, fc1, dc0, dc1, NNc);
+        if (on) restr_flux_one<NF, SPLIT>(P, nz, si, sd, x, d, ip, jp, e, fp0, fp1, fc0, fc1, dc0, dc1, NNc);
       }
       __syncthreads();
     }
@@ -429,7 +440,7 @@ __global__ void __launch_bounds__(256 * NF, NF == 2 ? 2 : 4)
     }
   __syncthreads();
   if (!on) return;
-  restr_flux_one<NF>(P, nz, si, sd, x, d, ip, jp, e, fp0, fp1, fc0, fc1, dc0, dc1, NNc);
+  restr_flux_one<NF, SPLIT>(P, nz, si, sd, x, d, ip, jp, e, fp0, fp1, fc0, fc1, dc0, dc1, NNc);
 }
 
 // scalar_cpt_restr of one or two fields (b null: one) over parents [0, n]^2, every

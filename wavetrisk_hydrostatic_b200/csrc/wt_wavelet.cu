@@ -212,10 +212,13 @@ void inverse(wt_handle* h, int partial = 0) {
     const ParentList PL = rec ? wt_level_plist(h, l) : kNoList;
     const dim3 pb = plan_block(nz);
     const int pt = (int)(pb.x * pb.y);
-    // Seven or eight layers: two a thread.  With one, the outer kernel's blocks of one edge have
-    // nothing to run beside their staging (inverse J5..J8 x 8: 514 us with eight rows, 452 with
-    // four, 508 with blocks of three edges); at five and six three rows cost the RK step 1-2 %.
-    const dim3 po(32, nz == 7 || nz == 8 ? 4 : pb.y);
+    // Seven or eight layers over more blocks than the device holds at once: two a thread.
+    // With one, the outer kernel's blocks of one edge have nothing to run beside their staging
+    // (inverse J5..J8 x 8: 514 us with eight rows, 452 with four, 508 with blocks of three
+    // edges).  With few blocks the rows are wanted (adaptive step J4..J6 x 8 970 us, 990 with
+    // four), and at five and six layers three rows cost the RK step 1-2 %.
+    const bool pairs = (nz == 7 || nz == 8) && 3 * plan_grid(par1) > 1200;
+    const dim3 po(32, pairs ? 4 : pb.y);
     const int ot = (int)(po.x * po.y);
     k_prolong_l<<<PL.ids ? pgrid(k_prolong_l, TPBL, nbl(par1, nz)) : nbl(par1, nz), TPBL, 0, sa>>>(P, C, nz, lpt_for(nz),
                                                                                                   rec, PL);
@@ -1026,11 +1029,12 @@ int restrict_flux(wt_handle* h, int level, double* par0, double* par1, const dou
   if (!V.rf_pi) return WT_ERR_ARG;
   const int m = h->at(level).n;
   const int64_t ne = (int64_t)3 * 10 * m * m;
-  // a lone layer has two warps stage its plan
-  const dim3 blk(32, (par1 ? 2 : 1) * std::min(nz, 8) + (!par1 && nz == 1));
   const ParentList PL = wt_level_plist(h, level);
   const unsigned dense = (unsigned)((ne + 31) / 32);
-  const auto k = par1 ? k_restr_flux3<2> : k_restr_flux3<1>;
+  const bool split = par1 && (PL.ids ? nz <= RF_SPLIT_LIST : nz <= RF_SPLIT && dense <= RF_SPLIT_BLOCKS);
+  // a lone layer has two warps stage its plan
+  const dim3 blk(32, (split ? 2 : 1) * std::min(nz, 8) + (!split && nz == 1));
+  const auto k = split ? k_restr_flux3<2, true> : par1 ? k_restr_flux3<2, false> : k_restr_flux3<1, false>;
   k<<<PL.ids ? pgrid(k, (int)(blk.x * blk.y), dense) : dense, blk, 0, h->stream>>>(
       view(h, level), m, nz, V.rf_pi, V.rf_pd, par0, par1, chd0, chd1, dsc0, dsc1, (int)h->at(level + 1).NN, PL);
   CKW(cudaGetLastError());
